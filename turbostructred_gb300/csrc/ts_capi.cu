@@ -153,7 +153,14 @@ struct ts_handle {
         if ((s = alloc(&pb.U, NV * L.plane)) != TS_OK) return s;
         TS_CUDA(cudaMemsetAsync(pb.U, 0, NV * L.plane * sizeof(double), stream));
         if (linear && (s = alloc(&pb.G, (size_t)nd * NV * L.plane)) != TS_OK) return s;
-        if (limited && (s = alloc(&pb.Lim, NV * L.plane)) != TS_OK) return s;
+        // a periodic face samples the opposite cell with the ghost's size
+        pb.fold = 1;
+        for (int a = 0; a < nd; ++a) {
+            const std::vector<double>& H = a == 0 ? grid.hx : (a == 1 ? grid.hy : grid.hz);
+            const int n = L.n(a);
+            if (ph.periodic[a] && (H[0] != H[n] || H[n + 1] != H[1])) pb.fold = 0;
+        }
+        if (limited && !pb.fold && (s = alloc(&pb.Lim, NV * L.plane)) != TS_OK) return s;
         for (int a = 0; a < nd; ++a) {
             if ((s = alloc(&pb.F[a], NV * L.plane)) != TS_OK) return s;
             if ((s = alloc(&pb.Lam[a], L.plane)) != TS_OK) return s;

@@ -179,6 +179,9 @@ Phys make_phys(const ts_config& c) {
     for (int a = 0; a < 3; ++a) p.periodic[a] = (a < c.n_dims) ? (c.periodic[a] != 0) : 1;
     p.gamma = c.gamma;
     p.p_inf = c.eos == TS_EOS_STIFFENED_GAS ? c.p_inf : 0.0;
+    p.gm1 = p.gamma - 1.0;
+    p.hgm1 = 0.5 * (p.gamma - 1.0);
+    p.gpinf = p.gamma * p.p_inf;
     p.eps = c.eps;
     p.cfl = c.cfl;
     for (int id = 0; id < kBcIds; ++id) {

@@ -106,6 +106,7 @@ struct Phys {
     int recon, limiter, solver, eos;
     int periodic[3];
     double gamma, p_inf, eps, cfl;
+    double gm1, hgm1, gpinf;   // gamma - 1, 0.5 (gamma - 1), gamma p_inf, as the kernels would round them
     BcSet bc;
     int force, accel;          // source terms on (kernel.h:941-989)
     double sigma[3], g[3];     // Sigma, UniformAcceleration

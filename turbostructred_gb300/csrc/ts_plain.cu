@@ -7,7 +7,7 @@
 // exact zeros: products with the zero components of axis normals, which the
 // reference evaluates, are dropped here).
 //
-// One step is six launches on the handle's stream:
+// One step, on the handle's stream:
 //   k_ghost<A>   ghost layers per axis: periodic copy or boundary condition
 //                (Kernel::ExchangeValues + ComputeDummyCellValues, kernel.h:334-915)
 //   k_recon      per-cell slopes and limiter (ComputeSolutionReconstruction, :879-925)
@@ -16,17 +16,36 @@
 //   k_dt         spectral radius per cell, V/SR, warp-shuffle min, last block
 //                finalises dt (ComputeTimeStep, :1427-1437)
 //   k_update     flux divergence fused with the stage update
-//                (residual accumulation :1232 + Kernel::UpdateSolution, kernel.h:319-331)
-//   k_finish     time/iteration and the Kernel::Run termination rules
-// FP64 is scarce on GB300 (about 2 FMA/clk/SM), so this path is compute-bound;
-// the layout and launches are chosen for coalescing, not for bandwidth.
+//                (residual accumulation :1232 + Kernel::UpdateSolution,
+//                kernel.h:319-331); the last block closes the step: time,
+//                iteration and the Kernel::Run termination rules
+//
+// What bounds it: the FP64 pipe.  GB300 takes 19 clocks per SM for an FP64
+// warp instruction of any kind, comparisons, min/max and |x| included, while
+// the issue slots are 85 % idle.  So everything but the additions and
+// multiplications themselves runs on the integer pipe: divisions and square
+// roots (ts_exact64.cuh), comparisons, sign changes and halvings; terms that
+// are exact zeros are skipped where a whole warp agrees (transverse momentum
+// of 1D and 2D flows, constant neighbourhoods, equal fluxes); the slope
+// projections lim * (slope * h/2) are formed once per cell instead of at each
+// of its faces; and the residual norms are summed per thread over many
+// cells before the block's reduction.  The results are bit for bit the same.
+// Measured on one GB300, time per step before and after: 3D blast 192^3 (Roe,
+// Barth-Jespersen) 28.4 -> 9.98 ms (k_recon 8.1 -> 0.69, each k_flux 5.9 ->
+// 2.7, k_update 3.0 -> 0.72); 2D shear layer 1024^2 (HLLC) 3.27 -> 0.70 ms.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <type_traits>
+
+#include "ts_exact64.cuh"
 #include "ts_plain.h"
 
 namespace ts {
 
 namespace {
+
+typedef unsigned long long u64;
 
 __device__ __forceinline__ long long vidx(const Layout& L, int v) { return (long long)v * L.plane; }
 
@@ -74,87 +93,185 @@ __device__ __forceinline__ void bc_values(const Phys& ph, int side, int A, doubl
     // Natural and SubsonicOutlet copy the inner state (BCGeneral.h:200-211).
 }
 
+// Comparisons of doubles on the integer pipe.  GB300 executes FP64 at about
+// 1.7 operations per clock per SM, and half of k_recon's FP64-pipe
+// instructions were comparisons (measured with ncu).  dkey is monotone in the
+// value and gives -0 and +0 the same key, so dkey(a) < dkey(b) is exactly
+// a < b, and the sign tests below are exactly x > 0 and x < 0, for every
+// non-NaN a, b, x (a NaN only arises in a run whose health flags stop it).
+__device__ __forceinline__ long long dkey(double x) {
+    const long long b = __double_as_longlong(x);
+    return b < 0 ? (b ^ 0x7FFFFFFFFFFFFFFFLL) + 1 : b;
+}
+__device__ __forceinline__ bool dlt(double a, double b) { return dkey(a) < dkey(b); }
+__device__ __forceinline__ bool dpos(double x) { return __double_as_longlong(x) > 0; }
+__device__ __forceinline__ bool dneg(double x) {
+    const long long b = __double_as_longlong(x);
+    return b < 0 && b != (long long)0x8000000000000000ULL;
+}
+__device__ __forceinline__ bool dzero(double x) { return x64::is_zero(x64::hi_of(x), x64::lo_of(x)); }
+// |x| and -x on the integer pipe
+__device__ __forceinline__ double dabs(double x) { return x64::of_words(x64::hi_of(x) & 0x7FFFFFFFu, x64::lo_of(x)); }
+__device__ __forceinline__ double dneg_of(double x) { return x64::of_words(x64::hi_of(x) ^ 0x80000000u, x64::lo_of(x)); }
+// |a| < |b|: the magnitudes' bit patterns order like their values
+__device__ __forceinline__ bool dabs_lt(double a, double b) {
+    return (__double_as_longlong(a) & 0x7FFFFFFFFFFFFFFFLL) < (__double_as_longlong(b) & 0x7FFFFFFFFFFFFFFFLL);
+}
+
+// ---------------------------------------------------------------------------
+// Arithmetic of the two instances of every heavy routine
+// ---------------------------------------------------------------------------
+// Fast: divisions, square roots and halvings on the integer pipe
+// (ts_exact64.cuh), correctly rounded like the hardware's, for operands in the
+// ranges stated there; anything else sets `bad` and the result is discarded.
+// Plain: the hardware operations, for the faces and cells where Fast gave up
+// (zero, subnormal, infinite or NaN divisors and the like).  Both perform the
+// same additions and multiplications in the same order.
+struct Fast {
+    typedef x64::Divisor Div;
+    bool bad = false;
+    __device__ __forceinline__ Div divisor(double b) { return x64::divisor(b, bad); }
+    __device__ __forceinline__ double over(double a, const Div& d) { return x64::quotient(a, d, bad); }
+    __device__ __forceinline__ double div(double a, double b) { return x64::div(a, b, bad); }
+    __device__ __forceinline__ double root(double a) { return x64::root(a, bad); }
+    __device__ __forceinline__ double half(double a) { return x64::half(a, bad); }
+    __device__ __forceinline__ double min(double a, double b) { return dlt(a, b) ? a : b; }
+    __device__ __forceinline__ double max(double a, double b) { return dlt(a, b) ? b : a; }
+    __device__ __forceinline__ bool lt(double a, double b) { return dlt(a, b); }
+    __device__ __forceinline__ bool ge0(double a) { return !dneg(a); }
+    __device__ __forceinline__ bool le0(double a) { return !dpos(a); }
+};
+struct Plain {
+    typedef double Div;
+    __device__ __forceinline__ Div divisor(double b) { return b; }
+    __device__ __forceinline__ double over(double a, Div d) { return a / d; }
+    __device__ __forceinline__ double div(double a, double b) { return a / b; }
+    __device__ __forceinline__ double root(double a) { return sqrt(a); }
+    __device__ __forceinline__ double half(double a) { return a * 0.5; }
+    __device__ __forceinline__ double min(double a, double b) { return fmin(a, b); }
+    __device__ __forceinline__ double max(double a, double b) { return fmax(a, b); }
+    __device__ __forceinline__ bool lt(double a, double b) { return a < b; }
+    __device__ __forceinline__ bool ge0(double a) { return a >= 0.0; }
+    __device__ __forceinline__ bool le0(double a) { return a <= 0.0; }
+};
+
 // ---------------------------------------------------------------------------
 // Riemann solvers
 // ---------------------------------------------------------------------------
+// Momentum components NC.. of both states are exact zeros (NC < 3: 1D and 2D
+// flows without transverse momentum, checked by the caller): every term they
+// enter is an exact zero and is left out, and their flux is zero.
+
 __device__ __forceinline__ double pressure(const Phys& ph, double ro, double vx, double vy, double vz, double roE) {
     double p = (ph.gamma - 1.0) * (roE - ro * (vx * vx + vy * vy + vz * vz) / 2.0);
     if (ph.eos == TS_EOS_STIFFENED_GAS) p = p - ph.gamma * ph.p_inf;
     return p;
 }
 
-// F(U).e_A (RoeSolverPerfectGasEOS.h:41-58).
-template <int A>
-__device__ __forceinline__ void phys_flux(const Phys& ph, const double U[NV], double res[NV]) {
-    const double ro = U[0];
-    const double vel[3] = {U[1] / ro, U[2] / ro, U[3] / ro};
-    const double roE = U[4];
-    const double p = pressure(ph, ro, vel[0], vel[1], vel[2], roE);
-    const double vn = vel[A];
-    const double rvn = ro * vn;
-    res[0] = rvn;
-#pragma unroll
-    for (int b = 0; b < 3; ++b) res[1 + b] = (b == A) ? rvn * vel[b] + p : rvn * vel[b];
-    res[4] = vn * (roE + p);
-}
-
-__device__ __forceinline__ double harten(double z, double eps) {
-    z = fabs(z);
-    if (z < eps) z = ((z * z) / eps + eps) * 0.5;
+template <class O>
+__device__ __forceinline__ double harten(double z, double eps, O& o) {
+    z = dabs(z);
+    if (o.lt(z, eps)) z = o.half(o.div(z * z, eps) + eps);
     return z;
 }
 
+template <int NC>
+__device__ __forceinline__ double dot(const double a[3], const double b[3]) {
+    double s = a[0] * b[0];
+    if (NC > 1) s = s + a[1] * b[1];
+    if (NC > 2) s = s + a[2] * b[2];
+    return s;
+}
+
+// Velocity, |u|^2 and pressure of a face state (the pressure of
+// RoeSolverPerfectGasEOS.h:41-58, shared by the solvers below).
+template <int NC, class O>
+struct Side {
+    typename O::Div ro;
+    double v[3], q, p;
+    __device__ __forceinline__ Side(const Phys& ph, const double U[NV], O& o) {
+        ro = o.divisor(U[0]);
+        v[1] = v[2] = 0.0;
+#pragma unroll
+        for (int b = 0; b < NC; ++b) v[b] = o.over(U[1 + b], ro);
+        q = dot<NC>(v, v);
+        p = ph.gm1 * (U[4] - o.half(U[0] * q));
+        if (ph.eos == TS_EOS_STIFFENED_GAS) p = p - ph.gpinf;
+    }
+    // F(U).e_A (RoeSolverPerfectGasEOS.h:41-58)
+    template <int A>
+    __device__ __forceinline__ void flux(const double U[NV], double res[NV]) const {
+        const double rvn = U[0] * v[A];
+        res[0] = rvn;
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            res[1 + b] = b < NC ? rvn * v[b] : 0.0;
+            if (b == A) res[1 + b] = res[1 + b] + p;
+        }
+        res[4] = v[A] * (U[4] + p);
+    }
+};
+
 // RoeSolverPerfectGasEOS::ComputeFlux (RoeSolverPerfectGasEOS.h:74-160) with
 // fn = e_A; dn = 1 so dn*c = c and 1/(dn*dn) = 1 exactly.
-template <int A>
-__device__ double roe_flux(const Phys& ph, const double UL[NV], const double UR[NV], double flux[NV]) {
+template <int A, int NC, class O>
+__device__ __forceinline__ double roe_flux(const Phys& ph, const double UL[NV], const double UR[NV], double flux[NV],
+                                           O& o) {
     const double g = ph.gamma;
-    double FL[NV], FR[NV];
-    phys_flux<A>(ph, UL, FL);
-    phys_flux<A>(ph, UR, FR);
+    const Side<NC, O> l(ph, UL, o), r(ph, UR, o);
+    {
+        double FL[NV], FR[NV];
+        l.template flux<A>(UL, FL);
+        r.template flux<A>(UR, FR);
 #pragma unroll
-    for (int i = 0; i < NV; ++i) flux[i] = FL[i] + FR[i];
+        for (int i = 0; i < NV; ++i) flux[i] = FL[i] + FR[i];
+    }
     const double ro_l = UL[0], ro_r = UR[0];
-    const double vl[3] = {UL[1] / ro_l, UL[2] / ro_l, UL[3] / ro_l};
-    const double vr[3] = {UR[1] / ro_r, UR[2] / ro_r, UR[3] / ro_r};
-    const double e_l = UL[4] / ro_l, e_r = UR[4] / ro_r;
-    double k = 0.5 * (vl[0] * vl[0] + vl[1] * vl[1] + vl[2] * vl[2]);
+    const double e_l = o.over(UL[4], l.ro), e_r = o.over(UR[4], r.ro);
+    double k = o.half(l.q);
     double h_l = (e_l - k) * g + k;
-    k = 0.5 * (vr[0] * vr[0] + vr[1] * vr[1] + vr[2] * vr[2]);
+    k = o.half(r.q);
     double h_r = (e_r - k) * g + k;
     if (ph.eos == TS_EOS_STIFFENED_GAS) {
-        h_l = h_l - g * ph.p_inf / ro_l;
-        h_r = h_r - g * ph.p_inf / ro_r;
+        h_l = h_l - o.over(ph.gpinf, l.ro);
+        h_r = h_r - o.over(ph.gpinf, r.ro);
     }
-    const double sl = sqrt(ro_l), sr = sqrt(ro_r);
-    const double ql = sl / (sl + sr);
-    const double qr = sr / (sl + sr);
-    const double vel[3] = {ql * vl[0] + qr * vr[0], ql * vl[1] + qr * vr[1], ql * vl[2] + qr * vr[2]};
+    const double sl = o.root(ro_l), sr = o.root(ro_r);
+    const typename O::Div ss = o.divisor(sl + sr);
+    const double ql = o.over(sl, ss);
+    const double qr = o.over(sr, ss);
+    double vel[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int b = 0; b < NC; ++b) vel[b] = ql * l.v[b] + qr * r.v[b];
     const double h = ql * h_l + qr * h_r;
-    const double phi2 = 0.5 * (g - 1) * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]);
-    const double c = sqrt((g - 1) * h - phi2);
+    const double phi2 = ph.hgm1 * dot<NC>(vel, vel);
+    const double c = o.root(ph.gm1 * h - phi2);
     const double uw = vel[A];
-    const double eig_max = fabs(uw) + c;
-    const double he = ph.eps * eig_max;
-    const double AA1 = harten(uw, he);
-    const double AA3 = harten(uw + c, he);
-    const double AA4 = harten(uw - c, he);
+    const double eig_max = dabs(uw) + c;
+    double AA1 = dabs(uw), AA3 = dabs(uw + c), AA4 = dabs(uw - c);
+    if (ph.eps != 0.0) {
+        const double he = ph.eps * eig_max;
+        AA1 = harten(AA1, he, o);
+        AA3 = harten(AA3, he, o);
+        AA4 = harten(AA4, he, o);
+    }
     const double Eig1 = AA1;
-    const double Eiga = (AA3 - AA4) * 0.5 / c;
-    const double Eigb = (AA3 + AA4) * 0.5 - AA1;
-    const double R1 = phi2 * ro_r - (g - 1) * ro_r * ((vel[0] * vr[0] + vel[1] * vr[1] + vel[2] * vr[2]) - e_r);
-    const double D1 = ro_r * (vr[A] - vel[A]);
-    const double R2 = phi2 * ro_l - (g - 1) * ro_l * ((vel[0] * vl[0] + vel[1] * vl[1] + vel[2] * vl[2]) - e_l);
-    const double D2 = ro_l * (vl[A] - vel[A]);
-    const double C2 = 1.0 / (c * c);
+    const double Eiga = o.div(o.half(AA3 - AA4), c);
+    const double Eigb = o.half(AA3 + AA4) - AA1;
+    const double R1 = phi2 * ro_r - ph.gm1 * ro_r * (dot<NC>(vel, r.v) - e_r);
+    const double D1 = ro_r * (r.v[A] - vel[A]);
+    const double R2 = phi2 * ro_l - ph.gm1 * ro_l * (dot<NC>(vel, l.v) - e_l);
+    const double D2 = ro_l * (l.v[A] - vel[A]);
+    const double C2 = o.div(1.0, c * c);
     // Qa = (0, e_A, uw), Qb = (1, vel, h); terms multiplying a zero Qa entry
     // are exact zeros and are left out.
     {
         const double t = Eig1 * UL[0] + Eiga * D2 + Eigb * (R2 * C2) - Eig1 * UR[0] - Eiga * D1 - Eigb * (R1 * C2);
-        flux[0] = (flux[0] + t) * 0.5;
+        flux[0] = o.half(flux[0] + t);
     }
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
+        if (b >= NC) continue;
         double t;
         if (b == A)
             t = Eig1 * UL[1 + b] + Eiga * (R2 + D2 * vel[b]) + Eigb * (R2 * vel[b] * C2 + D2) - Eig1 * UR[1 + b] -
@@ -162,68 +279,77 @@ __device__ double roe_flux(const Phys& ph, const double UL[NV], const double UR[
         else
             t = Eig1 * UL[1 + b] + Eiga * (D2 * vel[b]) + Eigb * (R2 * vel[b] * C2) - Eig1 * UR[1 + b] -
                 Eiga * (D1 * vel[b]) - Eigb * (R1 * vel[b] * C2);
-        flux[1 + b] = (flux[1 + b] + t) * 0.5;
+        flux[1 + b] = o.half(flux[1 + b] + t);
     }
     {
         const double t = Eig1 * UL[4] + Eiga * (R2 * uw + D2 * h) + Eigb * (R2 * h * C2 + D2 * uw) - Eig1 * UR[4] -
                          Eiga * (R1 * uw + D1 * h) - Eigb * (R1 * h * C2 + D1 * uw);
-        flux[4] = (flux[4] + t) * 0.5;
+        flux[4] = o.half(flux[4] + t);
     }
     return eig_max;
 }
 
 // HLLC (Toro ch. 10.4) with Einfeldt-type speeds from Roe averages; same
-// operation order as the oracle's restatement.  Not in the reference.
-template <int A>
-__device__ double hllc_flux(const Phys& ph, const double UL[NV], const double UR[NV], double flux[NV]) {
+// operation order as the oracle's restatement.  Not in the reference.  The
+// flux and star state of the side that S* selects are formed once, from the
+// selected operands.
+template <int A, int NC, class O>
+__device__ __forceinline__ double hllc_flux(const Phys& ph, const double UL[NV], const double UR[NV], double flux[NV],
+                                            O& o) {
     const double g = ph.gamma;
-    const double pinf = ph.eos == TS_EOS_STIFFENED_GAS ? ph.p_inf : 0.0;
-    const int m = 1 + A;
+    const bool stiff = ph.eos == TS_EOS_STIFFENED_GAS;
+    const double pinf = stiff ? ph.p_inf : 0.0;
     const double rl = UL[0], rr = UR[0];
-    const double ul = UL[m] / rl, ur = UR[m] / rr;
-    const double vlx = UL[1] / rl, vly = UL[2] / rl, vlz = UL[3] / rl;
-    const double vrx = UR[1] / rr, vry = UR[2] / rr, vrz = UR[3] / rr;
-    const double pl = pressure(ph, rl, vlx, vly, vlz, UL[4]);
-    const double pr = pressure(ph, rr, vrx, vry, vrz, UR[4]);
-    const double cl = sqrt(g * (pl + pinf) / rl);
-    const double cr = sqrt(g * (pr + pinf) / rr);
-    const double hl = (UL[4] + pl) / rl;
-    const double hr = (UR[4] + pr) / rr;
-    const double sl = sqrt(rl), sr = sqrt(rr);
-    const double wl = sl / (sl + sr), wr = sr / (sl + sr);
-    const double ut = wl * ul + wr * ur;
-    const double vtx = wl * vlx + wr * vrx, vty = wl * vly + wr * vry, vtz = wl * vlz + wr * vrz;
+    const Side<NC, O> l(ph, UL, o), r(ph, UR, o);
+    const double ul = l.v[A], ur = r.v[A];
+    // p + 0 = p for every p but -0, whose sound speed is zero either way
+    const double cl = o.root(o.over(g * (stiff ? l.p + pinf : l.p), l.ro));
+    const double cr = o.root(o.over(g * (stiff ? r.p + pinf : r.p), r.ro));
+    const double hl = o.over(UL[4] + l.p, l.ro);
+    const double hr = o.over(UR[4] + r.p, r.ro);
+    const double sl = o.root(rl), sr = o.root(rr);
+    const typename O::Div ss = o.divisor(sl + sr);
+    const double wl = o.over(sl, ss), wr = o.over(sr, ss);
+    double vt[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int b = 0; b < NC; ++b) vt[b] = wl * l.v[b] + wr * r.v[b];
+    const double ut = vt[A];
     const double ht = wl * hl + wr * hr;
-    const double ct = sqrt((g - 1) * (ht - 0.5 * (vtx * vtx + vty * vty + vtz * vtz)));
-    const double SL = fmin(ul - cl, ut - ct);
-    const double SR = fmax(ur + cr, ut + ct);
-    const double lam = fmax(fabs(SL), fabs(SR));
+    const double ct = o.root(ph.gm1 * (ht - o.half(dot<NC>(vt, vt))));
+    const double a0 = ul - cl, a1 = ut - ct, b0 = ur + cr, b1 = ut + ct;
+    const double SL = o.min(a0, a1), SR = o.max(b0, b1);
+    const double lam = o.max(dabs(SL), dabs(SR));
     const double ml = rl * (SL - ul), mr = rr * (SR - ur);
-    const double sstar = (pr - pl + ul * ml - ur * mr) / (ml - mr);
-    if (SL >= 0.0) {
-        phys_flux<A>(ph, UL, flux);
-    } else if (SR <= 0.0) {
-        phys_flux<A>(ph, UR, flux);
-    } else if (sstar >= 0.0) {
-        double F[NV], us[NV];
-        phys_flux<A>(ph, UL, F);
-        const double coef = ml / (SL - sstar);
-        us[0] = coef;
-        us[1] = coef * vlx; us[2] = coef * vly; us[3] = coef * vlz;
-        us[m] = coef * sstar;
-        us[4] = coef * (UL[4] / rl + (sstar - ul) * (sstar + pl / ml));
+    const double sstar = o.div(r.p - l.p + ul * ml - ur * mr, ml - mr);
+    // F_L if S_L >= 0, F_R if S_R <= 0, else the star state on the side of S*
+    const bool supl = o.ge0(SL), supr = !supl && o.le0(SR);
+    const bool left = supl || (!supr && o.ge0(sstar));
+    double U[NV], v[3];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) flux[v] = F[v] + SL * (us[v] - UL[v]);
-    } else {
-        double F[NV], us[NV];
-        phys_flux<A>(ph, UR, F);
-        const double coef = mr / (SR - sstar);
-        us[0] = coef;
-        us[1] = coef * vrx; us[2] = coef * vry; us[3] = coef * vrz;
-        us[m] = coef * sstar;
-        us[4] = coef * (UR[4] / rr + (sstar - ur) * (sstar + pr / mr));
+    for (int i = 0; i < NV; ++i) U[i] = left ? UL[i] : UR[i];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) flux[v] = F[v] + SR * (us[v] - UR[v]);
+    for (int b = 0; b < 3; ++b) v[b] = left ? l.v[b] : r.v[b];
+    const double p = left ? l.p : r.p;
+    const double rvn = U[0] * v[A];
+    flux[0] = rvn;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+        flux[1 + b] = b < NC ? rvn * v[b] : 0.0;
+        if (b == A) flux[1 + b] = flux[1 + b] + p;
+    }
+    flux[4] = v[A] * (U[4] + p);
+    if (!supl && !supr) {
+        const double S = left ? SL : SR, m = left ? ml : mr;
+        const double coef = o.div(m, S - sstar);
+        const double Er = o.over(U[4], left ? l.ro : r.ro);
+        double us[NV];
+        us[0] = coef;
+#pragma unroll
+        for (int b = 0; b < 3; ++b) us[1 + b] = b < NC ? coef * (b == A ? sstar : v[b]) : 0.0;
+        us[4] = coef * (Er + (sstar - v[A]) * (sstar + o.div(p, m)));
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            if (i < 1 + NC || i == 4) flux[i] = flux[i] + S * (us[i] - U[i]);
     }
     return lam;
 }
@@ -663,126 +789,199 @@ __device__ void visc_flux(const PlainBufs& b, const Phys& ph, long long cl, long
     }
 }
 
-// Venkatakrishnan l-function (Limiters.h:102-115).
-// Comparisons of doubles on the integer pipe.  GB300 executes FP64 at about
-// two operations per clock per SM, and half of k_recon's FP64-pipe
-// instructions were comparisons (measured with ncu).  dkey is monotone in the
-// value and gives -0 and +0 the same key, so dkey(a) < dkey(b) is exactly
-// a < b, and the sign tests below are exactly x > 0 and x < 0, for every
-// non-NaN a, b, x (a NaN only arises in a run whose health flags stop it).
-__device__ __forceinline__ long long dkey(double x) {
-    const long long b = __double_as_longlong(x);
-    return b < 0 ? (b ^ 0x7FFFFFFFFFFFFFFFLL) + 1 : b;
-}
-__device__ __forceinline__ bool dlt(double a, double b) { return dkey(a) < dkey(b); }
-__device__ __forceinline__ bool dpos(double x) { return __double_as_longlong(x) > 0; }
-__device__ __forceinline__ bool dneg(double x) {
-    const long long b = __double_as_longlong(x);
-    return b < 0 && b != (long long)0x8000000000000000ULL;
-}
-// |a| < |b|: the magnitudes' bit patterns order like their values
-__device__ __forceinline__ bool dabs_lt(double a, double b) {
-    return (__double_as_longlong(a) & 0x7FFFFFFFFFFFFFFFLL) < (__double_as_longlong(b) & 0x7FFFFFFFFFFFFFFFLL);
-}
-
-__device__ __forceinline__ double venkat(double um, double ui, double d2, double umax, double umin, double eps2) {
-    const double un = 0.5 * (umax - umin);
-    um /= un;
-    ui /= un;
-    d2 /= un;
+// Venkatakrishnan l-function (Limiters.h:102-115): um, ui, d2 already divided
+// by un = (umax - umin) / 2.
+template <class O>
+__device__ __forceinline__ double venkat(double um, double ui, double d2, double eps2, O& o) {
     const double dm = um - ui;
-    return ((dm * dm + eps2) + 2 * d2 * dm) / (dm * dm + 2 * d2 * d2 + dm * d2 + eps2);
+    return o.div((dm * dm + eps2) + 2 * d2 * dm, dm * dm + 2 * d2 * d2 + dm * d2 + eps2);
 }
 
-// Per interior cell: slopes (Linear2PointsStencil.h:147-178 or
-// ENO2PointsStencil.h:202-239) and, for Linear2psLim, the limiter
-// (Linear2psLim.h:305-374, Limiters.h:28-119).
-__global__ void k_recon(PlainBufs b, Phys ph) {
-    if (b.ctl->stop_req) return;
-    const Layout& L = b.L;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= L.nx) return;
-    const int nd = ph.nd;
-    const long long c = L.at(i, j, k);
-    const int ix[3] = {i, j, k};
-    double val[NV], nb[6][NV], g[3][NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) val[v] = b.U[vidx(L, v) + c];
-    for (int a = 0; a < nd; ++a) {
-        const long long st = L.stride(a);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            nb[2 * a][v] = b.U[vidx(L, v) + c - st];
-            nb[2 * a + 1][v] = b.U[vidx(L, v) + c + st];
-        }
-    }
-    for (int a = 0; a < nd; ++a) {
-        const double* X = b.cx[a];
-        const int g0 = (a == 0) ? L.gx : (a == 1 ? L.gy : L.gz);
-        const double xm = X[ix[a] - 1 + g0], xc = X[ix[a] + g0], xp = X[ix[a] + 1 + g0];
-        if (ph.recon == TS_RECON_ENO2_2POINTS) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const double gl = (val[v] - nb[2 * a][v]) / (xc - xm);
-                const double gr = (nb[2 * a + 1][v] - val[v]) / (xp - xc);
-                g[a][v] = dabs_lt(gl, gr) ? gl : gr;
-            }
-        } else {
-            const double d = xp - xm;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) g[a][v] = (nb[2 * a + 1][v] - nb[2 * a][v]) / d;
-        }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) b.G[vidx(L, a * NV + v) + c] = g[a][v];
-    }
-    if (ph.recon != TS_RECON_LINEAR_2POINTS_LIMITED) return;
+// Reconstruction kinds (the limiter choice folded in).
+enum { P_LINEAR = 1, P_ENO2 = 2, P_LIM_BJ = 3, P_LIM_VK = 4 };
 
-    // Projections (SampleSolution(+-h/2) - vals) to the 2*nDim faces.
-    double hcell[3];
-    hcell[0] = b.ch[0][i + L.gx];
-    hcell[1] = b.ch[1][j + L.gy];
-    hcell[2] = b.ch[2][k + L.gz];
-    const double eps2 = b.eps2 ? b.eps2[c] : 0.0;
+// a1 / d1 < a2 / d2 as rounded quotients, for ratios too close for the FP32
+// estimates in recon_var.
+__device__ __noinline__ bool ratio_less(double a1, double d1, double a2, double d2) { return a1 / d1 < a2 / d2; }
+
+// FP32 estimate (truncated, relative error 2^-23) of a positive double with
+// an exponent field in [897, 1150].
+__device__ __forceinline__ float est32(u64 b) { return __uint_as_float((unsigned)(b >> 29) - 0xC0000000u); }
+__device__ __forceinline__ bool est32_ok(u64 b) { return (unsigned)(b >> 52) - 897u < 254u; }
+
+// Slopes (Linear2PointsStencil.h:147-178 or ENO2PointsStencil.h:202-239) and,
+// for Linear2psLim, the limiter (Linear2psLim.h:305-374, Limiters.h:28-119) of
+// variable v in cell c.  d: divisors of the slopes (ENO2: left and right);
+// hs: half cell sizes.  With b.fold the stored value is the projection
+// lim * (slope * h/2) to the high face (its negative goes to the low face),
+// otherwise slope and limiter.
+template <int ND, int KIND, class O>
+__device__ __forceinline__ void recon_var(const PlainBufs& b, int v, long long c, const typename O::Div* d,
+                                          const double* hs, double eps2, O& o) {
+    const Layout& L = b.L;
+    const double* U = b.U + vidx(L, v) + c;
+    const double val = U[0];
+    double nm[ND], np[ND], g[ND], gs[ND];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        double umax = val[v], umin = val[v];
-        long long kmax = dkey(umax), kmin = kmax;
-        for (int f = 0; f < 2 * nd; ++f) {
-            const double vn = nb[f][v];
+    for (int a = 0; a < ND; ++a) {
+        const long long st = L.stride(a);
+        nm[a] = U[-st];
+        np[a] = U[st];
+    }
+    // the largest and smallest of the cell and its neighbours
+    long long kmax = dkey(val), kmin = kmax;
+    double umax = val, umin = val;
+    if (KIND == P_LIM_BJ || KIND == P_LIM_VK) {
+#pragma unroll
+        for (int f = 0; f < 2 * ND; ++f) {
+            const double vn = (f & 1) ? np[f >> 1] : nm[f >> 1];
             const long long kv = dkey(vn);
             if (kmax < kv) { umax = vn; kmax = kv; }
             if (kmin > kv) { umin = vn; kmin = kv; }
         }
-        double lmin = 1.0;
-        if (!dlt(umax - umin, 3.0 * 2.2250738585072014e-308)) {
-            for (int f = 0; f < 2 * nd; ++f) {
-                const int a = f >> 1;
-                const double s = (f & 1) ? 0.5 * hcell[a] : -0.5 * hcell[a];
-                const double d2 = (val[v] + g[a][v] * s) - val[v];
-                double lv = 1.0;
-                if (ph.limiter == TS_LIM_VENKATAKRISHNAN) {
-                    if (dpos(d2)) lv = venkat(umax, val[v], d2, umax, umin, eps2);
-                    if (dneg(d2)) lv = venkat(umin, val[v], d2, umax, umin, eps2);
-                } else {
-                    // r = (umax - u) / d2 (or umin) only matters below 1: where
-                    // the exact quotient is >= 1, the rounded one is too (RN is
-                    // monotone and 1 is representable), so lv = 1 without the
-                    // division, bit for bit
-                    if (dpos(d2)) {
-                        const double a = umax - val[v];
-                        if (dlt(a, d2)) { const double r = a / d2; lv = dlt(r, 1.0) ? r : 1.0; }
-                    }
-                    if (dneg(d2)) {
-                        const double a = umin - val[v];
-                        if (dlt(d2, a)) { const double r = a / d2; lv = dlt(r, 1.0) ? r : 1.0; }
+        // a constant neighbourhood (finite): slopes and projections are zero
+        if (kmax == kmin && (__double2hiint(val) & 0x7FF00000) != 0x7FF00000) {
+#pragma unroll
+            for (int a = 0; a < ND; ++a) b.G[vidx(L, a * NV + v) + c] = 0.0;
+            if (!b.fold) b.Lim[vidx(L, v) + c] = 1.0;
+            return;
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < ND; ++a) {
+        if (KIND == P_ENO2) {
+            const double gl = o.over(val - nm[a], d[2 * a]);
+            const double gr = o.over(np[a] - val, d[2 * a + 1]);
+            g[a] = dabs_lt(gl, gr) ? gl : gr;
+        } else {
+            g[a] = o.over(np[a] - nm[a], d[a]);
+        }
+        gs[a] = g[a] * hs[a];
+    }
+    double lmin = 1.0;
+    if (KIND == P_LIM_BJ || KIND == P_LIM_VK) {
+        // umax - umin < 3 DBL_MIN: for unequal values of magnitude 2^-960 or
+        // more the difference is larger, no subtraction needed
+        const bool big = ((__double2hiint(umax) & 0x7FF00000) >= 0x03F00000) ||
+                         ((__double2hiint(umin) & 0x7FF00000) >= 0x03F00000);
+        const bool flat = kmax == kmin || (!big && dlt(umax - umin, 3.0 * 2.2250738585072014e-308));
+        if (!flat) {
+            // differences (SampleSolution(+-h/2) - val) to the 2 ND faces
+            const double am = umax - val, an = umin - val;
+            if constexpr (KIND == P_LIM_VK) {
+                const typename O::Div un = o.divisor(o.half(umax - umin));
+                const double xm = o.over(umax, un), xn = o.over(umin, un), xu = o.over(val, un);
+#pragma unroll
+                for (int f = 0; f < 2 * ND; ++f) {
+                    const double s = (f & 1) ? gs[f >> 1] : -gs[f >> 1];
+                    const double d2 = (val + s) - val;
+                    if (dzero(d2)) continue;
+                    const double lv = venkat(dpos(d2) ? xm : xn, xu, o.over(d2, un), eps2, o);
+                    if (o.lt(lv, lmin)) lmin = lv;
+                }
+            } else if constexpr (std::is_same_v<O, Plain>) {
+#pragma unroll
+                for (int f = 0; f < 2 * ND; ++f) {
+                    const double s = (f & 1) ? gs[f >> 1] : -gs[f >> 1];
+                    const double d2 = (val + s) - val;
+                    double lv = 1.0;
+                    if (d2 > 0) { const double r = am / d2; lv = r < 1.0 ? r : 1.0; }
+                    if (d2 < 0) { const double r = an / d2; lv = r < 1.0 ? r : 1.0; }
+                    if (lv < lmin) lmin = lv;
+                }
+            } else {
+                // The limiter is the smallest of the rounded ratios a / d2
+                // (a = umax - val or umin - val) below 1.  Rounding is
+                // monotone, so only the smallest ratio is divided out: it is
+                // found on FP32 estimates (error < 2^-20), and estimates
+                // closer than 2^-18 are settled by their quotients.  A ratio
+                // with |a| >= |d2| rounds to 1 or more and is dropped.
+                const u64 ap = (u64)__double_as_longlong(am), aq = (u64)__double_as_longlong(dabs(an));
+                u64 ba = 0, bd = 0;
+                float br = 2.0f;
+#pragma unroll
+                for (int f = 0; f < 2 * ND; ++f) {
+                    const double s = (f & 1) ? gs[f >> 1] : -gs[f >> 1];
+                    const double d2 = (val + s) - val;
+                    const u64 ad = (u64)__double_as_longlong(dabs(d2));
+                    const u64 aa = __double2hiint(d2) < 0 ? aq : ap;
+                    if (aa < ad) {
+                        o.bad |= !est32_ok(ad);
+                        const float r = est32_ok(aa) ? __fdividef(est32(aa), est32(ad)) : 0.0f;
+                        bool take = r < br * (1.0f - 3.8e-6f);
+                        // (a zero or the same ratio cannot be undercut: local extrema,
+                        // and states that differ by a few ulps)
+                        if (!take && r <= br * (1.0f + 3.8e-6f) && ba != 0 && !(aa == ba && ad == bd))
+                            take = ratio_less(__longlong_as_double(aa), __longlong_as_double(ad),
+                                              __longlong_as_double(ba), __longlong_as_double(bd));
+                        if (take) { ba = aa; bd = ad; br = r; }
                     }
                 }
-                if (dlt(lv, lmin)) lmin = lv;
+                if (br < 2.0f) lmin = o.div(__longlong_as_double(ba), __longlong_as_double(bd));
             }
         }
-        b.Lim[vidx(L, v) + c] = lmin;
     }
+    if (b.fold) {
+#pragma unroll
+        for (int a = 0; a < ND; ++a)
+            b.G[vidx(L, a * NV + v) + c] = (KIND == P_LIM_BJ || KIND == P_LIM_VK) ? lmin * gs[a] : gs[a];
+    } else {
+#pragma unroll
+        for (int a = 0; a < ND; ++a) b.G[vidx(L, a * NV + v) + c] = g[a];
+        if (KIND == P_LIM_BJ || KIND == P_LIM_VK) b.Lim[vidx(L, v) + c] = lmin;
+    }
+}
+
+template <int ND, int KIND, class O>
+__device__ __forceinline__ void recon_cell(const PlainBufs& b, int i, int j, int k, O& o) {
+    const Layout& L = b.L;
+    const long long c = L.at(i, j, k);
+    const int ix[3] = {i, j, k};
+    typename O::Div d[KIND == P_ENO2 ? 2 * ND : ND];
+    double hs[ND];
+#pragma unroll
+    for (int a = 0; a < ND; ++a) {
+        const int at = ix[a] + (a == 0 ? L.gx : (a == 1 ? L.gy : L.gz));
+        const double* X = b.cx[a];
+        if (KIND == P_ENO2) {
+            d[2 * a] = o.divisor(X[at] - X[at - 1]);
+            d[2 * a + 1] = o.divisor(X[at + 1] - X[at]);
+        } else {
+            d[a] = o.divisor(X[at + 1] - X[at - 1]);
+        }
+        hs[a] = o.half(b.ch[a][at]);
+    }
+    const double eps2 = KIND == P_LIM_VK ? b.eps2[c] : 0.0;
+#pragma unroll 1
+    for (int v = 0; v < NV; ++v) recon_var<ND, KIND, O>(b, v, c, d, hs, eps2, o);
+}
+
+template <int ND, int KIND>
+__device__ __noinline__ void recon_plain(const PlainBufs& b, int i, int j, int k) {
+    Plain o;
+    recon_cell<ND, KIND, Plain>(b, i, j, k, o);
+}
+
+// Cell t of the interior in storage order (one flat index over all rows: no
+// warp holds the end of a row alone).
+__device__ __forceinline__ void cell_of(const Layout& L, unsigned t, int& i, int& j, int& k) {
+    const unsigned row = t / (unsigned)L.nx;
+    i = (int)(t - row * (unsigned)L.nx);
+    k = (int)(row / (unsigned)L.ny);
+    j = (int)(row - (unsigned)k * (unsigned)L.ny);
+}
+
+// Per interior cell: slopes and limiter (ComputeSolutionReconstruction).
+template <int ND, int KIND>
+__global__ void __launch_bounds__(kPlainBlock) k_recon(const __grid_constant__ PlainBufs b) {
+    if (b.ctl->stop_req) return;
+    const unsigned t = blockIdx.x * kPlainBlock + threadIdx.x;
+    if (t >= (unsigned)b.L.cells()) return;
+    int i, j, k;
+    cell_of(b.L, t, i, j, k);
+    Fast o;
+    recon_cell<ND, KIND, Fast>(b, i, j, k, o);
+    if (o.bad) recon_plain<ND, KIND>(b, i, j, k);
 }
 
 __device__ __forceinline__ double face_area(const PlainBufs& b, int nd, int a, int i, int j, int k) {
@@ -793,13 +992,25 @@ __device__ __forceinline__ double face_area(const PlainBufs& b, int nd, int a, i
     return hx * hy;
 }
 
-// Face-centred sample of a cell's reconstruction (SampleSolution).
-__device__ __forceinline__ void sample(const PlainBufs& b, const Phys& ph, long long c, int a, double s,
+// Face-centred sample of a cell's reconstruction (SampleSolution) at its high
+// (HI) or low face along axis a; h is the cell size the reference samples
+// with.
+template <bool HI>
+__device__ __forceinline__ void sample(const PlainBufs& b, const Phys& ph, long long c, int a, double h,
                                        double out[NV]) {
     const Layout& L = b.L;
 #pragma unroll
     for (int v = 0; v < NV; ++v) out[v] = b.U[vidx(L, v) + c];
     if (ph.recon == TS_RECON_PIECEWISE_CONSTANT) return;
+    if (b.fold) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const double d = b.G[vidx(L, a * NV + v) + c];
+            out[v] = HI ? out[v] + d : out[v] - d;
+        }
+        return;
+    }
+    const double s = (HI ? 0.5 : -0.5) * h;
     if (ph.recon == TS_RECON_LINEAR_2POINTS_LIMITED) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) out[v] = out[v] + b.Lim[vidx(L, v) + c] * (b.G[vidx(L, a * NV + v) + c] * s);
@@ -809,28 +1020,57 @@ __device__ __forceinline__ void sample(const PlainBufs& b, const Phys& ph, long 
     }
 }
 
+// The Riemann flux and eigenvalue of one face.  1D and 2D problems whose
+// transverse momentum is zero in every state of the warp take the instance
+// without its terms.
+template <int A, int SOLVER, int NC, class O>
+__device__ __forceinline__ double riemann(const Phys& ph, const double UL[NV], const double UR[NV], double F[NV], O& o) {
+    if (SOLVER == TS_RS_HLLC) return hllc_flux<A, NC, O>(ph, UL, UR, F, o);
+    return roe_flux<A, NC, O>(ph, UL, UR, F, o);
+}
+
+template <int A, int SOLVER>
+__device__ __noinline__ double riemann_plain(const Phys& ph, const double* UL, const double* UR, double* F) {
+    Plain o;
+    return riemann<A, SOLVER, 3, Plain>(ph, UL, UR, F, o);
+}
+
+template <int A, int ND, int SOLVER>
+__device__ __forceinline__ double face_flux(const Phys& ph, const double UL[NV], const double UR[NV], double F[NV]) {
+    Fast o;
+    double lam;
+    bool z = false;
+    if (ND < 3) {
+        bool mine = true;
+#pragma unroll
+        for (int b = ND; b < 3; ++b) mine = mine && dzero(UL[1 + b]) && dzero(UR[1 + b]);
+        z = __all_sync(__activemask(), mine);
+    }
+    if (ND < 3 && z) lam = riemann<A, SOLVER, ND, Fast>(ph, UL, UR, F, o);
+    else lam = riemann<A, SOLVER, 3, Fast>(ph, UL, UR, F, o);
+    if (o.bad) {
+        double l[NV], r[NV], f[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) { l[v] = UL[v]; r[v] = UR[v]; }
+        lam = riemann_plain<A, SOLVER>(ph, l, r, f);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) F[v] = f[v];
+    }
+    return lam;
+}
+
 // One face per thread along axis A; faces are stored at their right cell.
-template <int A>
-__global__ void k_flux(PlainBufs b, Phys ph) {
+template <int A, int ND, int SOLVER>
+__global__ void __launch_bounds__(kPlainBlock) k_flux(const __grid_constant__ PlainBufs b,
+                                                      const __grid_constant__ Phys ph) {
     if (b.ctl->stop_req) return;
     const Layout& L = b.L;
-    int i, j, k;
-    if (A == 0) {
-        // nx + 1 faces per row: one flat index over all rows, so that no
-        // block holds a row's last face alone
-        const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-        const long long row = L.nx + 1;
-        if (t >= row * L.ny * L.nz) return;
-        i = (int)(t % row);
-        const long long r = t / row;
-        j = (int)(r % L.ny);
-        k = (int)(r / L.ny);
-    } else {
-        i = blockIdx.x * blockDim.x + threadIdx.x;
-        j = blockIdx.y;
-        k = blockIdx.z;
-        if (i >= L.nx) return;
-    }
+    // one flat index over the faces of all rows
+    const unsigned t = blockIdx.x * kPlainBlock + threadIdx.x;
+    const unsigned mx = L.nx + (A == 0), my = L.ny + (A == 1), mz = L.nz + (A == 2);
+    const unsigned row = t / mx;
+    const int i = (int)(t - row * mx), k = (int)(row / my), j = (int)(row - (unsigned)k * my);
+    if (k >= (int)mz) return;
     const int s = (A == 0) ? i : (A == 1 ? j : k);
     const int n = L.n(A);
     const long long st = L.stride(A);
@@ -839,27 +1079,27 @@ __global__ void k_flux(PlainBufs b, Phys ph) {
     const int g0 = (A == 0) ? L.gx : (A == 1 ? L.gy : L.gz);
     double UL[NV], UR[NV];
     if (s == 0 && !ph.periodic[A]) {
-        sample(b, ph, cf, A, -0.5 * H[s + g0], UR);
+        sample<false>(b, ph, cf, A, H[s + g0], UR);
         bc_values(ph, bc_id(ph.bc.mark, 2 * A, face_index(2 * A, i, j, k, L.nx, L.ny)), A, 1.0, UR, UL);
     } else if (s == n && !ph.periodic[A]) {
-        sample(b, ph, cf - st, A, 0.5 * H[s - 1 + g0], UL);
+        sample<true>(b, ph, cf - st, A, H[s - 1 + g0], UL);
         bc_values(ph, bc_id(ph.bc.mark, 2 * A + 1, face_index(2 * A + 1, i, j, k, L.nx, L.ny)), A, 1.0, UL, UR);
     } else {
         // A ghost reconstruction on a periodic axis is the opposite interior
         // cell's object sampled with the ghost's own h (ExchangeReconstructions).
         const long long cl = (s == 0) ? cf + (long long)(n - 1) * st : cf - st;
         const long long cr = (s == n) ? cf - (long long)n * st : cf;
-        sample(b, ph, cl, A, 0.5 * H[s - 1 + g0], UL);
-        sample(b, ph, cr, A, -0.5 * H[s + g0], UR);
+        sample<true>(b, ph, cl, A, H[s - 1 + g0], UL);
+        sample<false>(b, ph, cr, A, H[s + g0], UR);
     }
     double F[NV];
     double lam;
-    if (ph.solver == TS_RS_GODUNOV) {
+    if (SOLVER == TS_RS_GODUNOV) {
         bool ok;
         lam = godunov_flux<A>(ph, UL, UR, F, ok);
         if (!ok) atomicOr(&b.ctl->health, (unsigned)TS_HEALTH_RIEMANN);
     } else {
-        lam = (ph.solver == TS_RS_HLLC) ? hllc_flux<A>(ph, UL, UR, F) : roe_flux<A>(ph, UL, UR, F);
+        lam = face_flux<A, ND, SOLVER>(ph, UL, UR, F);
     }
     // viscous flux subtracted from the convective one (ExplicitRungeKuttaFVM.h:1220-1222);
     // the cell values and gradients of the ghost cells serve the domain faces
@@ -889,150 +1129,244 @@ __global__ void k_flux(PlainBufs b, Phys ph) {
     }
 }
 
-__device__ __forceinline__ double warp_min(double v) {
+// Minimum of the warp's values of V/SR.  They are not negative (a NaN of
+// either sign has a larger pattern than +inf), so they order like their bits.
+__device__ __forceinline__ u64 umin64(u64 a, u64 b) { return a < b ? a : b; }
+__device__ __forceinline__ u64 warp_min(u64 v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = umin64(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
+constexpr u64 kInfBits = 0x7FF0000000000000ULL;
 
+// Bits of V / sr.
+__device__ __forceinline__ u64 ratio_bits(double V, double sr) {
+    bool bad = false;
+    double r = x64::div(V, sr, bad);
+    if (bad) r = V / sr;
+    return (u64)__double_as_longlong(r);
+}
 
 // Spectral radius per cell in the reference's accumulation order (x-left,
 // x-right, y-left, ...), V/SR, block min by warp shuffles; the high-side
 // ghost cells, whose SR is their single face term, join the min.  The last
 // block to finish reduces the block minima and sets dt.
-__global__ void k_dt(PlainBufs b, Phys ph) {
+template <int ND>
+__global__ void __launch_bounds__(kPlainBlock) k_dt(const __grid_constant__ PlainBufs b,
+                                                    const __grid_constant__ Phys ph) {
     if (b.ctl->stop_req) return;
     const Layout& L = b.L;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    const int nd = ph.nd;
-    double r = __longlong_as_double(0x7ff0000000000000LL);  // +inf
-    if (i < L.nx) {
+    const unsigned cells = (unsigned)L.cells(), step = gridDim.x * kPlainBlock;
+    u64 r = kInfBits;
+    for (unsigned t = blockIdx.x * kPlainBlock + threadIdx.x; t < cells; t += step) {
+        int i, j, k;
+        cell_of(L, t, i, j, k);
         const long long c = L.at(i, j, k);
         const double hx = b.ch[0][i + L.gx], hy = b.ch[1][j + L.gy], hz = b.ch[2][k + L.gz];
         const double V = hx * hy * hz;
         double sr = 0.0;
         const int ix[3] = {i, j, k};
-        for (int a = 0; a < nd; ++a) {
-            const double fS = face_area(b, nd, a, i, j, k);
+#pragma unroll
+        for (int a = 0; a < ND; ++a) {
+            const double fS = face_area(b, ND, a, i, j, k);
             const long long st = L.stride(a);
-            sr += fS * b.Lam[a][c];
-            sr += fS * b.Lam[a][c + st];
+            const double lo = fS * b.Lam[a][c], hi = fS * b.Lam[a][c + st];
+            sr = a == 0 ? lo : sr + lo;
+            sr += hi;
             if (ph.visc != 0.0) sr += b.VSR[a][c + st];
             if (ix[a] == L.n(a) - 1) {
                 double hg[3] = {hx, hy, hz};
                 hg[a] = b.ch[a][L.n(a) + (a == 0 ? L.gx : (a == 1 ? L.gy : L.gz))];
-                const double Vg = hg[0] * hg[1] * hg[2];
-                r = fmin(r, Vg / (fS * b.Lam[a][c + st]));
+                r = umin64(r, ratio_bits(hg[0] * hg[1] * hg[2], hi));
             }
         }
-        r = fmin(r, V / sr);
+        r = umin64(r, ratio_bits(V, sr));
+        if (step > cells - t) break;  // t + step would not fit 32 bits for the largest grids
     }
-    __shared__ double wmin[32];
+    __shared__ u64 wmin[kPlainBlock / 32];
     r = warp_min(r);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0) wmin[wid] = r;
     __syncthreads();
-    const int nblk = gridDim.x * gridDim.y * gridDim.z;
-    const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    const int nblk = gridDim.x;
     __shared__ bool last;
     if (threadIdx.x == 0) {
-        double m = wmin[0];
-        for (int w = 1; w < (int)(blockDim.x + 31) / 32; ++w) m = fmin(m, wmin[w]);
-        b.partial[bid] = m;
+        u64 m = wmin[0];
+        for (int w = 1; w < kPlainBlock / 32; ++w) m = umin64(m, wmin[w]);
+        b.partial[blockIdx.x] = __longlong_as_double((long long)m);
         __threadfence();
         last = (atomicAdd(&b.ctl->blocks_done, 1u) == (unsigned)(nblk - 1));
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    double m = __longlong_as_double(0x7ff0000000000000LL);
-    for (int t = threadIdx.x; t < nblk; t += blockDim.x) m = fmin(m, ((volatile double*)b.partial)[t]);
+    u64 m = kInfBits;
+    for (int t = threadIdx.x; t < nblk; t += kPlainBlock)
+        m = umin64(m, (u64)__double_as_longlong(((volatile double*)b.partial)[t]));
     m = warp_min(m);
     if (lane == 0) wmin[wid] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
         m = wmin[0];
-        for (int w = 1; w < (int)(blockDim.x + 31) / 32; ++w) m = fmin(m, wmin[w]);
+        for (int w = 1; w < kPlainBlock / 32; ++w) m = umin64(m, wmin[w]);
+        const double least = __longlong_as_double((long long)m);
         Ctl* ctl = b.ctl;
-        double dt = m * ph.cfl;
+        double dt = least * ph.cfl;
         if ((ctl->save_sol > 0) && (ctl->next_sol < ctl->time + dt)) dt = ctl->next_sol - ctl->time;
         if ((ctl->save_slice > 0) && (ctl->next_slice < ctl->time + dt)) dt = ctl->next_slice - ctl->time;
-        ctl->dt_min_raw = m;
+        ctl->dt_min_raw = least;
         ctl->dt = dt;
         for (int v = 0; v < NV; ++v) ctl->res[v] = 0.0;
         ctl->blocks_done = 0;
     }
 }
 
+// Health flags of an updated state.  The pressure test is settled in FP32
+// where the pressure is a thousandth of the energy or more (the FP32 estimate
+// is off by 1e-6 of the energy), and formed in FP64 otherwise.
+__device__ __noinline__ unsigned int health_plain(const Phys& ph, double u0, double u1, double u2, double u3,
+                                                  double u4) {
+    unsigned int health = 0;
+    const double ke = 0.5 * (u1 * u1 + u2 * u2 + u3 * u3) / u0;
+    const double p = pressure(ph, u0, 0.0, 0.0, 0.0, u4 - ke);
+    if (!(u0 == u0) || !(u4 == u4) || !(p == p)) health |= TS_HEALTH_NAN;
+    if (u0 <= 0.0) health |= TS_HEALTH_NEG_DENSITY;
+    if (p <= 0.0 && ph.eos == TS_EOS_IDEAL_GAS) health |= TS_HEALTH_NEG_PRESSURE;
+    if (ph.eos == TS_EOS_STIFFENED_GAS && p + ph.p_inf <= 0.0) health |= TS_HEALTH_NEG_PRESSURE;
+    return health;
+}
+// FP32 estimate of a double of either sign; false outside the normal range
+// (zero gives 0).
+__device__ __forceinline__ bool est32_signed(double x, float& f) {
+    const u64 b = (u64)__double_as_longlong(dabs(x));
+    f = est32(b);
+    if (__double2hiint(x) < 0) f = -f;
+    if (b < ((u64)897 << 52)) { f = 0.0f; return true; }  // below 2^-126: nothing beside the energy's tolerance
+    return est32_ok(b);
+}
+__device__ __forceinline__ unsigned int health_of(const Phys& ph, const double u[NV]) {
+    float r, m1, m2, m3, e;
+    bool ok = est32_signed(u[0], r);
+    ok = est32_signed(u[1], m1) && ok;
+    ok = est32_signed(u[2], m2) && ok;
+    ok = est32_signed(u[3], m3) && ok;
+    ok = est32_signed(u[4], e) && ok;
+    // p + p_inf = (g - 1) (E - kinetic - p_inf) for both equations of state
+    const float pr = e - 0.5f * (m1 * m1 + m2 * m2 + m3 * m3) / r - (float)ph.p_inf;
+    if (ok && r > 1e-30f && pr > 1e-3f * e && e > 1e-30f && pr < 1e37f) return 0u;
+    return health_plain(ph, u[0], u[1], u[2], u[3], u[4]);
+}
+
+// U + dt (R / V) of one cell's variables; F = the face fluxes.
+template <int ND, class O>
+__device__ __forceinline__ void update_cell(const PlainBufs& b, const Phys& ph, int i, int j, int k, double dt,
+                                            double u[NV], double nrm[NV], O& o) {
+    const Layout& L = b.L;
+    const long long c = L.at(i, j, k);
+    const double hx = b.ch[0][i + L.gx], hy = b.ch[1][j + L.gy], hz = b.ch[2][k + L.gz];
+    const double V = hx * hy * hz;
+    double R[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) R[v] = 0.0;
+#pragma unroll
+    for (int a = 0; a < ND; ++a) {
+        const double fS = face_area(b, ND, a, i, j, k);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const double* F = b.F[a] + vidx(L, v) + c;
+            const double fh = F[L.stride(a)], fl = F[0];
+            // equal (finite) fluxes: the difference is a zero
+            if (__double_as_longlong(fh) == __double_as_longlong(fl) && (__double2hiint(fh) & 0x7FF00000) != 0x7FF00000)
+                continue;
+            const double d = (fh - fl) * fS;
+            R[v] = a == 0 ? dneg_of(d) : R[v] - d;
+        }
+    }
+    double uo[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) uo[v] = b.U[vidx(L, v) + c];
+    // source terms after the face fluxes (ExplicitRungeKuttaFVM.h:1421-1423;
+    // ProcessExternalForces and ProcessExternalAcceleration, kernel.h:941-989)
+    if (ph.force || ph.accel) {
+        const typename O::Div ro = o.divisor(uo[0]);
+        const double vu = o.over(uo[1], ro), vv = o.over(uo[2], ro), vw = o.over(uo[3], ro);
+        if (ph.force) {
+            R[1] += V * ph.sigma[0];
+            R[2] += V * ph.sigma[1];
+            R[3] += V * ph.sigma[2];
+            R[4] += (ph.sigma[0] * vu + ph.sigma[1] * vv + ph.sigma[2] * vw) * V;
+        }
+        if (ph.accel) {
+            const double r0 = uo[0];
+            R[1] += r0 * V * ph.g[0];
+            R[2] += r0 * V * ph.g[1];
+            R[3] += r0 * V * ph.g[2];
+            R[4] += ((r0 * ph.g[0]) * vu + (r0 * ph.g[1]) * vv + (r0 * ph.g[2]) * vw) * V;
+        }
+    }
+    const typename O::Div iv = o.divisor(V);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        u[v] = uo[v];
+        nrm[v] = 0.0;
+        if (dzero(R[v])) continue;
+        u[v] = uo[v] + dt * o.over(R[v], iv);
+        nrm[v] = V * dabs(R[v]);
+    }
+}
+template <int ND>
+__device__ __noinline__ void update_plain(const PlainBufs& b, const Phys& ph, int i, int j, int k, double dt,
+                                          double* u, double* nrm) {
+    Plain o;
+    update_cell<ND, Plain>(b, ph, i, j, k, dt, u, nrm, o);
+}
+
 // Residual R = -sum_a (F_{a,+} - F_{a,-}) fS_a accumulated from zero in the
 // reference's direction order, then U += dt*(R/V); residual norms and health.
-__global__ void k_update(PlainBufs b, Phys ph) {
+// The last block closes the step: time += dt, iteration++ (IterationStep
+// :1486-1487); under Run also the snapshot-time bookkeeping and termination
+// test (kernel.h:1763-1846).
+template <int ND>
+__global__ void __launch_bounds__(kPlainBlock) k_update(const __grid_constant__ PlainBufs b,
+                                                        const __grid_constant__ Phys ph) {
     if (b.ctl->stop_req) return;
     const Layout& L = b.L;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    const int nd = ph.nd;
-    double nrm[NV] = {0, 0, 0, 0, 0};
+    const unsigned cells = (unsigned)L.cells(), step = gridDim.x * kPlainBlock;
+    const double dt = b.ctl->dt;
+    double sum[NV] = {0, 0, 0, 0, 0};
     unsigned int health = 0;
-    if (i < L.nx) {
+    for (unsigned t = blockIdx.x * kPlainBlock + threadIdx.x; t < cells; t += step) {
+        int i, j, k;
+        cell_of(L, t, i, j, k);
         const long long c = L.at(i, j, k);
-        const double hx = b.ch[0][i + L.gx], hy = b.ch[1][j + L.gy], hz = b.ch[2][k + L.gz];
-        const double V = hx * hy * hz;
-        const double dt = b.ctl->dt;
-        double R[NV] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        for (int a = 0; a < nd; ++a) {
-            const double fS = face_area(b, nd, a, i, j, k);
-            const long long st = L.stride(a);
+        double u[NV], nrm[NV];
+        Fast o;
+        update_cell<ND, Fast>(b, ph, i, j, k, dt, u, nrm, o);
+        if (o.bad) {
+            double w[NV], m[NV];
+            update_plain<ND>(b, ph, i, j, k, dt, w, m);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const double* F = b.F[a] + vidx(L, v);
-                R[v] -= (F[c + st] - F[c]) * fS;
-            }
-        }
-        double uo[NV], u[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) uo[v] = b.U[vidx(L, v) + c];
-        // source terms after the face fluxes (ExplicitRungeKuttaFVM.h:1421-1423;
-        // ProcessExternalForces and ProcessExternalAcceleration, kernel.h:941-989)
-        if (ph.force || ph.accel) {
-            const double vu = uo[1] / uo[0], vv = uo[2] / uo[0], vw = uo[3] / uo[0];
-            if (ph.force) {
-                R[1] += V * ph.sigma[0];
-                R[2] += V * ph.sigma[1];
-                R[3] += V * ph.sigma[2];
-                R[4] += (ph.sigma[0] * vu + ph.sigma[1] * vv + ph.sigma[2] * vw) * V;
-            }
-            if (ph.accel) {
-                const double ro = uo[0];
-                R[1] += ro * V * ph.g[0];
-                R[2] += ro * V * ph.g[1];
-                R[3] += ro * V * ph.g[2];
-                R[4] += ((ro * ph.g[0]) * vu + (ro * ph.g[1]) * vv + (ro * ph.g[2]) * vw) * V;
-            }
+            for (int v = 0; v < NV; ++v) { u[v] = w[v]; nrm[v] = m[v]; }
         }
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            u[v] = uo[v] + dt * (R[v] / V);
             b.U[vidx(L, v) + c] = u[v];
-            nrm[v] = V * fabs(R[v]);
+            if (!dzero(nrm[v])) sum[v] += nrm[v];
         }
-        const double ke = 0.5 * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) / u[0];
-        const double p = pressure(ph, u[0], 0.0, 0.0, 0.0, u[4] - ke);
-        if (!(u[0] == u[0]) || !(u[4] == u[4]) || !(p == p)) health |= TS_HEALTH_NAN;
-        if (u[0] <= 0.0) health |= TS_HEALTH_NEG_DENSITY;
-        if (p <= 0.0 && ph.eos == TS_EOS_IDEAL_GAS) health |= TS_HEALTH_NEG_PRESSURE;
-        if (ph.eos == TS_EOS_STIFFENED_GAS && p + ph.p_inf <= 0.0) health |= TS_HEALTH_NEG_PRESSURE;
+        health |= health_of(ph, u);
+        if (step > cells - t) break;
     }
     // block sums of the diagnostic norms (accumulation order differs from the
     // reference's serial sum; the norms are reported, never fed back)
-    __shared__ double red[NV][32];
+    __shared__ double red[NV][kPlainBlock / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        double s = nrm[v];
+        double s = sum[v];
+        if (__any_sync(0xffffffffu, !dzero(s))) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        }
         if (lane == 0) red[v][wid] = s;
     }
     health = __reduce_or_sync(0xffffffffu, health);
@@ -1040,28 +1374,54 @@ __global__ void k_update(PlainBufs b, Phys ph) {
     __syncthreads();
     if (threadIdx.x < NV) {
         double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) s += red[threadIdx.x][w];
-        atomicAdd(&b.ctl->res[threadIdx.x], s);
+        for (int w = 0; w < kPlainBlock / 32; ++w) s += red[threadIdx.x][w];
+        if (!dzero(s)) atomicAdd(&b.ctl->res[threadIdx.x], s);
+        __threadfence();
     }
-}
-
-// time += dt, iteration++ (IterationStep :1486-1487); under Run also the
-// snapshot-time bookkeeping and termination test (kernel.h:1763-1846).
-__global__ void k_finish(Ctl* ctl) {
-    if (ctl->stop_req) return;
-    ctl->time += ctl->dt;
-    ctl->iteration += 1;
-    if (!ctl->run_mode) return;
-    if ((ctl->save_sol > 0) && (ctl->next_sol == ctl->time)) ctl->next_sol += ctl->save_sol;
-    if ((ctl->save_slice > 0) && (ctl->next_slice == ctl->time)) ctl->next_slice += ctl->save_slice;
-    if (ctl->iteration == ctl->max_iteration || ctl->time >= ctl->max_time) ctl->stop_req = 1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        Ctl* ctl = b.ctl;
+        __threadfence();
+        if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
+            ctl->blocks_done = 0;
+            ctl->time += ctl->dt;
+            ctl->iteration += 1;
+            if (ctl->run_mode) {
+                if ((ctl->save_sol > 0) && (ctl->next_sol == ctl->time)) ctl->next_sol += ctl->save_sol;
+                if ((ctl->save_slice > 0) && (ctl->next_slice == ctl->time)) ctl->next_slice += ctl->save_slice;
+                if (ctl->iteration == ctl->max_iteration || ctl->time >= ctl->max_time) ctl->stop_req = 1;
+            }
+        }
+    }
 }
 
 }  // namespace
 
-int plain_partial_blocks(const Layout& L) {
-    const int bx = (L.nx + kPlainBlock - 1) / kPlainBlock;
-    return bx * L.ny * L.nz;
+// Blocks of k_dt and k_update: each thread takes several cells of a large
+// grid, so that the block's closing reductions are a small part of its work.
+static unsigned reduce_blocks(const Layout& L) {
+    const long long full = (L.cells() + kPlainBlock - 1) / kPlainBlock;
+    return (unsigned)std::min<long long>(full, kPlainReduceBlocks);
+}
+
+int plain_partial_blocks(const Layout& L) { return (int)reduce_blocks(L); }
+
+template <int ND>
+static void launch_recon(const PlainBufs& b, const Phys& ph, unsigned blocks, cudaStream_t st) {
+    if (ph.recon == TS_RECON_LINEAR_2POINTS) k_recon<ND, P_LINEAR><<<blocks, kPlainBlock, 0, st>>>(b);
+    else if (ph.recon == TS_RECON_ENO2_2POINTS) k_recon<ND, P_ENO2><<<blocks, kPlainBlock, 0, st>>>(b);
+    else if (ph.limiter == TS_LIM_VENKATAKRISHNAN) k_recon<ND, P_LIM_VK><<<blocks, kPlainBlock, 0, st>>>(b);
+    else k_recon<ND, P_LIM_BJ><<<blocks, kPlainBlock, 0, st>>>(b);
+}
+
+template <int A, int ND>
+static void launch_flux(const PlainBufs& b, const Phys& ph, cudaStream_t st) {
+    const Layout& L = b.L;
+    const long long faces = (long long)(L.nx + (A == 0)) * (L.ny + (A == 1)) * (L.nz + (A == 2));
+    const unsigned blocks = (unsigned)((faces + kPlainBlock - 1) / kPlainBlock);
+    if (ph.solver == TS_RS_GODUNOV) k_flux<A, ND, TS_RS_GODUNOV><<<blocks, kPlainBlock, 0, st>>>(b, ph);
+    else if (ph.solver == TS_RS_HLLC) k_flux<A, ND, TS_RS_HLLC><<<blocks, kPlainBlock, 0, st>>>(b, ph);
+    else k_flux<A, ND, TS_RS_ROE_PIKE><<<blocks, kPlainBlock, 0, st>>>(b, ph);
 }
 
 cudaError_t plain_step(const PlainBufs& b, const Phys& ph, cudaStream_t st, cudaEvent_t* ev, int* n_launch,
@@ -1093,18 +1453,30 @@ cudaError_t plain_step(const PlainBufs& b, const Phys& ph, cudaStream_t st, cuda
         if (ph.nd > 1) { k_vgrad_bc<1><<<ghost_grid(1), blk, 0, st>>>(b, ph); mark("k_vgrad_bc_y"); }
         if (ph.nd > 2) { k_vgrad_bc<2><<<ghost_grid(2), blk, 0, st>>>(b, ph); mark("k_vgrad_bc_z"); }
     }
-    if (ph.recon != TS_RECON_PIECEWISE_CONSTANT) { k_recon<<<cells, blk, 0, st>>>(b, ph); mark("k_recon"); }
-    const long long xfaces = (long long)(L.nx + 1) * L.ny * L.nz;
-    k_flux<0><<<dim3((unsigned)((xfaces + kPlainBlock - 1) / kPlainBlock)), blk, 0, st>>>(b, ph);
+    if (ph.recon != TS_RECON_PIECEWISE_CONSTANT) {
+        const unsigned blocks = (unsigned)((L.cells() + kPlainBlock - 1) / kPlainBlock);
+        if (ph.nd == 3) launch_recon<3>(b, ph, blocks, st);
+        else if (ph.nd == 2) launch_recon<2>(b, ph, blocks, st);
+        else launch_recon<1>(b, ph, blocks, st);
+        mark("k_recon");
+    }
+    if (ph.nd == 3) launch_flux<0, 3>(b, ph, st);
+    else if (ph.nd == 2) launch_flux<0, 2>(b, ph, st);
+    else launch_flux<0, 1>(b, ph, st);
     mark("k_flux_x");
-    if (ph.nd > 1) { k_flux<1><<<dim3(cells.x, L.ny + 1, L.nz), blk, 0, st>>>(b, ph); mark("k_flux_y"); }
-    if (ph.nd > 2) { k_flux<2><<<dim3(cells.x, L.ny, L.nz + 1), blk, 0, st>>>(b, ph); mark("k_flux_z"); }
-    k_dt<<<cells, blk, 0, st>>>(b, ph);
+    if (ph.nd == 3) launch_flux<1, 3>(b, ph, st);
+    else if (ph.nd == 2) launch_flux<1, 2>(b, ph, st);
+    if (ph.nd > 1) mark("k_flux_y");
+    if (ph.nd > 2) { launch_flux<2, 3>(b, ph, st); mark("k_flux_z"); }
+    const unsigned rb = reduce_blocks(L);
+    if (ph.nd == 3) k_dt<3><<<rb, blk, 0, st>>>(b, ph);
+    else if (ph.nd == 2) k_dt<2><<<rb, blk, 0, st>>>(b, ph);
+    else k_dt<1><<<rb, blk, 0, st>>>(b, ph);
     mark("k_dt");
-    k_update<<<cells, blk, 0, st>>>(b, ph);
+    if (ph.nd == 3) k_update<3><<<rb, blk, 0, st>>>(b, ph);
+    else if (ph.nd == 2) k_update<2><<<rb, blk, 0, st>>>(b, ph);
+    else k_update<1><<<rb, blk, 0, st>>>(b, ph);
     mark("k_update");
-    k_finish<<<1, 1, 0, st>>>(b.ctl);
-    mark("k_finish");
     if (n_launch) *n_launch = nl;
     return cudaGetLastError();
 }

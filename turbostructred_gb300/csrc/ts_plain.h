@@ -9,12 +9,21 @@
 namespace ts {
 
 constexpr int kPlainBlock = 128;
+// Most blocks of k_dt and k_update: 16 per SM of 152, whose threads then take
+// up to 23 cells each at 192^3 (k_update 3.0 -> 0.72 ms there, with its
+// divisions on the integer pipe).
+constexpr int kPlainReduceBlocks = 152 * 16;
 
 struct PlainBufs {
     Layout L;
     double* U;           // NV planes: conserved state
-    double* G;           // 3*NV planes: slopes, plane a*NV+v
-    double* Lim;         // NV planes: limiter values
+    // With `fold`, G holds the (limited) projections lim * (slope * h/2) to the
+    // cell's high faces, and the low faces take their negatives.  Without it
+    // (a periodic axis whose ghost cells differ in size from the cells they
+    // repeat, so a face samples with another h) G holds slopes, Lim limiters.
+    int fold;
+    double* G;           // nd*NV planes, plane a*NV+v
+    double* Lim;         // NV planes: limiter values (null with fold)
     double* F[3];        // NV planes per axis: face fluxes stored at the face's right cell
     double* Lam[3];      // 1 plane per axis: face max eigenvalue
     const double* cx[3]; // cell centres per axis, index i + ghost width
