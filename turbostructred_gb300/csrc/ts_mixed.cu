@@ -764,6 +764,11 @@ __global__ void __launch_bounds__(512, 1) k_mix_tail(const ProbDesc* __restrict_
     const int tid = threadIdx.x;
     const unsigned int rank = cluster.block_rank();
     const ProbDesc& d = probs[list[blockIdx.x / cluster.num_blocks()]];
+    // A finished problem that is still listed is left alone (every CTA of its
+    // cluster leaves here): it may be read back, and its memory given to
+    // another problem, on other streams beside this launch, so writing its
+    // state back unchanged is not harmless.
+    if (d.ctl->stop_req) return;
     const MixPhys& mp = d.mp;
     const int i0 = (int)rank * T::TX;
     const long long plane = d.L.plane;
