@@ -100,3 +100,43 @@ def test_kernels_outside_the_fast_ranges(spec, tslib, oracle_mod):
         got = s.get_state(capi.LAYOUT_WITH_GHOSTS)
     assert np.array_equal(got, ref)
     assert info["time"] == rinfo["time"] and info["dt"] == rinfo["dt"]
+
+
+@pytest.mark.parametrize("kind", ["random", "near_powers", "ties", "zero_dividends", "all_patterns"])
+def test_products_are_correctly_rounded(kind, tmp_path):
+    exe = str(tmp_path / "mul_check")
+    subprocess.run(["g++", "-O2", "-std=c++20", "-ffp-contract=off", "-I" + CSRC,
+                    os.path.join(ROOT, "tests", "exact64_mul_check.cpp"), "-o", exe], check=True)
+    if kind == "ties":  # short significands: products of exactly 54 bits, and exact ones
+        r = np.random.default_rng(3)
+        a, b = (r.integers(1 << 26, 1 << 27, 400_000).astype(np.float64) for _ in range(2))
+    else:
+        a, b = operands(kind)
+    out = subprocess.run([exe], input=np.stack([a, b], 1).tobytes(), capture_output=True, check=True).stdout
+    wrong, refused = (int(x) for x in out.split())
+    assert wrong == 0
+    assert (refused == 0) == (kind != "all_patterns")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale,w", [(1.0, None), (2.0 ** -520, None), (1.0, 1e-190)], ids=["usual", "tiny_state", "tiny_w"])
+@pytest.mark.parametrize("eps", [0.0, 0.1])
+def test_3d_roe_faces(scale, w, eps, tslib, oracle_mod):
+    """The 3D Roe faces, whose products run on the integer pipe, on sizes that leave partial warps and blocks."""
+    from oracle import oracle as O
+    from turbostructred_gb300 import capi
+    case = O.make_case(ndims=3, nx=13, ny=7, nz=5, periodic=(1, 0, 0), recon=3, solver=1, eps=eps, cfl=0.4, bc=[SYM] * 6)
+    r = np.random.default_rng(5)
+    rho, p = r.uniform(0.5, 2.0, (5, 7, 13)), r.uniform(0.5, 2.0, (5, 7, 13))
+    v = r.uniform(-0.5, 0.5, (5, 7, 13, 3)) * (r.uniform(size=(5, 7, 13, 1)) < 0.7)
+    if w is not None:
+        v[..., 2] = w
+    ic = np.concatenate([rho[..., None], rho[..., None] * v, (p / 0.4 + 0.5 * rho * (v * v).sum(-1))[..., None]], -1) * scale
+    full = oracle_mod.embed(case, ic)
+    ref, rinfo = oracle_mod.advance(case, full, 6)
+    with capi.Solver(capi.make_case(**case)) as s:
+        s.set_state(full, capi.LAYOUT_WITH_GHOSTS)
+        info = s.step(6)
+        got = s.get_state(capi.LAYOUT_WITH_GHOSTS)
+    assert np.array_equal(got, ref)
+    assert info["time"] == rinfo["time"] and info["dt"] == rinfo["dt"]

@@ -135,12 +135,33 @@ struct Fast {
     __device__ __forceinline__ double div(double a, double b) { return x64::div(a, b, bad); }
     __device__ __forceinline__ double root(double a) { return x64::root(a, bad); }
     __device__ __forceinline__ double half(double a) { return x64::half(a, bad); }
+    __device__ __forceinline__ double mul(double a, double b) { return a * b; }
     __device__ __forceinline__ double min(double a, double b) { return dlt(a, b) ? a : b; }
     __device__ __forceinline__ double max(double a, double b) { return dlt(a, b) ? b : a; }
     __device__ __forceinline__ bool lt(double a, double b) { return dlt(a, b); }
     __device__ __forceinline__ bool ge0(double a) { return !dneg(a); }
     __device__ __forceinline__ bool le0(double a) { return !dpos(a); }
 };
+// FastMul: also the products written o.mul on the integer pipe (the 56 of the
+// Roe flux's closing sums, of its 106).  An integer product takes 14.4 clocks
+// per warp and SM, beside the FP64 pipe's 19 for the rest of the flux, so about
+// half of them balances the two; with all of them there the code no longer fits the
+// instruction cache.  One step of the 3D blast 192^3: none 9.96 ms, these 56
+// 8.6 ms, the other 50 9.4 ms, all 9.8 ms.
+struct FastMul : Fast {
+    __device__ __forceinline__ double mul(double a, double b) {
+        bool rare;
+        const double r = x64::mul(a, b, rare);
+        bad |= rare;
+        return r;
+    }
+};
+// 3D Roe faces use it: those grids keep the pipes full.  A grid of 1D or 2D
+// ends in latency instead, which the integer products lengthen (2D box
+// 203x157: 2741 -> 2763 us, 1D tube of 1000 cells: 40.0 -> 44.1 ms), and HLLC
+// has too few products for it (2D shear layer 1024^2: 10.8 -> 10.3 ms with all).
+template <int ND, int SOLVER>
+using FaceArith = std::conditional_t<ND == 3 && SOLVER == TS_RS_ROE_PIKE, FastMul, Fast>;
 struct Plain {
     typedef double Div;
     __device__ __forceinline__ Div divisor(double b) { return b; }
@@ -148,6 +169,7 @@ struct Plain {
     __device__ __forceinline__ double div(double a, double b) { return a / b; }
     __device__ __forceinline__ double root(double a) { return sqrt(a); }
     __device__ __forceinline__ double half(double a) { return a * 0.5; }
+    __device__ __forceinline__ double mul(double a, double b) { return a * b; }
     __device__ __forceinline__ double min(double a, double b) { return fmin(a, b); }
     __device__ __forceinline__ double max(double a, double b) { return fmax(a, b); }
     __device__ __forceinline__ bool lt(double a, double b) { return a < b; }
@@ -266,7 +288,8 @@ __device__ __forceinline__ double roe_flux(const Phys& ph, const double UL[NV], 
     // Qa = (0, e_A, uw), Qb = (1, vel, h); terms multiplying a zero Qa entry
     // are exact zeros and are left out.
     {
-        const double t = Eig1 * UL[0] + Eiga * D2 + Eigb * (R2 * C2) - Eig1 * UR[0] - Eiga * D1 - Eigb * (R1 * C2);
+        const double t = o.mul(Eig1, UL[0]) + o.mul(Eiga, D2) + o.mul(Eigb, o.mul(R2, C2)) - o.mul(Eig1, UR[0]) -
+                         o.mul(Eiga, D1) - o.mul(Eigb, o.mul(R1, C2));
         flux[0] = o.half(flux[0] + t);
     }
 #pragma unroll
@@ -274,16 +297,20 @@ __device__ __forceinline__ double roe_flux(const Phys& ph, const double UL[NV], 
         if (b >= NC) continue;
         double t;
         if (b == A)
-            t = Eig1 * UL[1 + b] + Eiga * (R2 + D2 * vel[b]) + Eigb * (R2 * vel[b] * C2 + D2) - Eig1 * UR[1 + b] -
-                Eiga * (R1 + D1 * vel[b]) - Eigb * (R1 * vel[b] * C2 + D1);
+            t = o.mul(Eig1, UL[1 + b]) + o.mul(Eiga, R2 + o.mul(D2, vel[b])) +
+                o.mul(Eigb, o.mul(o.mul(R2, vel[b]), C2) + D2) - o.mul(Eig1, UR[1 + b]) -
+                o.mul(Eiga, R1 + o.mul(D1, vel[b])) - o.mul(Eigb, o.mul(o.mul(R1, vel[b]), C2) + D1);
         else
-            t = Eig1 * UL[1 + b] + Eiga * (D2 * vel[b]) + Eigb * (R2 * vel[b] * C2) - Eig1 * UR[1 + b] -
-                Eiga * (D1 * vel[b]) - Eigb * (R1 * vel[b] * C2);
+            t = o.mul(Eig1, UL[1 + b]) + o.mul(Eiga, o.mul(D2, vel[b])) +
+                o.mul(Eigb, o.mul(o.mul(R2, vel[b]), C2)) - o.mul(Eig1, UR[1 + b]) -
+                o.mul(Eiga, o.mul(D1, vel[b])) - o.mul(Eigb, o.mul(o.mul(R1, vel[b]), C2));
         flux[1 + b] = o.half(flux[1 + b] + t);
     }
     {
-        const double t = Eig1 * UL[4] + Eiga * (R2 * uw + D2 * h) + Eigb * (R2 * h * C2 + D2 * uw) - Eig1 * UR[4] -
-                         Eiga * (R1 * uw + D1 * h) - Eigb * (R1 * h * C2 + D1 * uw);
+        const double t = o.mul(Eig1, UL[4]) + o.mul(Eiga, o.mul(R2, uw) + o.mul(D2, h)) +
+                         o.mul(Eigb, o.mul(o.mul(R2, h), C2) + o.mul(D2, uw)) - o.mul(Eig1, UR[4]) -
+                         o.mul(Eiga, o.mul(R1, uw) + o.mul(D1, h)) -
+                         o.mul(Eigb, o.mul(o.mul(R1, h), C2) + o.mul(D1, uw));
         flux[4] = o.half(flux[4] + t);
     }
     return eig_max;
@@ -1037,7 +1064,8 @@ __device__ __noinline__ double riemann_plain(const Phys& ph, const double* UL, c
 
 template <int A, int ND, int SOLVER>
 __device__ __forceinline__ double face_flux(const Phys& ph, const double UL[NV], const double UR[NV], double F[NV]) {
-    Fast o;
+    typedef FaceArith<ND, SOLVER> O;
+    O o;
     double lam;
     bool z = false;
     if (ND < 3) {
@@ -1046,8 +1074,8 @@ __device__ __forceinline__ double face_flux(const Phys& ph, const double UL[NV],
         for (int b = ND; b < 3; ++b) mine = mine && dzero(UL[1 + b]) && dzero(UR[1 + b]);
         z = __all_sync(__activemask(), mine);
     }
-    if (ND < 3 && z) lam = riemann<A, SOLVER, ND, Fast>(ph, UL, UR, F, o);
-    else lam = riemann<A, SOLVER, 3, Fast>(ph, UL, UR, F, o);
+    if (ND < 3 && z) lam = riemann<A, SOLVER, ND, O>(ph, UL, UR, F, o);
+    else lam = riemann<A, SOLVER, 3, O>(ph, UL, UR, F, o);
     if (o.bad) {
         double l[NV], r[NV], f[NV];
 #pragma unroll
@@ -1061,7 +1089,7 @@ __device__ __forceinline__ double face_flux(const Phys& ph, const double UL[NV],
 
 // One face per thread along axis A; faces are stored at their right cell.
 template <int A, int ND, int SOLVER>
-__global__ void __launch_bounds__(kPlainBlock) k_flux(const __grid_constant__ PlainBufs b,
+__global__ void __launch_bounds__(kPlainBlock, ND == 3 ? 4 : 1) k_flux(const __grid_constant__ PlainBufs b,
                                                       const __grid_constant__ Phys ph) {
     if (b.ctl->stop_req) return;
     const Layout& L = b.L;
