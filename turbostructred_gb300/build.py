@@ -1,7 +1,7 @@
 """Builds the CUDA extension in-tree: turbostructred_gb300/libtsfvm.so.
 
 Every translation unit is compiled for sm_103a only, in parallel, with nvcc.
-ts_plain.cu (the bit-for-bit FP64 path) is compiled with --fmad=false so no
+ts_plain.cu and ts_tube64.cu (the bit-for-bit FP64 path) are compiled with --fmad=false so no
 multiply-add contraction changes its rounding; the other units keep FMA.
 """
 from __future__ import annotations
@@ -27,6 +27,7 @@ COMMON = ["-O3", "-std=c++20", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 
 UNITS = {
     "ts_plain.cu": ["--fmad=false"],
+    "ts_tube64.cu": ["--fmad=false"],
     # FP32 flux path: flush-to-zero and approximate FP32 division/sqrt; FP64
     # arithmetic is unaffected by these flags.
     "ts_mixed.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],

@@ -73,6 +73,9 @@ __global__ void k_gather(double* __restrict__ aos, Layout L, const double* __res
 
 }  // namespace
 
+// Steps of one launch of the resident 1D kernel.
+constexpr int kTubeSteps = 4096;
+
 struct ts_handle {
     ts_config cfg{};
     std::vector<ts_block_node> blocks[3];
@@ -84,6 +87,7 @@ struct ts_handle {
     cudaStream_t stream = nullptr;
     std::vector<void*> allocations;
     PlainBufs pb{};
+    int tube_ctas = 0;        // 1D FP64: CTAs of the resident kernel (0: stage kernels)
     MixedBufs mb{};
     Ctl* ctl_d = nullptr;
     Ctl* ctl_h = nullptr;     // pinned mirror
@@ -192,6 +196,8 @@ struct ts_handle {
             pb.eps2 = d;
         }
         if ((s = alloc(&pb.partial, (size_t)plain_partial_blocks(L))) != TS_OK) return s;
+        if ((s = alloc(&pb.norms, (size_t)NV * kNormSlots)) != TS_OK) return s;
+        TS_CUDA(cudaMemsetAsync(pb.norms, 0, sizeof(double) * NV * kNormSlots, stream));
         if (cfg.viscous) {
             if ((s = alloc(&pb.VG, (size_t)9 * L.plane)) != TS_OK) return s;
             TS_CUDA(cudaMemsetAsync(pb.VG, 0, (size_t)9 * L.plane * sizeof(double), stream));
@@ -200,6 +206,7 @@ struct ts_handle {
             for (int a = 0; a < nd; ++a)
                 if ((s = alloc(&pb.VSR[a], L.plane)) != TS_OK) return s;
         pb.ctl = ctl_d;
+        tube_ctas = tube64_ctas(L, ph, pb.fold);
         return TS_OK;
     }
 
@@ -231,6 +238,12 @@ struct ts_handle {
     }
 
     ts_status launch_steps(int n) {
+        if (tube_ctas) {
+            // at most some 30 ms per launch
+            for (; n > 0; n -= std::min(n, kTubeSteps))
+                TS_CUDA(tube64_steps(pb, ph, tube_ctas, std::min(n, kTubeSteps), stream));
+            return TS_OK;
+        }
         static const int chunks[3] = {64, 8, 1};
         for (int c : chunks) {
             while (n >= c) {
@@ -515,13 +528,14 @@ ts_status ts_run(ts_handle* h, ts_step_info* info) {
     h->ctl_h->health = 0;
     if ((s = h->push_ctl()) != TS_OK) return s;
     // Steps past termination are no-ops on the device (stop_req), so chunks
-    // may overshoot; the chunk grows while the run continues.
-    int chunk = 8;
+    // may overshoot; the chunk grows while the run continues.  (The resident
+    // kernel ends by itself.)
+    int chunk = h->tube_ctas ? kTubeSteps : 8;
     for (;;) {
         if ((s = h->launch_steps(chunk)) != TS_OK) return s;
         if ((s = h->pull_ctl()) != TS_OK) return s;
         if (h->ctl_h->stop_req) break;
-        if (chunk < 512) chunk *= 2;
+        if (!h->tube_ctas && chunk < 512) chunk *= 2;
     }
     h->fill_info(info);
     return TS_OK;

@@ -14,6 +14,11 @@ constexpr int kPlainBlock = 128;
 // divisions on the integer pipe).
 constexpr int kPlainReduceBlocks = 152 * 16;
 
+// Running sums that the blocks of k_update add each norm to (one per lane of
+// the warp that sums them up).
+constexpr int kNormSlots = 32;
+constexpr unsigned kNormDirectBlocks = 512;
+
 struct PlainBufs {
     Layout L;
     double* U;           // NV planes: conserved state
@@ -30,6 +35,7 @@ struct PlainBufs {
     const double* ch[3]; // cell sizes per axis
     const double* eps2;  // Venkatakrishnan eps^2 per cell (one plane) or null
     double* partial;     // per-block minima of V/SR
+    double* norms;       // NV x kNormSlots running sums of V |R| (zero between steps)
     Ctl* ctl;
     double* VG;          // viscous flow: 9 planes, d(velocity d)/d(axis e) at plane 3d+e
     double* VSR[3];      // viscosity > 0: 1 plane per axis, the face's viscous
@@ -44,5 +50,12 @@ int plain_partial_blocks(const Layout& L);
 constexpr int kPlainMaxLaunches = 14;
 cudaError_t plain_step(const PlainBufs& b, const Phys& ph, cudaStream_t st, cudaEvent_t* ev = nullptr,
                        int* n_launch = nullptr, const char** names = nullptr);
+
+// 1D problems: many steps per launch by one thread-block cluster that keeps
+// the state on chip (ts_tube64.cu).  The CTAs of the cluster, or 0 when the
+// problem takes the stage kernels.
+int tube64_ctas(const Layout& L, const Phys& ph, int fold);
+// `steps` steps (fewer when a Run ends) in one launch.
+cudaError_t tube64_steps(const PlainBufs& b, const Phys& ph, int ctas, int steps, cudaStream_t st);
 
 }  // namespace ts
