@@ -32,6 +32,7 @@ UNITS = {
     # arithmetic is unaffected by these flags.
     "ts_mixed.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
     "ts_mix3d.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
+    "ts_flat2d.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
     "ts_capi.cu": [],
     "ts_batch.cu": [],
     "ts_host.cpp": [],

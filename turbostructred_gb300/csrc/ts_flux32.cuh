@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include "ts_exact64.cuh"
 #include "ts_mixed.h"
 
 namespace ts {
@@ -216,14 +217,28 @@ __device__ __forceinline__ void add_norms(Ctl* ctl, const float (&nrm)[NV], unsi
     }
 }
 
+// cfl / m and 1 / m, correctly rounded, on the integer pipe: a division on the
+// FP64 pipe is 470 clocks, and every stage ends with these.
+__device__ __forceinline__ void step_size(double cfl, float m, double& dt, double& raw) {
+    bool bad = false;
+    const x64::Divisor by = x64::divisor((double)m, bad);
+    dt = x64::quotient(cfl, by, bad);
+    raw = x64::quotient(1.0, by, bad);
+    if (bad) {
+        dt = cfl / (double)m;
+        raw = 1.0 / (double)m;
+    }
+}
+
 // dt of one problem from its CFL maximum, and the step's bookkeeping
 // (ComputeTimeStep :1427-1437, time += dt and iteration++ :1486-1487, and the
 // Kernel::Run snapshot/termination rules kernel.h:1763-1846).
 __device__ __forceinline__ void finish_with(Ctl* ctl, float m, double cfl) {
-    double dt = cfl / (double)m;
+    double dt, raw;
+    step_size(cfl, m, dt, raw);
     if ((ctl->save_sol > 0) && (ctl->next_sol < ctl->time + dt)) dt = ctl->next_sol - ctl->time;
     if ((ctl->save_slice > 0) && (ctl->next_slice < ctl->time + dt)) dt = ctl->next_slice - ctl->time;
-    ctl->dt_min_raw = 1.0 / (double)m;
+    ctl->dt_min_raw = raw;
     // the stage's residual norms (zeros when they are not formed)
 #pragma unroll
     for (int v = 0; v < NV; ++v) {

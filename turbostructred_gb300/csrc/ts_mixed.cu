@@ -1077,6 +1077,11 @@ cudaError_t mixed_launch_tail(int solver, int cluster, int n_problems, const Pro
                                 : tail_launch<TS_RS_ROE_PIKE>(cluster, n_problems, d_probs, d_list, budget, st);
 }
 
+// 2D problems of at most this many cells (362 x 362) march nothing: stage
+// times, k_flat2d against k_mix_step: 128^2 6.9 / 11.4 us, 256^2 11.1 / 14.0,
+// 384^2 17.5 / 17.4, 512^2 27.4 / 24.3.
+constexpr long long kFlatCells = 1LL << 17;
+
 void mixed_tile_cells(int nd, int tx, int ty, int* cx, int* cy) {
     *cx = nd == 3 ? tx : tx - 2 * HB;
     *cy = nd == 3 ? ty : 1;
@@ -1144,6 +1149,7 @@ ts_status mixed_set_tile(MixedBufs& mb, int tx, int ty, int zchunks, std::string
     if (per_sm < 1) { err = "mixed kernel does not fit on an SM with this tile"; return TS_ERR_UNSUPPORTED; }
     mb.tx = tx;
     mb.ty = ty;
+    mb.flat = 0;
     mb.smem = bytes;
     const long long slots = (long long)mb.sms * per_sm;
     mixed_items(mb.desc, tx, ty, zchunks, slots);
@@ -1305,16 +1311,19 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
     // 12.2e9 cell-updates/s for 260-thread rows)
     const int tx = L.nd == 3 ? 32 : (L.nd == 2 ? 132 : 256);
     const int ty = L.nd == 3 ? 8 : 1;
-    return mixed_set_tile(mb, tx, ty, 0, err, st);
+    if ((s = mixed_set_tile(mb, tx, ty, 0, err, st)) != TS_OK) return s;
+    if (L.nd == 2 && L.cells() <= kFlatCells) mb.flat = flat2d_tiles(d, &d.ncx);
+    return TS_OK;
 }
 
 void mixed_step(MixedBufs& mb, const Phys&, cudaStream_t st, cudaEvent_t* ev, int* n_launch, const char** names) {
     const bool d3 = mb.desc.L.nd == 3;
     if (ev) cudaEventRecord(ev[0], st);
     if (d3) mix3d_launch(mb.tx, mb.ty, mb.grid, mb.desc, mb.maps, st);
+    else if (mb.flat) flat2d_launch(mb.desc, mb.flat, st);
     else mixed_launch_single(mb.desc.L.nd, mb.tx, mb.ty, mb.desc.mp.solver, mb.grid, mb.desc, st);
     if (ev) cudaEventRecord(ev[1], st);
-    if (names) names[0] = d3 ? "k_mix3d" : "k_mix_step";
+    if (names) names[0] = d3 ? "k_mix3d" : (mb.flat ? "k_flat2d" : "k_mix_step");
     if (n_launch) *n_launch = 1;
 }
 

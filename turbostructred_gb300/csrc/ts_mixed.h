@@ -88,6 +88,7 @@ struct MixedBufs {
     int grid = 0;                  // persistent CTAs
     size_t smem = 0;
     int sms = 0;
+    int flat = 0;                  // tiles of the 2D kernel that marches nothing (0: not used)
 };
 
 using DeviceAlloc = std::function<ts_status(size_t bytes, void** out)>;
@@ -144,6 +145,11 @@ bool mix3d_tile_info(int tx, int ty, int solver, int recon, int limiter, size_t*
 // Tensor maps of the four state buffers for the tile's box.
 ts_status mix3d_make_maps(const ProbDesc& d, int tx, int ty, Mix3dMaps& maps, std::string& err);
 void mix3d_launch(int tx, int ty, int grid, const ProbDesc& d, const Mix3dMaps& maps, cudaStream_t st);
+
+// 2D problems: one CTA per 32 x 4 tile, nothing marched (ts_flat2d.cu).  Its
+// tiles (and tile columns), and one stage.
+int flat2d_tiles(const ProbDesc& d, int* ncx);
+void flat2d_launch(const ProbDesc& d, int tiles, cudaStream_t st);
 
 constexpr int kMixedMaxLaunches = 4;
 void mixed_step(MixedBufs& mb, const Phys& ph, cudaStream_t st, cudaEvent_t* ev = nullptr, int* n_launch = nullptr,
