@@ -1087,6 +1087,34 @@ void mixed_tile_cells(int nd, int tx, int ty, int* cx, int* cy) {
     *cy = nd == 3 ? ty : 1;
 }
 
+// Chunks of the marching axis for a 3D problem of `cols` tile columns and nz
+// planes: the count with the shortest modelled stage, in us, which is
+// returned.  An item of ch planes costs ch + 2.5 (its start-up) plane passes
+// of 3.45 us while it has its SM to itself, rising to 4.4 us with all CTA
+// slots taken; a last wave that is partly filled costs half of what is
+// missing, since its CTAs run faster alone.  Fitted on sweeps of the chunk
+// length over ten grids from 32^3 to 256^3 (32x8 tiles): within 12 % of the
+// measured times and the fastest or next to it on each.  Against chunks of at
+// least 16 planes: 32^3 70 -> 21 us per stage, 64^3 72 -> 34, 45x150x25 106 ->
+// 33, 97x61x83 87 -> 61; 128^3 and larger as before.
+double plan3d(long long cols, int nz, long long slots, int* zchunks) {
+    double best = 1e300;
+    const double s = (double)std::max(1LL, slots);
+    for (int c = 1; c <= nz; ++c) {
+        const int ch = (nz + c - 1) / c;
+        if (ch < 2 && nz > 1) break;
+        const double q = (double)(cols * ((nz + ch - 1) / ch));
+        const double w = q / s;
+        const double passes = w <= 0.5 ? 3.45 : (w <= 1.0 ? 3.45 + 0.95 * (2.0 * w - 1.0) : 2.2 * (w + std::ceil(w)));
+        const double t = 6.0 + (ch + 2.5) * passes;
+        if (t < best - 1e-9) {
+            best = t;
+            *zchunks = c;
+        }
+    }
+    return best;
+}
+
 void mixed_items(ProbDesc& d, int tx, int ty, int zchunks, long long slots) {
     const int nd = d.L.nd;
     int cx, cy;
@@ -1116,19 +1144,7 @@ void mixed_items(ProbDesc& d, int tx, int ty, int zchunks, long long slots) {
             if (t < best - 1e-9) { best = t; zchunks = c; }
         }
     }
-    if (march && zchunks <= 0) {
-        // Chunks of >= 16 planes; pick the count that best fills the
-        // persistent grid, charging ~2 planes of start-up per chunk.
-        double best = -1.0;
-        for (int c = 1; c <= std::max(1, nz / 16); ++c) {
-            const int ch = (nz + c - 1) / c;
-            const int nch = (nz + ch - 1) / ch;
-            const long long q = (long long)d.ncol * nch;
-            const double waves = std::ceil((double)q / (double)std::max(1LL, slots));
-            const double score = (double)q / (waves * (double)std::max(1LL, slots)) / (1.0 + 2.0 / ch);
-            if (score > best + 1e-9) { best = score; zchunks = c; }
-        }
-    }
+    if (nd == 3 && zchunks <= 0) plan3d(d.ncol, nz, slots, &zchunks);
     zchunks = march ? std::max(1, std::min(zchunks, nz)) : 1;
     d.ch = march ? (nz + zchunks - 1) / zchunks : 1;
     d.nq = d.ncol * ((nz + d.ch - 1) / d.ch);
@@ -1309,8 +1325,17 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
     cudaDeviceGetAttribute(&mb.sms, cudaDevAttrMultiProcessorCount, dev);
     // 2D: 132-thread rows (measured on the 1024^2 shear layer: 13.3e9 against
     // 12.2e9 cell-updates/s for 260-thread rows)
-    const int tx = L.nd == 3 ? 32 : (L.nd == 2 ? 132 : 256);
-    const int ty = L.nd == 3 ? 8 : 1;
+    int tx = L.nd == 3 ? 32 : (L.nd == 2 ? 132 : 256);
+    int ty = L.nd == 3 ? 8 : 1;
+    if (L.nd == 3) {
+        // 16x16 tiles where they cover the grid with enough fewer columns
+        // (a plane pass of theirs takes 5 % longer: 64^3 35.6 against 34.1 us;
+        // but 97x61x83 60.6 against 67.4, 200x30x120 68.6 against 75.1)
+        const long long slots = 2LL * mb.sms;
+        int z;
+        auto cols = [&](int x, int y) { return (long long)((L.nx + x - 1) / x) * ((L.ny + y - 1) / y); };
+        if (1.05 * plan3d(cols(16, 16), L.nz, slots, &z) < plan3d(cols(32, 8), L.nz, slots, &z)) tx = ty = 16;
+    }
     if ((s = mixed_set_tile(mb, tx, ty, 0, err, st)) != TS_OK) return s;
     if (L.nd == 2 && L.cells() <= kFlatCells) mb.flat = flat2d_tiles(d, &d.ncx);
     return TS_OK;
