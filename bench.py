@@ -576,7 +576,7 @@ def run_tubes(args, rank, ws, lr, dist, emit=True):
                         "d2h_bytes_per_step": bytes_in, "seconds_per_job": e2e_s},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": profile_traffic("tubes", "k_mix_step", cu),
-                             "kernel": "k_mix_step (batched, one-row 1D tiles) and k_mix_tail",
+                             "kernel": "k_mix_step (batched, one-row 1D tiles) and k_tube32",
                              "kernel_ms": None, "algorithmic_bytes": BYTES_PER_CELL_UPDATE * cu,
                              "basis": "80 B x the batch's cell-updates over the whole solve's wall time (stage "
                                       "kernels, finish kernels, the cluster tail kernel and launch gaps): a lower "

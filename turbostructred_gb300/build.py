@@ -33,6 +33,7 @@ UNITS = {
     "ts_mixed.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
     "ts_mix3d.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
     "ts_flat2d.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
+    "ts_tube32.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
     "ts_capi.cu": [],
     "ts_batch.cu": [],
     "ts_host.cpp": [],

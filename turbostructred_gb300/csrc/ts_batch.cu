@@ -181,7 +181,7 @@ struct ts_batch {
     // the last few long 1D problems run in the cluster tail kernel: many
     // stages per launch, state on chip (one list per Riemann solver)
     bool tail_enabled = true, tail_mode = false;
-    int tail_cluster = 0;
+    int tail_cluster = 0, tail_cells = 0;  // CTAs per problem, cells of the largest
     int* d_tail[2] = {nullptr, nullptr};
     int tail_n[2] = {0, 0}, tail_cap[2] = {0, 0};
     Arena arena;
@@ -358,27 +358,28 @@ struct ts_batch {
     }
 
     // Tail mode when every unfinished problem is 1D, fits one cluster, and
-    // all clusters together fit the GPU at once (one CTA per SM).
+    // all clusters together fit the GPU at once (one CTA per SM); the clusters are as
+    // large as that allows.
     ts_status plan_tail() {
         tail_mode = false;
         tail_n[0] = tail_n[1] = 0;
         if (!tail_enabled) return TS_OK;
-        const int cells = mixed_tail_cells();
         std::vector<int> lists[2];
-        int cmax = 0, nact = 0;
+        int nact = 0;
+        tail_cells = 0;
         for (int s = 0; s < capacity; ++s) {
             if (!slots[s].used || h_ctl[s].stop_req) continue;
             const ProbDesc& d = desc[s];
-            const int items = (d.kn[0] + cells - 1) / cells;
-            // the tail kernel forms no residual norms
-            if (d.L.nd != 1 || items > kTailMaxCluster || d.mp.norms) return TS_OK;
-            cmax = std::max(cmax, items);
+            // the resident kernel forms no residual norms
+            if (d.L.nd != 1 || d.kn[0] < 4 || d.kn[0] > tube32_max_cells() || d.mp.norms) return TS_OK;
+            tail_cells = std::max(tail_cells, d.kn[0]);
             lists[d.mp.solver == TS_RS_HLLC ? 1 : 0].push_back(s);
             ++nact;
         }
-        if (nact == 0 || (long long)nact * cmax > sms) return TS_OK;
+        if (nact == 0 || nact > sms) return TS_OK;
+        tail_cluster = std::min({kTailMaxCluster, sms / nact, std::max(1, tail_cells / 30)});
         for (int k = 0; k < 2; ++k)
-            if (!lists[k].empty() && !mixed_tail_ready(k ? TS_RS_HLLC : TS_RS_ROE_PIKE, cmax)) return TS_OK;
+            if (!lists[k].empty() && !tube32_ready(k ? TS_RS_HLLC : TS_RS_ROE_PIKE, tail_cluster, tail_cells)) return TS_OK;
         for (int k = 0; k < 2; ++k) {
             tail_n[k] = (int)lists[k].size();
             if (!tail_n[k]) continue;
@@ -391,7 +392,6 @@ struct ts_batch {
             TB_CUDA(cudaMemcpyAsync(d_tail[k], lists[k].data(), sizeof(int) * tail_n[k], cudaMemcpyHostToDevice,
                                     stream));
         }
-        tail_cluster = cmax;
         tail_mode = true;
         return TS_OK;
     }
@@ -437,8 +437,8 @@ struct ts_batch {
             // every tail problem advances up to n stages in one launch
             for (int k = 0; k < 2; ++k) {
                 if (!tail_n[k]) continue;
-                TB_CUDA(mixed_launch_tail(k ? TS_RS_HLLC : TS_RS_ROE_PIKE, tail_cluster, tail_n[k], d_desc, d_tail[k],
-                                          n, stream));
+                TB_CUDA(tube32_launch(k ? TS_RS_HLLC : TS_RS_ROE_PIKE, tail_cluster, tail_n[k], tail_cells, d_desc,
+                                      d_tail[k], n, stream));
                 ++launches;
             }
             stages += n;

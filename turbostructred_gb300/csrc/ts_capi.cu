@@ -73,7 +73,7 @@ __global__ void k_gather(double* __restrict__ aos, Layout L, const double* __res
 
 }  // namespace
 
-// Steps of one launch of the resident 1D kernel.
+// Steps of one launch of the resident 1D kernels.
 constexpr int kTubeSteps = 4096;
 
 struct ts_handle {
@@ -237,11 +237,16 @@ struct ts_handle {
         return TS_OK;
     }
 
+    // 1D problems on the resident kernels
+    bool resident() const { return tube_ctas != 0 || mb.tube != 0; }
+
     ts_status launch_steps(int n) {
-        if (tube_ctas) {
+        if (resident()) {
             // at most some 30 ms per launch
-            for (; n > 0; n -= std::min(n, kTubeSteps))
-                TS_CUDA(tube64_steps(pb, ph, tube_ctas, std::min(n, kTubeSteps), stream));
+            for (; n > 0; n -= std::min(n, kTubeSteps)) {
+                const int k = std::min(n, kTubeSteps);
+                TS_CUDA(tube_ctas ? tube64_steps(pb, ph, tube_ctas, k, stream) : mixed_resident_steps(mb, k, stream));
+            }
             return TS_OK;
         }
         static const int chunks[3] = {64, 8, 1};
@@ -530,12 +535,12 @@ ts_status ts_run(ts_handle* h, ts_step_info* info) {
     // Steps past termination are no-ops on the device (stop_req), so chunks
     // may overshoot; the chunk grows while the run continues.  (The resident
     // kernel ends by itself.)
-    int chunk = h->tube_ctas ? kTubeSteps : 8;
+    int chunk = h->resident() ? kTubeSteps : 8;
     for (;;) {
         if ((s = h->launch_steps(chunk)) != TS_OK) return s;
         if ((s = h->pull_ctl()) != TS_OK) return s;
         if (h->ctl_h->stop_req) break;
-        if (!h->tube_ctas && chunk < 512) chunk *= 2;
+        if (!h->resident() && chunk < 512) chunk *= 2;
     }
     h->fill_info(info);
     return TS_OK;

@@ -89,6 +89,7 @@ struct MixedBufs {
     size_t smem = 0;
     int sms = 0;
     int flat = 0;                  // tiles of the 2D kernel that marches nothing (0: not used)
+    int tube = 0;                  // CTAs of the resident 1D kernel (0: not used)
 };
 
 using DeviceAlloc = std::function<ts_status(size_t bytes, void** out)>;
@@ -119,17 +120,6 @@ bool mixed_launch_batch(int nd, int tx, int ty, int solver, int grid, const Prob
                         const int2* d_items, int n_items, cudaStream_t st, bool close_in_kernel = false);
 void mixed_batch_finish(const ProbDesc* d_probs, const int* d_slots, int n, cudaStream_t st);
 
-// Tail of a batch: n_problems 1D problems (d_list: their descriptor indices),
-// each advanced by up to `budget` stages in one launch by a cluster of
-// `cluster` CTAs that own mixed_tail_cells() cells each and keep the state
-// on chip between stages (same arithmetic as the batched kernel).
-constexpr int kTailMaxCluster = 16;
-int mixed_tail_cells();
-// The tail kernel can run clusters of this size on this device.
-bool mixed_tail_ready(int solver, int cluster);
-cudaError_t mixed_launch_tail(int solver, int cluster, int n_problems, const ProbDesc* d_probs, const int* d_list,
-                              int budget, cudaStream_t st);
-
 // Set-up of one problem's buffers; every upload and (with zero_buffers) the
 // clearing of the state and residual buffers are queued on `st`.
 ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const HostGrid& g, Ctl* ctl,
@@ -138,6 +128,16 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
 // Choose the tile shape (tx, ty) and the z chunking (0 = automatic), and
 // recompute the persistent grid (descriptor upload queued on `st`).
 ts_status mixed_set_tile(MixedBufs& mb, int tx, int ty, int zchunks, std::string& err, cudaStream_t st);
+
+// 1D problems (without residual norms): up to `budget` stages in one launch, a
+// cluster of `cluster` CTAs per problem, the state on chip (ts_tube32.cu).
+// d_list: descriptor indices (null: d_probs[0] alone); cells: those of the
+// largest problem.
+constexpr int kTailMaxCluster = 16;
+int tube32_max_cells();
+bool tube32_ready(int solver, int cluster, int cells);
+cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, const ProbDesc* d_probs, const int* d_list,
+                          int budget, cudaStream_t st);
 
 // 3D problems: the TMA-staged fused kernel (ts_mix3d.cu).  Compiled tiles
 // 32x8 and 16x16; smem bytes and resident CTAs per SM, or false.
@@ -154,6 +154,8 @@ void flat2d_launch(const ProbDesc& d, int tiles, cudaStream_t st);
 constexpr int kMixedMaxLaunches = 4;
 void mixed_step(MixedBufs& mb, const Phys& ph, cudaStream_t st, cudaEvent_t* ev = nullptr, int* n_launch = nullptr,
                 const char** names = nullptr);
+// mb.tube: `steps` stages (fewer when a Run ends) in one launch.
+cudaError_t mixed_resident_steps(const MixedBufs& mb, int steps, cudaStream_t st);
 // After a new state was written into U[parity]: no pending residual.
 void mixed_reset(MixedBufs& mb, cudaStream_t st);
 // Applies the pending residual so U[parity] holds the current state.
