@@ -8,13 +8,13 @@ pytestmark = pytest.mark.gpu
 SIDES = {"natural": 5, "symmetry": 1, "wall": 0, "moving": 2, "inlet": 3}
 
 
-def wave(nx, ny, nz):
+def wave(nx, ny, nz, w3=False):
     x, y, z = [(np.arange(n) + 0.5) / n for n in (nx, ny, nz)]
     Z, Y, X = np.meshgrid(z, y, x, indexing="ij")
     nd3 = nz > 1
     rho = 1.0 + 0.2 * np.sin(6 * X) * np.cos(5 * Y) + 0.1 * np.sin(4 * Z) * nd3
     p = 1.0 + 0.1 * np.cos(4 * X + 3 * Y) + 0.1 * np.cos(5 * Z) * nd3
-    v = np.stack([0.3 * np.cos(5 * Y), 0.2 * np.sin(4 * X), 0.1 * np.cos(6 * X) * nd3], -1)
+    v = np.stack([0.3 * np.cos(5 * Y), 0.2 * np.sin(4 * X), 0.1 * np.cos(6 * X) * (1.0 if w3 else nd3)], -1)
     return np.concatenate([rho[..., None], rho[..., None] * v, (p / 0.4 + 0.5 * rho * (v * v).sum(-1))[..., None]], -1)
 
 

@@ -124,6 +124,19 @@ struct Group {
     int grid = 0;
 };
 
+// 1D problems that share a launch of the resident kernel: their solver, CTAs
+// each, cells of the largest, and their place in the device list.
+struct TailGroup {
+    int solver, cluster, cells, n, first;
+};
+// Sets of 1D problems of at most this many cells in all run in the resident
+// kernel.  Measured, resident against stage launches (tubes of 64 to 4096
+// cells): 9481 cells in all, 300 stages 1.2 / 3.4 ms; 193377, 300 stages 5.7 /
+// 6.7; 285269, 200 stages 5.0 / 5.7; 353694, 200 stages 6.3 / 6.3; 3988212, 60
+// stages 25.8 / 15.0 (its two CTAs of 256 threads per SM are fewer warps than
+// the stage kernel's, and every stage waits for its cluster twice).
+constexpr long long kTailCells = 300000;
+
 // Launch policy of one dimension: a fixed tile or (tx = 0) a tile chosen per
 // problem from its x extent; ctas = resident CTAs per SM (0: as many as fit).
 struct Tune {
@@ -178,12 +191,12 @@ struct ts_batch {
     // short work lists close each problem's step in the stage kernel itself
     // (the CTA finishing a problem's last item), saving the finish launch
     bool fused_close = false;
-    // the last few long 1D problems run in the cluster tail kernel: many
-    // stages per launch, state on chip (one list per Riemann solver)
+    // sets of 1D problems run in the resident cluster kernel: many stages per
+    // launch, state on chip
     bool tail_enabled = true, tail_mode = false;
-    int tail_cluster = 0, tail_cells = 0;  // CTAs per problem, cells of the largest
-    int* d_tail[2] = {nullptr, nullptr};
-    int tail_n[2] = {0, 0}, tail_cap[2] = {0, 0};
+    std::vector<TailGroup> tails;
+    int* d_tail = nullptr;
+    int tail_cap = 0;
     Arena arena;
     std::vector<Slot> slots;
     std::vector<ProbDesc> desc;
@@ -218,8 +231,7 @@ struct ts_batch {
         drop_graphs();
         for (auto& g : groups) cudaFree(g.d_items);
         cudaFree(d_slots);
-        cudaFree(d_tail[0]);
-        cudaFree(d_tail[1]);
+        cudaFree(d_tail);
         for (int k = 0; k < kSide; ++k) {
             if (side[k]) cudaStreamDestroy(side[k]);
             if (join[k]) cudaEventDestroy(join[k]);
@@ -357,41 +369,62 @@ struct ts_batch {
         return TS_OK;
     }
 
-    // Tail mode when every unfinished problem is 1D, fits one cluster, and
-    // all clusters together fit the GPU at once (one CTA per SM); the clusters are as
-    // large as that allows.
+    // Tail mode when every unfinished problem is 1D and fits one cluster, and
+    // the set is one that the resident kernel is faster for: few enough cells
+    // (kTailCells).  While the clusters fit the GPU at one CTA per SM they are
+    // made of CTAs as small as that allows (latency), otherwise of CTAs of up to 254
+    // cells (fewer halo cells); problems of equal solver and cluster size share a launch.
     ts_status plan_tail() {
         tail_mode = false;
-        tail_n[0] = tail_n[1] = 0;
+        tails.clear();
         if (!tail_enabled) return TS_OK;
-        std::vector<int> lists[2];
-        int nact = 0;
-        tail_cells = 0;
+        std::vector<int> act;
+        long long cells = 0;
         for (int s = 0; s < capacity; ++s) {
             if (!slots[s].used || h_ctl[s].stop_req) continue;
             const ProbDesc& d = desc[s];
             // the resident kernel forms no residual norms
             if (d.L.nd != 1 || d.kn[0] < 4 || d.kn[0] > tube32_max_cells() || d.mp.norms) return TS_OK;
-            tail_cells = std::max(tail_cells, d.kn[0]);
-            lists[d.mp.solver == TS_RS_HLLC ? 1 : 0].push_back(s);
-            ++nact;
+            cells += d.kn[0];
+            act.push_back(s);
         }
-        if (nact == 0 || nact > sms) return TS_OK;
-        tail_cluster = std::min({kTailMaxCluster, sms / nact, std::max(1, tail_cells / 30)});
-        for (int k = 0; k < 2; ++k)
-            if (!lists[k].empty() && !tube32_ready(k ? TS_RS_HLLC : TS_RS_ROE_PIKE, tail_cluster, tail_cells)) return TS_OK;
-        for (int k = 0; k < 2; ++k) {
-            tail_n[k] = (int)lists[k].size();
-            if (!tail_n[k]) continue;
-            if (tail_n[k] > tail_cap[k]) {
-                cudaFree(d_tail[k]);
-                d_tail[k] = nullptr;
-                tail_cap[k] = std::max(64, tail_n[k]);
-                TB_CUDA(cudaMalloc(&d_tail[k], sizeof(int) * tail_cap[k]));
+        if (act.empty() || cells > kTailCells) return TS_OK;
+        auto ctas = [&](int s, int own) {
+            // few distinct sizes: a launch each
+            for (int c : {1, 2, 3, 4, 6, 8, 10, 12, 14})
+                if (c * own >= desc[s].kn[0]) return c;
+            return kTailMaxCluster;
+        };
+        int own = 30;
+        for (int t : {30, 62, 126, 254}) {
+            own = t;
+            long long all = 0;
+            for (int s : act) all += ctas(s, t);
+            if (all <= sms) break;
+        }
+        std::map<std::array<int, 2>, std::vector<int>> bykey;
+        for (int s : act) bykey[{desc[s].mp.solver, ctas(s, own)}].push_back(s);
+        std::vector<int> flat;
+        std::vector<TailGroup> plan;
+        for (auto& kv : bykey) {
+            TailGroup g{kv.first[0], kv.first[1], 0, (int)kv.second.size(), (int)flat.size()};
+            for (int s : kv.second) {
+                g.cells = std::max(g.cells, desc[s].kn[0]);
+                flat.push_back(s);
             }
-            TB_CUDA(cudaMemcpyAsync(d_tail[k], lists[k].data(), sizeof(int) * tail_n[k], cudaMemcpyHostToDevice,
-                                    stream));
+            if (!tube32_ready(g.solver, g.cluster, g.n, g.cells)) return TS_OK;
+            plan.push_back(g);
         }
+        if ((int)flat.size() > tail_cap) {
+            cudaFree(d_tail);
+            d_tail = nullptr;
+            tail_cap = 2 * (int)flat.size() + 64;
+            TB_CUDA(cudaMalloc(&d_tail, sizeof(int) * tail_cap));
+        }
+        TB_CUDA(cudaMemcpyAsync(d_tail, flat.data(), sizeof(int) * flat.size(), cudaMemcpyHostToDevice, stream));
+        // the largest clusters first: they are the longest
+        std::stable_sort(plan.begin(), plan.end(), [](const TailGroup& a, const TailGroup& b) { return a.cluster > b.cluster; });
+        tails.swap(plan);
         tail_mode = true;
         return TS_OK;
     }
@@ -422,24 +455,39 @@ struct ts_batch {
         ++stages;
     }
 
+    ts_status replan() {
+        stable = 0;
+        return rebuild();
+    }
+
     // Stages are launched one by one right after the work list changed (a
     // capture costs more than it saves when membership keeps changing, as in
     // a served stream); once the list has been stable for a few launches,
     // chunks of stages are captured into graphs and replayed.
     ts_status launch(int n) {
         if (dirty) {
-            ts_status s = rebuild();
+            ts_status s = replan();
             if (s != TS_OK) return s;
-            stable = 0;
         }
         if (groups.empty()) return TS_OK;
         if (tail_mode) {
-            // every tail problem advances up to n stages in one launch
-            for (int k = 0; k < 2; ++k) {
-                if (!tail_n[k]) continue;
-                TB_CUDA(tube32_launch(k ? TS_RS_HLLC : TS_RS_ROE_PIKE, tail_cluster, tail_n[k], tail_cells, d_desc,
-                                      d_tail[k], n, stream));
+            // every problem advances up to n stages in one launch of its group
+            // (the groups side by side)
+            const int ng = (int)tails.size();
+            if (ng > 1) TB_CUDA(cudaEventRecord(fork, stream));
+            for (int k = 0; k < ng; ++k) {
+                const TailGroup& g = tails[k];
+                cudaStream_t st = stream;
+                if (k % (kSide + 1)) {
+                    st = side[k % (kSide + 1) - 1];
+                    if (k <= kSide) TB_CUDA(cudaStreamWaitEvent(st, fork, 0));
+                }
+                TB_CUDA(tube32_launch(g.solver, g.cluster, g.n, g.cells, d_desc, d_tail + g.first, n, st));
                 ++launches;
+            }
+            for (int k = 0; k < std::min(ng - 1, kSide); ++k) {
+                TB_CUDA(cudaEventRecord(join[k], side[k]));
+                TB_CUDA(cudaStreamWaitEvent(stream, join[k], 0));
             }
             stages += n;
             return TS_OK;
@@ -701,7 +749,9 @@ ts_status ts_batch_run(ts_batch* b, int32_t max_stages, int32_t* active) {
         if (a == 0) break;
         if (max_stages > 0 && done >= max_stages) break;
         if (2 * ia < il) b->dirty = true;  // most listed items belong to finished problems
-        int n = chunk;
+        if (b->dirty && (s = b->replan()) != TS_OK) return s;
+        // the resident kernel's problems end by themselves
+        int n = b->tail_mode ? std::max(chunk, 1024) : chunk;
         if (max_stages > 0) n = (int)std::min<long long>(n, max_stages - done);
         if ((s = b->launch(n)) != TS_OK) return s;
         if ((s = b->pull()) != TS_OK) return s;

@@ -1083,24 +1083,27 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
     if (L.nd == 3) {
         // 16x16 tiles where they cover the grid with enough fewer columns
         // (a plane pass of theirs takes 5 % longer: 64^3 35.6 against 34.1 us;
-        // but 97x61x83 60.6 against 67.4, 200x30x120 68.6 against 75.1)
+        // but 97x61x83 60.6 against 67.4, 200x30x120 68.6 against 75.1).  The two
+        // compiled tiles give the same bits, but for first-order HLLC, which the
+        // compiler contracts differently in them: that keeps 32x8.
         const long long slots = 2LL * mb.sms;
         int z;
         auto cols = [&](int x, int y) { return (long long)((L.nx + x - 1) / x) * ((L.ny + y - 1) / y); };
-        if (1.05 * plan3d(cols(16, 16), L.nz, slots, &z) < plan3d(cols(32, 8), L.nz, slots, &z)) tx = ty = 16;
+        const bool same = d.mp.solver != TS_RS_HLLC || d.mp.recon != TS_RECON_PIECEWISE_CONSTANT;
+        if (same && 1.05 * plan3d(cols(16, 16), L.nz, slots, &z) < plan3d(cols(32, 8), L.nz, slots, &z)) tx = ty = 16;
     }
     if ((s = mixed_set_tile(mb, tx, ty, 0, err, st)) != TS_OK) return s;
     if (L.nd == 2 && L.cells() <= kFlatCells) mb.flat = flat2d_tiles(d, &d.ncx);
     if (L.nd == 1 && !d.mp.norms) {
         // about 30 cells, a warp, per CTA while the cluster has CTAs left
         const int ctas = std::min(kTailMaxCluster, std::max(1, L.nx / 30));
-        if (tube32_ready(d.mp.solver, ctas, L.nx)) mb.tube = ctas;
+        if (tube32_ready(d.mp.solver, ctas, 1, L.nx)) mb.tube = ctas;
     }
     return TS_OK;
 }
 
 cudaError_t mixed_resident_steps(const MixedBufs& mb, int steps, cudaStream_t st) {
-    return tube32_launch(mb.desc.mp.solver, mb.tube, 1, mb.desc.L.nx, mb.d_desc, nullptr, steps, st);
+    return tube32_launch_one(mb.tube, mb.desc, steps, st);
 }
 
 void mixed_step(MixedBufs& mb, const Phys&, cudaStream_t st, cudaEvent_t* ev, int* n_launch, const char** names) {

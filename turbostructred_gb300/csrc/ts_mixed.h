@@ -131,11 +131,11 @@ ts_status mixed_set_tile(MixedBufs& mb, int tx, int ty, int zchunks, std::string
 
 // 1D problems (without residual norms): up to `budget` stages in one launch, a
 // cluster of `cluster` CTAs per problem, the state on chip (ts_tube32.cu).
-// d_list: descriptor indices (null: d_probs[0] alone); cells: those of the
-// largest problem.
+// d_list: descriptor indices; cells: those of the largest problem.
 constexpr int kTailMaxCluster = 16;
 int tube32_max_cells();
-bool tube32_ready(int solver, int cluster, int cells);
+bool tube32_ready(int solver, int cluster, int problems, int cells);
+cudaError_t tube32_launch_one(int cluster, const ProbDesc& d, int budget, cudaStream_t st);
 cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, const ProbDesc* d_probs, const int* d_list,
                           int budget, cudaStream_t st);
 

@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "ts_flux32.cuh"
 #include "ts_mixed.h"
@@ -80,22 +81,30 @@ __device__ __forceinline__ float half_slope(int kind, float nm, float w0, float 
 
 // list: the problems' descriptor indices (null: descriptor 0 alone).  A
 // non-physical state ends a batched problem's loop (the host stops it).
-template <int SOLVER>
-__global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const ProbDesc* __restrict__ probs,
+// ONE: a single domain, its descriptor a kernel parameter as in k_mix_step
+// (with the descriptor in shared memory the compiler contracts the Roe
+// flux's multiply-adds differently, as it does in the batched k_mix_step: each
+// instance gives the bits of its counterpart).  Otherwise list holds the
+// problems' descriptor indices, and a non-physical state ends a
+// problem's loop (the host stops it).
+template <int SOLVER, bool ONE>
+__global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant__ ProbDesc one,
+                                                           const ProbDesc* __restrict__ probs,
                                                            const int* __restrict__ list, int budget) {
     extern __shared__ float sm[];
-    __shared__ ProbDesc d;
+    __shared__ ProbDesc sd;
     __shared__ unsigned int smax[kTailMaxCluster * kMaxWarps];
     __shared__ unsigned int shealth;
     cg::cluster_group cluster = cg::this_cluster();
     const int nblk = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, W = blockDim.x >> 5;
-    {
-        const int* src = (const int*)(probs + (list ? list[blockIdx.x / nblk] : 0));
-        for (int k = tid; k < (int)(sizeof(ProbDesc) / sizeof(int)); k += blockDim.x) ((int*)&d)[k] = src[k];
+    if (!ONE) {
+        const int* src = (const int*)(probs + list[blockIdx.x / nblk]);
+        for (int k = tid; k < (int)(sizeof(ProbDesc) / sizeof(int)); k += blockDim.x) ((int*)&sd)[k] = src[k];
         if (tid == 0) shealth = 0u;
         __syncthreads();
     }
+    const ProbDesc& d = ONE ? one : sd;
     // A finished problem that is still listed is left alone (the whole cluster
     // leaves here): it may be read back, and its memory given to another
     // problem, on other streams beside this launch.
@@ -261,7 +270,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const ProbDesc* __res
         // srmax >= 0: its bits order like unsigned integers
         const unsigned int mbits = __reduce_max_sync(0xffffffffu, __float_as_uint(srmax));
         if (remote_max) *remote_max = mbits;
-        if (list && health) {  // rare
+        if (!ONE && health) {  // rare
             for (int k = 0; k < nblk; ++k) atomicOr(cluster.map_shared_rank(&shealth, k), health);
         }
         cg::cluster_group::arrival_token second = cluster.barrier_arrive();
@@ -306,7 +315,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const ProbDesc* __res
             stop = iteration == max_iteration || time >= max_time;
         }
         const bool finished = stop;
-        if (list && shealth) stop = true;
+        if (!ONE && shealth) stop = true;
         if (rank == 0 && tid == 0 && (stop || st == budget - 1)) {
             Ctl* c = d.ctl;
             c->time = time;
@@ -335,20 +344,24 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const ProbDesc* __res
     cluster.sync();  // no CTA leaves while another may still write to it
 }
 
+int own_cells(int cluster, int cells) {
+    // (a problem with fewer than two cells per CTA leaves CTAs idle and has up
+    // to three in the others)
+    return std::max(3, (cells + cluster - 1) / cluster);
+}
+int block_threads(int cluster, int cells) { return (own_cells(cluster, cells) + 2 + 31) / 32 * 32; }
+
 template <class F>
 auto with_solver(int solver, F&& f) {
     return solver == TS_RS_HLLC ? f.template operator()<TS_RS_HLLC>() : f.template operator()<TS_RS_ROE_PIKE>();
 }
 
-template <int S>
+template <int S, bool ONE>
 cudaError_t config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
-    // (a problem with fewer than two cells per CTA leaves CTAs idle and has up
-    // to three in the others)
-    const int own = std::max(3, (cells + cluster - 1) / cluster);
     cfg = cudaLaunchConfig_t{};
     cfg.gridDim = dim3((unsigned)(cluster * problems));
-    cfg.blockDim = dim3((unsigned)((own + 2 + 31) / 32 * 32));
-    cfg.dynamicSmemBytes = sizeof(float) * Tube32Mem(own).total;
+    cfg.blockDim = dim3((unsigned)block_threads(cluster, cells));
+    cfg.dynamicSmemBytes = sizeof(float) * Tube32Mem(own_cells(cluster, cells)).total;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)cluster;
     attr[0].val.clusterDim.y = 1;
@@ -356,9 +369,9 @@ cudaError_t config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     // static and dynamic shared memory together may pass 48 KB
-    cudaError_t e = cudaFuncSetAttribute(k_tube32<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_tube32<S, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(sizeof(float) * Tube32Mem(kMaxOwn).total));
-    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k_tube32<S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k_tube32<S, ONE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 
@@ -366,30 +379,48 @@ cudaError_t config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg
 
 int tube32_max_cells() { return kTailMaxCluster * kMaxOwn; }
 
-bool tube32_ready(int solver, int cluster, int cells) {
+bool tube32_ready(int solver, int cluster, int problems, int cells) {
     if (cluster < 1 || cluster > kTailMaxCluster || cells < 4 || (cells + cluster - 1) / cluster > kMaxOwn) return false;
-    return with_solver(solver, [&]<int S>() {
+    auto fits = [&]<int S, bool ONE>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         int active = 0;
-        if (config<S>(cluster, 1, cells, cfg, attr) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&active, k_tube32<S>, &cfg) != cudaSuccess) {
+        if (config<S, ONE>(cluster, problems, cells, cfg, attr) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&active, k_tube32<S, ONE>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
         return active > 0;
+    };
+    return with_solver(solver, [&]<int S>() {
+        return fits.template operator()<S, true>() && fits.template operator()<S, false>();
+    });
+}
+
+cudaError_t tube32_launch_one(int cluster, const ProbDesc& d, int budget, cudaStream_t st) {
+    if (budget <= 0) return cudaSuccess;
+    return with_solver(d.mp.solver, [&]<int S>() {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        cudaError_t e = config<S, true>(cluster, 1, d.kn[0], cfg, attr);
+        cfg.stream = st;
+        return e != cudaSuccess ? e
+                                : cudaLaunchKernelEx(&cfg, k_tube32<S, true>, d, (const ProbDesc*)nullptr,
+                                                     (const int*)nullptr, budget);
     });
 }
 
 cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, const ProbDesc* d_probs, const int* d_list,
                           int budget, cudaStream_t st) {
     if (problems <= 0 || budget <= 0) return cudaSuccess;
+    ProbDesc none;
+    std::memset(&none, 0, sizeof none);
     return with_solver(solver, [&]<int S>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
-        cudaError_t e = config<S>(cluster, problems, cells, cfg, attr);
+        cudaError_t e = config<S, false>(cluster, problems, cells, cfg, attr);
         cfg.stream = st;
-        return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k_tube32<S>, d_probs, d_list, budget);
+        return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k_tube32<S, false>, none, d_probs, d_list, budget);
     });
 }
 
