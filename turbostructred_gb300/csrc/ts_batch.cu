@@ -86,13 +86,33 @@ public:
     }
 };
 
-__global__ void k_b_scatter(const double* __restrict__ aos, Layout L, double* __restrict__ U) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= L.cells()) return;
-    const int i = (int)(t % L.nx), j = (int)((t / L.nx) % L.ny), k = (int)(t / ((long long)L.nx * L.ny));
-    const long long c = L.at(i, j, k);
+// Puts a new problem in its place from page-locked host memory, in one launch:
+// geometry, control word and descriptor (`part`: words copied from src), the
+// state from AoS order, and no pending residual.
+struct Placing {
+    const unsigned int* src;
+    struct {
+        unsigned int* dst;
+        unsigned int at, words;
+    } part[5];
+    int parts;
+    const double* aos;
+    Layout L;
+    double* U;
+    float* R;
+};
+__global__ void k_b_place(const __grid_constant__ Placing p) {
+    const long long step = (long long)gridDim.x * blockDim.x, t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (int k = 0; k < p.parts; ++k)
+        for (long long t = t0; t < p.part[k].words; t += step) p.part[k].dst[t] = p.src[p.part[k].at + t];
+    for (long long t = t0; t < NV * p.L.plane; t += step) p.R[t] = 0.0f;
+    const Layout& L = p.L;
+    for (long long t = t0; t < L.cells(); t += step) {
+        const int i = (int)(t % L.nx), j = (int)((t / L.nx) % L.ny), k = (int)(t / ((long long)L.nx * L.ny));
+        const long long c = L.at(i, j, k);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) U[(long long)v * L.plane + c] = aos[t * NV + v];
+        for (int v = 0; v < NV; ++v) p.U[(long long)v * L.plane + c] = p.aos[t * NV + v];
+    }
 }
 
 // Interior cells of problem p's current state to AoS order.
@@ -220,6 +240,12 @@ struct ts_batch {
     size_t ustage_doubles = 0;
     double* dstage = nullptr;
     size_t dstage_doubles = 0;
+    // page-locked staging: new problems are copied to up_h in turn and put in
+    // place from there by a kernel on the upload stream (which has drained
+    // before the buffer starts over); results are read into down_h
+    static constexpr size_t kStage = size_t(8) << 20;
+    char *up_h = nullptr, *down_h = nullptr;
+    size_t up_size = 0, up_used = 0;
     std::vector<int> quarantine;  // removed slots, reusable once the main stream has drained
     double done_cell_updates = 0.0;  // of removed problems
     long long stages = 0, launches = 0;
@@ -242,6 +268,8 @@ struct ts_batch {
         cudaFreeHost(h_ctl);
         cudaFree(ustage);
         cudaFree(dstage);
+        cudaFreeHost(up_h);
+        cudaFreeHost(down_h);
         if (ustream) cudaStreamDestroy(ustream);
         if (dstream) cudaStreamDestroy(dstream);
         if (uploaded) cudaEventDestroy(uploaded);
@@ -609,6 +637,9 @@ ts_status ts_batch_create(int32_t device, size_t budget, ts_batch** out) {
     TB_CUDA(cudaStreamCreateWithFlags(&b->dstream, cudaStreamNonBlocking));
     TB_CUDA(cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming));
     TB_CUDA(b->arena.init(budget));
+    TB_CUDA(cudaHostAlloc((void**)&b->up_h, ts_batch::kStage, cudaHostAllocDefault));
+    b->up_size = ts_batch::kStage;
+    TB_CUDA(cudaHostAlloc((void**)&b->down_h, ts_batch::kStage, cudaHostAllocDefault));
     ts_status s = b->grow(64);
     if (s != TS_OK) return s;
     *out = b.release();
@@ -657,7 +688,43 @@ ts_status ts_batch_add(ts_batch* b, const ts_config* cfg, const double* values, 
     auto undo = [&]() { for (void* p : sl.mem) b->arena.give(p); sl = Slot(); };
     ProbDesc& d = b->desc[slot];
     std::memset(&d, 0, sizeof d);
-    if ((s = mixed_problem(*cfg, L, ph, grid, b->d_ctl + slot, take, d, err, b->ustream)) != TS_OK) {
+    // everything but a large state goes through one block of the page-locked
+    // staging buffer and one launch; a state that is page-locked already is read
+    // in place, a large one through device memory, and both are waited for
+    cudaStream_t us = b->ustream;
+    const size_t nvals = (size_t)L.cells() * NV;
+    const double* pinned = static_cast<const double*>(pinned_device_ptr(values, b->device));
+    const bool staged = !pinned && nvals * sizeof(double) <= ts_batch::kStage / 2;
+    const size_t geo = sizeof(AxisGeo) * ((L.nx + 2 * L.gx) + (L.ny + 2 * L.gy) + (L.nz + 2 * L.gz));
+    const size_t block = geo + sizeof(Ctl) + sizeof(ProbDesc) + (staged ? nvals * sizeof(double) : 0) + 16 * 16;
+    if (b->up_used + block > b->up_size) {
+        TB_CUDA(cudaStreamSynchronize(us));
+        b->up_used = 0;
+        if (block > b->up_size) {  // the geometry of a very long grid
+            cudaFreeHost(b->up_h);
+            b->up_h = nullptr;
+            b->up_size = 0;
+            TB_CUDA(cudaHostAlloc((void**)&b->up_h, block, cudaHostAllocDefault));
+            b->up_size = block;
+        }
+    }
+    Placing pl{};
+    pl.src = reinterpret_cast<const unsigned int*>(b->up_h);
+    auto put = [&](const void* src, size_t bytes) {
+        char* at = b->up_h + b->up_used;
+        std::memcpy(at, src, bytes);
+        b->up_used += (bytes + 15) / 16 * 16;
+        return at;
+    };
+    auto upload = [&](void* dst, const void* src, size_t bytes) {
+        if (pl.parts >= 5) return false;
+        auto& p = pl.part[pl.parts++];
+        p.at = (unsigned)((put(src, bytes) - b->up_h) / sizeof(int));
+        p.dst = static_cast<unsigned int*>(dst);
+        p.words = (unsigned)(bytes / sizeof(int));
+        return true;
+    };
+    if ((s = mixed_problem(*cfg, L, ph, grid, b->d_ctl + slot, take, upload, d, err)) != TS_OK) {
         undo();
         return err.empty() ? s : fail(s, err);
     }
@@ -666,24 +733,6 @@ ts_status ts_batch_add(ts_batch* b, const ts_config* cfg, const double* values, 
         if ((s = take(sizeof(float) * NV * L.plane, (void**)&d.R[k])) != TS_OK) { undo(); return s; }
     }
     b->place(slot);
-    // initial state: host -> staging -> U[0] (page-locked host memory is read
-    // in place); no pending residual.  All on the upload stream; the main
-    // stream waits for it before its next work, so stages already queued
-    // there keep running meanwhile.
-    const size_t nvals = (size_t)L.cells() * NV;
-    const double* pinned = static_cast<const double*>(pinned_device_ptr(values, b->device));
-    if (!pinned && b->ustage_doubles < nvals) {
-        TB_CUDA(cudaStreamSynchronize(b->ustream));
-        cudaFree(b->ustage);
-        b->ustage = nullptr;
-        b->ustage_doubles = 0;
-        if (cudaMalloc(&b->ustage, nvals * sizeof(double)) != cudaSuccess) { undo(); return fail(TS_ERR_NO_MEMORY, "staging buffer"); }
-        b->ustage_doubles = nvals;
-    }
-    cudaStream_t us = b->ustream;
-    if (!pinned) TB_CUDA(cudaMemcpyAsync(b->ustage, values, nvals * sizeof(double), cudaMemcpyHostToDevice, us));
-    k_b_scatter<<<(unsigned)((L.cells() + 255) / 256), 256, 0, us>>>(pinned ? pinned : b->ustage, L, d.U[0]);
-    TB_CUDA(cudaMemsetAsync(d.R[0], 0, sizeof(float) * NV * L.plane, us));
     Ctl& c = b->h_ctl[slot];
     std::memset(&c, 0, sizeof c);
     c.next_sol = cfg->save_solution_time;
@@ -693,13 +742,35 @@ ts_status ts_batch_add(ts_batch* b, const ts_config* cfg, const double* values, 
     c.max_iteration = cfg->max_iteration;
     c.max_time = cfg->max_time;
     c.run_mode = 1;
-    TB_CUDA(cudaMemcpyAsync(b->d_ctl + slot, &c, sizeof(Ctl), cudaMemcpyHostToDevice, us));
-    TB_CUDA(cudaMemcpyAsync(b->d_desc + slot, &d, sizeof(ProbDesc), cudaMemcpyHostToDevice, us));
+    upload(b->d_ctl + slot, &c, sizeof c);
+    upload(b->d_desc + slot, &d, sizeof d);
+    if (pinned) {
+        pl.aos = pinned;
+    } else if (staged) {
+        pl.aos = reinterpret_cast<const double*>(put(values, nvals * sizeof(double)));
+    } else {
+        if (b->ustage_doubles < nvals) {
+            TB_CUDA(cudaStreamSynchronize(us));
+            cudaFree(b->ustage);
+            b->ustage = nullptr;
+            b->ustage_doubles = 0;
+            if (cudaMalloc(&b->ustage, nvals * sizeof(double)) != cudaSuccess) { undo(); return fail(TS_ERR_NO_MEMORY, "staging buffer"); }
+            b->ustage_doubles = nvals;
+        }
+        TB_CUDA(cudaMemcpyAsync(b->ustage, values, nvals * sizeof(double), cudaMemcpyHostToDevice, us));
+        pl.aos = b->ustage;
+    }
+    pl.L = L;
+    pl.U = d.U[0];
+    pl.R = d.R[0];
+    // on the upload stream; the main stream waits for it before its next work, so
+    // stages already queued there keep running meanwhile
+    k_b_place<<<(unsigned)std::min<long long>((NV * L.plane + 255) / 256, 2048), 256, 0, us>>>(pl);
+    TB_CUDA(cudaGetLastError());
     TB_CUDA(cudaEventRecord(b->uploaded, us));
     TB_CUDA(cudaStreamWaitEvent(b->stream, b->uploaded, 0));
-    // the caller may reuse `values` on return; the upload stream only (not the
-    // stages queued on the main stream) has to finish for that
-    TB_CUDA(cudaStreamSynchronize(us));
+    // the caller may reuse `values` on return
+    if (!staged) TB_CUDA(cudaStreamSynchronize(us));
     sl.used = true;
     sl.id = b->next_id++;
     sl.cells = L.cells();
@@ -788,14 +859,13 @@ ts_status ts_batch_get(ts_batch* b, int32_t id, double* values, ts_step_info* in
     // the main stream; a running one is read in stream order.
     const bool finished = b->h_ctl[slot].stop_req != 0;
     cudaStream_t st = finished ? b->dstream : b->stream;
-    mixed_apply(b->d_desc, slot, L.cells(), st);
+    const size_t nvals = (size_t)L.cells() * NV;
     double* pinned = values ? static_cast<double*>(pinned_device_ptr(values, b->device)) : nullptr;
-    if (values && pinned) {
-        // page-locked host memory: gathered in place
-        k_b_gather<<<blocks, 256, 0, st>>>(pinned, b->d_desc, slot);
-        TB_CUDA(cudaGetLastError());
-    } else if (values) {
-        const size_t nvals = (size_t)L.cells() * NV;
+    // page-locked host memory is written in place, a small result through the
+    // page-locked staging buffer
+    const bool staged = values && !pinned && nvals * sizeof(double) <= ts_batch::kStage;
+    double* dst = pinned ? pinned : reinterpret_cast<double*>(b->down_h);
+    if (values && !pinned && !staged) {
         if (b->dstage_doubles < nvals) {
             cudaFree(b->dstage);
             b->dstage = nullptr;
@@ -803,14 +873,25 @@ ts_status ts_batch_get(ts_batch* b, int32_t id, double* values, ts_step_info* in
             TB_CUDA(cudaMalloc(&b->dstage, nvals * sizeof(double)));
             b->dstage_doubles = nvals;
         }
-        k_b_gather<<<blocks, 256, 0, st>>>(b->dstage, b->d_desc, slot);
-        TB_CUDA(cudaGetLastError());
-        TB_CUDA(cudaMemcpyAsync(values, b->dstage, nvals * sizeof(double), cudaMemcpyDeviceToHost, st));
+        dst = b->dstage;
     }
+    if (finished) {
+        if (values) mixed_read(b->d_desc, slot, L.cells(), dst, st);
+    } else {
+        mixed_apply(b->d_desc, slot, L.cells(), st);
+        if (values) k_b_gather<<<blocks, 256, 0, st>>>(dst, b->d_desc, slot);
+    }
+    TB_CUDA(cudaGetLastError());
+    if (values && !pinned && !staged)
+        TB_CUDA(cudaMemcpyAsync(values, b->dstage, nvals * sizeof(double), cudaMemcpyDeviceToHost, st));
     ts_status s = TS_OK;
-    if (finished) TB_CUDA(cudaStreamSynchronize(st));
-    else s = b->pull();
+    if (finished) {
+        if (values) TB_CUDA(cudaStreamSynchronize(st));
+    } else {
+        s = b->pull();
+    }
     if (s != TS_OK) return s;
+    if (staged) std::memcpy(values, b->down_h, nvals * sizeof(double));
     if (info) {
         const Ctl& c = b->h_ctl[slot];
         info->iteration = c.iteration;

@@ -753,6 +753,24 @@ __global__ void k_mix_apply(const ProbDesc* __restrict__ probs, int p) {
     }
 }
 
+// The state that k_mix_apply would leave, to AoS order.
+__global__ void k_mix_read(const ProbDesc* __restrict__ probs, int p, double* __restrict__ out) {
+    const ProbDesc& d = probs[p];
+    const Layout& L = d.L;
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= L.cells()) return;
+    const int i = (int)(t % L.nx), j = (int)((t / L.nx) % L.ny), k = (int)(t / ((long long)L.nx * L.ny));
+    const long long c = L.at(i, j, k);
+    const int a1 = L.nd == 3 ? j : 0, a2 = L.nd == 3 ? k : (L.nd == 2 ? j : 0);
+    const int par = d.ctl->parity;
+    const float dtf = __double2float_rn(d.ctl->dt_apply);
+    const float cf = (d.kgeo[0][i + d.kgoff[0]].ih * d.kgeo[1][a1 + d.kgoff[1]].ih) *
+                     (dtf * d.kgeo[2][a2 + d.kgoff[2]].ih);
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+        out[t * NV + v] = d.U[par][(long long)v * L.plane + c] + f32_to_f64(cf * d.R[par][(long long)v * L.plane + c]);
+}
+
 __global__ void k_mix_clear_pending(const ProbDesc* __restrict__ probs, int p) { probs[p].ctl->dt_apply = 0.0; }
 
 // Closes the stage of every listed problem that ran (batches): dt from its
@@ -940,7 +958,7 @@ ts_status mixed_set_tile(MixedBufs& mb, int tx, int ty, int zchunks, std::string
 }
 
 ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, const HostGrid& g, Ctl* ctl,
-                        const DeviceAlloc& alloc, ProbDesc& d, std::string& err, cudaStream_t st) {
+                        const DeviceAlloc& alloc, const DeviceUpload& upload, ProbDesc& d, std::string& err) {
     if (L.plane > (1LL << 31) - 1) { err = "grid too large for the mixed path"; return TS_ERR_INVALID; }
     d.L = L;
     d.ctl = ctl;
@@ -981,8 +999,7 @@ ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, con
         }
         void* p;
         if ((s = alloc(sizeof(AxisGeo) * geo.size(), &p)) != TS_OK) return s;
-        // pageable source: staged before the call returns, so `geo` may go
-        if (cudaMemcpyAsync(p, geo.data(), sizeof(AxisGeo) * geo.size(), cudaMemcpyHostToDevice, st) != cudaSuccess) {
+        if (!upload(p, geo.data(), sizeof(AxisGeo) * geo.size())) {
             err = "geometry upload failed";
             return TS_ERR_CUDA;
         }
@@ -1041,7 +1058,7 @@ ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, con
     if (marked) {
         void* p;
         if ((s = alloc(sizeof(MixBcKinds), &p)) != TS_OK) return s;
-        if (cudaMemcpyAsync(p, &kinds, sizeof kinds, cudaMemcpyHostToDevice, st) != cudaSuccess) {
+        if (!upload(p, &kinds, sizeof kinds)) {
             err = "boundary-condition table upload failed";
             return TS_ERR_CUDA;
         }
@@ -1062,7 +1079,11 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
     ts_status s;
     ProbDesc& d = mb.desc;
     std::memset(&d, 0, sizeof d);
-    if ((s = mixed_problem(c, L, ph, g, ctl, alloc, d, err, st)) != TS_OK) return s;
+    // pageable sources: staged before the call returns
+    auto upload = [st](void* dst, const void* src, size_t bytes) {
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
+    };
+    if ((s = mixed_problem(c, L, ph, g, ctl, alloc, upload, d, err)) != TS_OK) return s;
     for (int b = 0; b < 2; ++b) {
         if ((s = alloc(sizeof(double) * NV * L.plane, (void**)&d.U[b])) != TS_OK) return s;
         if ((s = alloc(sizeof(float) * NV * L.plane, (void**)&d.R[b])) != TS_OK) return s;
@@ -1125,6 +1146,10 @@ void mixed_reset(MixedBufs& mb, cudaStream_t st) {
 void mixed_apply(const ProbDesc* d_probs, int p, long long cells, cudaStream_t st) {
     k_mix_apply<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(d_probs, p);
     k_mix_clear_pending<<<1, 1, 0, st>>>(d_probs, p);
+}
+
+void mixed_read(const ProbDesc* d_probs, int p, long long cells, double* out, cudaStream_t st) {
+    k_mix_read<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(d_probs, p, out);
 }
 
 void mixed_batch_finish(const ProbDesc* d_probs, const int* d_slots, int n, cudaStream_t st) {

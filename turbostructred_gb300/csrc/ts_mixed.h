@@ -94,10 +94,12 @@ struct MixedBufs {
 
 using DeviceAlloc = std::function<ts_status(size_t bytes, void** out)>;
 
-// Geometry and physics of one problem (host work + uploads through `alloc`,
-// queued on stream `st`: work queued there later sees them).
+// Copies host bytes to device memory from `alloc`; the source may go when it returns.
+using DeviceUpload = std::function<bool(void* dst, const void* src, size_t bytes)>;
+
+// Geometry and physics of one problem (host work + uploads).
 ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, const HostGrid& g, Ctl* ctl,
-                        const DeviceAlloc& alloc, ProbDesc& d, std::string& err, cudaStream_t st);
+                        const DeviceAlloc& alloc, const DeviceUpload& upload, ProbDesc& d, std::string& err);
 // Cells per tile along x and y of a compiled tile of tx x ty threads (one-row
 // tiles of 1D and 2D problems own tx - 4 cells).
 void mixed_tile_cells(int nd, int tx, int ty, int* cx, int* cy);
@@ -162,6 +164,9 @@ void mixed_reset(MixedBufs& mb, cudaStream_t st);
 void mixed_materialize(MixedBufs& mb, const Phys& ph, cudaStream_t st);
 // The same for problem p of a device descriptor array.
 void mixed_apply(const ProbDesc* d_probs, int p, long long cells, cudaStream_t st);
+// The current state of problem p (pending residual applied, the problem left
+// as it is) in AoS order, into device or page-locked host memory.
+void mixed_read(const ProbDesc* d_probs, int p, long long cells, double* out, cudaStream_t st);
 // Current state buffer (host must have pulled ctl->parity).
 double* mixed_state(MixedBufs& mb, int parity);
 
