@@ -81,3 +81,26 @@ def test_3d_short_marches(n, tslib):
     for per in ((0, 0, 0), (1, 1, 1)):
         both(capi.make_case(ndims=3, nx=n[0], ny=n[1], nz=n[2], periodic=per, recon=3, solver=1, cfl=0.4,
                             bc=kinds("symmetry")), wave(*n), 5)
+
+
+@pytest.mark.parametrize("sizes", [((40, 3),), ((64, 64), (130, 65), (33, 200)), ((300, 300),) * 40])
+def test_batch_rows_per_item(sizes, tslib):
+    """2D problems of a batch, whose items get shorter as the set gets smaller (problems that end one after the
+    other), against each alone in a batch: the same bits whatever the split."""
+    from turbostructred_gb300 import capi
+    probs = [(capi.make_case(ndims=2, nx=n, ny=m, periodic=(k % 2, 0, 1), recon=3 * (k % 3 > 0), solver=1 + 2 * (k % 2),
+                             cfl=0.4, max_iter=10 + 7 * k, max_time=1e30, bc=kinds("symmetry")), wave(n, m, 1))
+             for k, (n, m) in enumerate(sizes[:8])] + \
+            [(capi.make_case(ndims=2, nx=n, ny=m, periodic=(1, 1, 1), recon=0, solver=1, cfl=0.4, max_iter=9, max_time=1e30),
+              wave(n, m, 1)) for n, m in sizes[8:]]
+    with capi.Batch(512 << 20) as b:
+        ids = [b.add(c, v) for c, v in probs]
+        b.run()
+        res = [b.get(i) for i in ids]
+    for k in range(min(8, len(probs))):
+        with capi.Batch(64 << 20) as b:
+            i = b.add(*probs[k])
+            b.run()
+            got, info = b.get(i)
+        assert info["iteration"] == 10 + 7 * k
+        assert np.array_equal(got, res[k][0]) and info["time"] == res[k][1]["time"]

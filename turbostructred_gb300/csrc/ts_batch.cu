@@ -166,7 +166,12 @@ struct Tune {
 // One-row tiles compiled for batched problems (threads along x).
 const int kTiles1D[3] = {512, 256, 128};
 const int kTiles2D[3] = {260, 132, 68};
-constexpr int kRowsPerItem = 64;  // marching-axis rows per work item of a 2D problem
+// Marching-axis rows per work item of a 2D problem: 64 when the listed
+// problems fill the CTA slots with such items, else the fewest with which
+// all items still run at once (a stage of a small set ends with its longest
+// march: 24 problems of 64^2 to 512^2 are 250 items of 64 rows for 760 slots).
+constexpr int kRowsPerItem[] = {1, 2, 3, 4, 6, 8, 11, 16, 22, 32, 44, 64};
+constexpr int kMostRows = 64;
 // Work lists of at most this many items close each problem's step inside the
 // stage kernel; longer lists use the separate finish kernel.
 constexpr long long kFusedCloseItems = 1024;
@@ -229,6 +234,8 @@ struct ts_batch {
     std::vector<Group> groups;
     bool dirty = true;
     int stable = 0;  // launches since the work list last changed
+    int rows = kMostRows;  // per work item of a 2D problem
+    std::map<std::array<int, 3>, int> resident;  // CTAs per SM of a tile and solver
     std::map<int, cudaGraphExec_t> graphs;
     Tune tune[4] = {{0, 0, 0}, {0, 1, 0}, {0, 1, 0}, {0, 0, 0}};
     // uploads of admitted problems and read-backs of finished ones run on
@@ -319,13 +326,57 @@ struct ts_batch {
         return TS_OK;
     }
 
-    int per_sm(const Group& g) const {
-        size_t b;
-        int n = 0;
-        mixed_tile_info(g.nd, g.tx, g.ty, g.solver, &b, &n, true);
+    int per_sm(const Group& g) {
+        int& n0 = resident[{g.nd, g.tx, g.solver}];  // asked for once
+        if (!n0) {
+            size_t b;
+            mixed_tile_info(g.nd, g.tx, g.ty, g.solver, &b, &n0, true);
+        }
+        int n = n0;
         if (tune[g.nd].ctas > 0) n = std::min(n, tune[g.nd].ctas);
         return std::max(n, 0);
     }
+
+    // Marching chunks of ny rows in items of about `rows`.
+    static int chunks_of(int ny, int rows) {
+        return rows == kMostRows ? std::max(1, ny / rows) : (ny + rows - 1) / rows;
+    }
+
+    // The rows per item for the unfinished 2D problems; their items are dealt
+    // again when it changes.
+    ts_status plan_rows() {
+        long long slots = 0;
+        std::vector<int> act;
+        for (int s = 0; s < capacity; ++s)
+            if (slots_used(s) && desc[s].L.nd == 2) act.push_back(s);
+        if (act.empty()) return TS_OK;
+        for (int s : act) {
+            Group g;
+            g.nd = 2;
+            g.solver = desc[s].mp.solver;
+            g.tx = this->slots[s].tx;
+            g.ty = 1;
+            const long long n = (long long)per_sm(g) * sms;
+            slots = slots ? std::min(slots, n) : n;
+        }
+        int want = kMostRows;
+        for (int r : kRowsPerItem) {
+            long long items = 0;
+            for (int s : act) items += (long long)desc[s].ncol * chunks_of(desc[s].kn[2], r);
+            if (items <= slots) {
+                want = r;
+                break;
+            }
+        }
+        if (want == rows) return TS_OK;
+        rows = want;
+        for (int s : act) {
+            place(s);
+            TB_CUDA(cudaMemcpyAsync(d_desc + s, &desc[s], sizeof(ProbDesc), cudaMemcpyHostToDevice, stream));
+        }
+        return TS_OK;
+    }
+    bool slots_used(int s) const { return slots[s].used && slots[s].id >= 0 && !h_ctl[s].stop_req; }
 
     // Tile of a problem under the current policy, and its work items.
     void place(int s) {
@@ -333,13 +384,15 @@ struct ts_batch {
         const int nd = d.L.nd;
         slots[s].tx = tune[nd].tx > 0 ? tune[nd].tx : pick_tile(nd, d.kn[0]);
         slots[s].ty = 1;
-        const int chunks = nd >= 2 ? std::max(1, d.kn[2] / kRowsPerItem) : 1;
+        const int chunks = nd >= 2 ? chunks_of(d.kn[2], rows) : 1;
         mixed_items(d, slots[s].tx, 1, chunks, (long long)sms);
     }
 
     // Work items of unfinished problems, grouped by (nd, solver), each group
     // sorted by problem size, largest first.
     ts_status rebuild() {
+        ts_status rs = plan_rows();
+        if (rs != TS_OK) return rs;
         std::map<std::array<int, 4>, std::vector<int>> bykey;
         for (int s = 0; s < capacity; ++s) {
             if (!slots[s].used || h_ctl[s].stop_req) continue;
