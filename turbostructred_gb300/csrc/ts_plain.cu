@@ -562,6 +562,13 @@ __device__ __forceinline__ double face_area(const PlainBufs& b, int nd, int a, i
     return hx * hy;
 }
 
+template <class O>
+__device__ __forceinline__ double face_area_of(int nd, int a, double hx, double hy, double hz, O& o) {
+    if (a == 0) return nd == 1 ? 1.0 : (nd == 2 ? hy : o.mul(hy, hz));
+    if (a == 1) return nd == 2 ? hx : o.mul(hx, hz);
+    return o.mul(hx, hy);
+}
+
 // Face-centred sample of a cell's reconstruction (SampleSolution) at its high
 // (HI) or low face along axis a; h is the cell size the reference samples
 // with.
@@ -660,9 +667,41 @@ __global__ void __launch_bounds__(kPlainBlock, ND == 3 ? 4 : 1) k_flux(const __g
     }
 }
 
-// Spectral radius per cell in the reference's accumulation order (x-left,
-// x-right, y-left, ...), V/SR, block min by warp shuffles; the high-side
-// ghost cells, whose SR is their single face term, join the min.  The last
+// Bits of V/SR of a cell (the least of its own and of the high-side ghost
+// cells', whose SR is their single face term), SR in the reference's
+// accumulation order (x-left, x-right, y-left, ...).
+template <int ND, class O>
+__device__ __forceinline__ u64 dt_cell(const PlainBufs& b, const Phys& ph, int i, int j, int k, O& o) {
+    const Layout& L = b.L;
+    const long long c = L.at(i, j, k);
+    const double hx = b.ch[0][i + L.gx], hy = b.ch[1][j + L.gy], hz = b.ch[2][k + L.gz];
+    const double V = o.mul(o.mul(hx, hy), hz);
+    double sr = 0.0;
+    u64 r = kInfBits;
+    const int ix[3] = {i, j, k};
+#pragma unroll
+    for (int a = 0; a < ND; ++a) {
+        const double fS = face_area_of(ND, a, hx, hy, hz, o);
+        const long long st = L.stride(a);
+        const double lo = o.mul(fS, b.Lam[a][c]), hi = o.mul(fS, b.Lam[a][c + st]);
+        sr = a == 0 ? lo : sr + lo;
+        sr += hi;
+        if (ph.visc != 0.0) sr += b.VSR[a][c + st];
+        if (ix[a] == L.n(a) - 1) {
+            double hg[3] = {hx, hy, hz};
+            hg[a] = b.ch[a][L.n(a) + (a == 0 ? L.gx : (a == 1 ? L.gy : L.gz))];
+            r = umin64(r, ratio_bits(hg[0] * hg[1] * hg[2], hi));
+        }
+    }
+    return umin64(r, ratio_bits(V, sr));
+}
+template <int ND>
+__device__ __noinline__ u64 dt_plain(const PlainBufs& b, const Phys& ph, int i, int j, int k) {
+    Plain o;
+    return dt_cell<ND, Plain>(b, ph, i, j, k, o);
+}
+
+// V/SR of every cell, block min by warp shuffles.  The last
 // block to finish reduces the block minima and sets dt.
 template <int ND>
 __global__ void __launch_bounds__(kPlainBlock) k_dt(const __grid_constant__ PlainBufs b,
@@ -674,26 +713,10 @@ __global__ void __launch_bounds__(kPlainBlock) k_dt(const __grid_constant__ Plai
     for (unsigned t = blockIdx.x * kPlainBlock + threadIdx.x; t < cells; t += step) {
         int i, j, k;
         cell_of(L, t, i, j, k);
-        const long long c = L.at(i, j, k);
-        const double hx = b.ch[0][i + L.gx], hy = b.ch[1][j + L.gy], hz = b.ch[2][k + L.gz];
-        const double V = hx * hy * hz;
-        double sr = 0.0;
-        const int ix[3] = {i, j, k};
-#pragma unroll
-        for (int a = 0; a < ND; ++a) {
-            const double fS = face_area(b, ND, a, i, j, k);
-            const long long st = L.stride(a);
-            const double lo = fS * b.Lam[a][c], hi = fS * b.Lam[a][c + st];
-            sr = a == 0 ? lo : sr + lo;
-            sr += hi;
-            if (ph.visc != 0.0) sr += b.VSR[a][c + st];
-            if (ix[a] == L.n(a) - 1) {
-                double hg[3] = {hx, hy, hz};
-                hg[a] = b.ch[a][L.n(a) + (a == 0 ? L.gx : (a == 1 ? L.gy : L.gz))];
-                r = umin64(r, ratio_bits(hg[0] * hg[1] * hg[2], hi));
-            }
-        }
-        r = umin64(r, ratio_bits(V, sr));
+        FastMul o;
+        u64 mine = dt_cell<ND, FastMul>(b, ph, i, j, k, o);
+        if (o.bad) mine = dt_plain<ND>(b, ph, i, j, k);
+        r = umin64(r, mine);
         if (step > cells - t) break;  // t + step would not fit 32 bits for the largest grids
     }
     __shared__ u64 wmin[kPlainBlock / 32];
@@ -741,13 +764,13 @@ __device__ __forceinline__ void update_cell(const PlainBufs& b, const Phys& ph, 
     const Layout& L = b.L;
     const long long c = L.at(i, j, k);
     const double hx = b.ch[0][i + L.gx], hy = b.ch[1][j + L.gy], hz = b.ch[2][k + L.gz];
-    const double V = hx * hy * hz;
+    const double V = o.mul(o.mul(hx, hy), hz);
     double R[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) R[v] = 0.0;
 #pragma unroll
     for (int a = 0; a < ND; ++a) {
-        const double fS = face_area(b, ND, a, i, j, k);
+        const double fS = face_area_of(ND, a, hx, hy, hz, o);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             const double* F = b.F[a] + vidx(L, v) + c;
@@ -755,7 +778,7 @@ __device__ __forceinline__ void update_cell(const PlainBufs& b, const Phys& ph, 
             // equal (finite) fluxes: the difference is a zero
             if (__double_as_longlong(fh) == __double_as_longlong(fl) && (__double2hiint(fh) & 0x7FF00000) != 0x7FF00000)
                 continue;
-            const double d = (fh - fl) * fS;
+            const double d = o.mul(fh - fl, fS);
             R[v] = a == 0 ? dneg_of(d) : R[v] - d;
         }
     }
@@ -787,8 +810,8 @@ __device__ __forceinline__ void update_cell(const PlainBufs& b, const Phys& ph, 
         u[v] = uo[v];
         nrm[v] = 0.0;
         if (dzero(R[v])) continue;
-        u[v] = uo[v] + dt * o.over(R[v], iv);
-        nrm[v] = V * dabs(R[v]);
+        u[v] = uo[v] + o.mul(dt, o.over(R[v], iv));
+        nrm[v] = o.mul(V, dabs(R[v]));
     }
 }
 template <int ND>
@@ -817,8 +840,8 @@ __global__ void __launch_bounds__(kPlainBlock) k_update(const __grid_constant__ 
         cell_of(L, t, i, j, k);
         const long long c = L.at(i, j, k);
         double u[NV], nrm[NV];
-        Fast o;
-        update_cell<ND, Fast>(b, ph, i, j, k, dt, u, nrm, o);
+        FastMul o;
+        update_cell<ND, FastMul>(b, ph, i, j, k, dt, u, nrm, o);
         if (o.bad) {
             double w[NV], m[NV];
             update_plain<ND>(b, ph, i, j, k, dt, w, m);
