@@ -165,7 +165,7 @@ struct Tune {
 
 // One-row tiles compiled for batched problems (threads along x).
 const int kTiles1D[3] = {512, 256, 128};
-const int kTiles2D[3] = {260, 132, 68};
+const int kTiles2D[5] = {260, 132, 96, 68, 64};
 // Marching-axis rows per work item of a 2D problem: 64 when the listed
 // problems fill the CTA slots with such items, else the fewest with which
 // all items still run at once (a stage of a small set ends with its longest
@@ -180,11 +180,19 @@ constexpr long long kFusedCloseItems = 1024;
 // covers the row with the fewest warp-slots per cell, charging each column
 // ~4 warps of fixed cost (setup, barriers, close).
 int pick_tile(int nd, int nx) {
-    // 2D: the 132-thread tile (128 cells, five resident CTAs per SM) measured
-    // fastest on mixed-size batches of 256^2-1024^2 problems (autotuner: 1.94e10
-    // against 1.75e10 cell-updates/s for the 260-thread tile); the 68-thread
-    // tile for rows that fit it
-    if (nd == 2) return nx <= 64 ? 68 : 132;
+    // 2D: the row that covers nx cells with the fewest warps (the threads beyond a
+    // multiple of 32 cost a warp: 132 threads five for 128 cells, 64 threads two
+    // for 60, 96 three for 92)
+    if (nd == 2) {
+        int best = 132, least = 1 << 30;
+        for (int t : {132, 96, 68, 64}) {
+            int cx, cy;
+            mixed_tile_cells(nd, t, 1, &cx, &cy);
+            const int warps = (nx + cx - 1) / cx * ((t + 31) / 32);
+            if (warps < least) { least = warps; best = t; }
+        }
+        return best;
+    }
     const int* c = kTiles1D;
     int best = c[0];
     double best_cost = 1e300;
@@ -345,25 +353,16 @@ struct ts_batch {
     // The rows per item for the unfinished 2D problems; their items are dealt
     // again when it changes.
     ts_status plan_rows() {
-        long long slots = 0;
         std::vector<int> act;
         for (int s = 0; s < capacity; ++s)
             if (slots_used(s) && desc[s].L.nd == 2) act.push_back(s);
         if (act.empty()) return TS_OK;
-        for (int s : act) {
-            Group g;
-            g.nd = 2;
-            g.solver = desc[s].mp.solver;
-            g.tx = this->slots[s].tx;
-            g.ty = 1;
-            const long long n = (long long)per_sm(g) * sms;
-            slots = slots ? std::min(slots, n) : n;
-        }
         int want = kMostRows;
         for (int r : kRowsPerItem) {
-            long long items = 0;
-            for (int s : act) items += (long long)desc[s].ncol * chunks_of(desc[s].kn[2], r);
-            if (items <= slots) {
+            long long warps = 0;
+            for (int s : act)
+                warps += (long long)desc[s].ncol * chunks_of(desc[s].kn[2], r) * ((slots[s].tx + 31) / 32);
+            if (warps <= 24LL * sms) {  // what the marching tiles are compiled for
                 want = r;
                 break;
             }
@@ -1044,7 +1043,8 @@ ts_status ts_batch_autotune(ts_batch* b, int32_t stages, int32_t* tx_out, int32_
     // each with as many resident CTAs as fit, and capped at 2 and 1
     std::vector<Tune> cand;
     const int* tiles = nd == 1 ? kTiles1D : kTiles2D;
-    for (int k = -1; k < 3; ++k) {
+    const int n_tiles = nd == 1 ? 3 : 5;
+    for (int k = -1; k < n_tiles; ++k) {
         const int tx = k < 0 ? 0 : tiles[k];
         size_t bytes;
         int per = 0;

@@ -785,7 +785,7 @@ __global__ void k_batch_finish(const ProbDesc* __restrict__ probs, const int* __
 
 // Compiled tiles: (problem dimension, threads).  2D: one-row tiles marching
 // y.  1D: one-row tiles, one plane.  (3D problems run k_mix3d.)
-#define TS_MIXED_TILES_2D(X) X(2, 260) X(2, 132) X(2, 68)
+#define TS_MIXED_TILES_2D(X) X(2, 260) X(2, 132) X(2, 96) X(2, 68) X(2, 64)
 #define TS_MIXED_TILES_1D(X) X(1, 512) X(1, 256) X(1, 128)
 
 // Calls f.template operator()<Tile, SOLVER>() for the compiled tile matching
@@ -1097,9 +1097,11 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&mb.sms, cudaDevAttrMultiProcessorCount, dev);
-    // 2D: 132-thread rows (measured on the 1024^2 shear layer: 13.3e9 against
-    // 12.2e9 cell-updates/s for 260-thread rows)
-    int tx = L.nd == 3 ? 32 : (L.nd == 2 ? 132 : 256);
+    // 2D: rows of 64 threads, two full warps for 60 cells, where 132 threads
+    // put a fifth warp behind 128: 1024^2 58.7 us per stage against 59.5, 768^2
+    // 33.7 / 38.0, 512^2 21.7 / 24.0, 400x900 26.5 / 30.8 (96 threads: 60.0, 34.4,
+    // 22.9, 26.6)
+    int tx = L.nd == 3 ? 32 : (L.nd == 2 ? 64 : 256);
     int ty = L.nd == 3 ? 8 : 1;
     if (L.nd == 3) {
         // 16x16 tiles where they cover the grid with enough fewer columns
