@@ -104,3 +104,20 @@ def test_batch_rows_per_item(sizes, tslib):
             got, info = b.get(i)
         assert info["iteration"] == 10 + 7 * k
         assert np.array_equal(got, res[k][0]) and info["time"] == res[k][1]["time"]
+
+
+@pytest.mark.parametrize("tiny", [1e-300, 3e-39, 1.1e-38, -2e-320])
+def test_tiny_momenta_are_zeros_in_fp32(tiny, tslib):
+    """Momenta below FP32's normal range are zeros of the working copy, whatever their bits."""
+    from turbostructred_gb300 import capi
+    case = capi.make_case(ndims=2, nx=40, ny=9, periodic=(0, 0, 1), recon=3, solver=1, cfl=0.4, bc=kinds("wall"))
+    out = []
+    for m in (0.0, tiny):
+        ic = wave(40, 9, 1)
+        ic[..., 3] = m
+        with capi.Solver(case, precision=1) as s:
+            s.set_state(ic)
+            s.step(5)
+            out.append(s.get_state())
+    assert np.array_equal(out[0][..., [0, 1, 2, 4]], out[1][..., [0, 1, 2, 4]])
+    assert np.abs(out[1][..., 3]).max() <= 2 * abs(tiny)

@@ -73,7 +73,7 @@ __device__ __forceinline__ void slopes2(float w0, const float (&nm)[2], const fl
     if (KIND == FK_LIM_BJ) {
         // the smallest admissible ratio over the four face projections; with
         // both slopes 0 the ratio is dropped by fminf
-        lim = fminf(1.0f, fminf(umax - w0, w0 - umin) / fmaxf(fabsf(dd[0]), fabsf(dd[1])));
+        lim = fminf(1.0f, quot(fminf(umax - w0, w0 - umin), fmaxf(fabsf(dd[0]), fabsf(dd[1]))));
     } else if (umax - umin > 0.0f) {
         const float iun = 2.0f / (umax - umin);
 #pragma unroll

@@ -250,7 +250,7 @@ __device__ __forceinline__ void half_slopes(float w0, const float nm[3], const f
             umin = fminf(umin, fminf(nm[ax], np[ax]));
             dmax = fmaxf(dmax, fabsf(dd[ax]));
         }
-        lim = fminf(1.0f, fminf(umax - w0, w0 - umin) / dmax);
+        lim = fminf(1.0f, quot(fminf(umax - w0, w0 - umin), dmax));
     }
     if (KIND == K_LIM_VK) {
         float umax = w0, umin = w0;

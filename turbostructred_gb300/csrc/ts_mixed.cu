@@ -345,7 +345,7 @@ __device__ __forceinline__ void recon_k(const ProbDesc& d, float* sm, int p, con
                     umin = fminf(umin, fminf(nm[ax], np[ax]));
                     dmax = fmaxf(dmax, fabsf(dd[ax]));
                 }
-                const float lim = fminf(1.0f, fminf(umax - w0, w0 - umin) / dmax);
+                const float lim = fminf(1.0f, quot(fminf(umax - w0, w0 - umin), dmax));
 #pragma unroll
                 for (int ax = 0; ax < T::NAX; ++ax) dd[ax] *= lim;
             }

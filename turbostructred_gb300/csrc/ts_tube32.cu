@@ -64,7 +64,7 @@ __device__ __forceinline__ float half_slope(int kind, float nm, float w0, float 
     const float umax = fmaxf(w0, fmaxf(nm, np)), umin = fminf(w0, fminf(nm, np));
     float lim = 1.0f;
     if (kind == T_LIM_BJ) {
-        lim = fminf(1.0f, fminf(umax - w0, w0 - umin) / fabsf(dd));
+        lim = fminf(1.0f, quot(fminf(umax - w0, w0 - umin), fabsf(dd)));
     } else if (umax - umin > 0.0f) {
         const float iun = 2.0f / (umax - umin);
 #pragma unroll
