@@ -87,6 +87,7 @@ struct ts_handle {
     cudaStream_t stream = nullptr;
     std::vector<void*> allocations;
     PlainBufs pb{};
+    PlainSide side{};         // branches of a captured FP64 step
     int tube_ctas = 0;        // 1D FP64: CTAs of the resident kernel (0: stage kernels)
     MixedBufs mb{};
     Ctl* ctl_d = nullptr;
@@ -100,6 +101,11 @@ struct ts_handle {
         DeviceGuard g(device);
         for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
         for (void* p : allocations) cudaFree(p);
+        for (int k = 0; k < 2; ++k) {
+            if (side.join[k]) cudaEventDestroy(side.join[k]);
+            if (side.stream[k]) cudaStreamDestroy(side.stream[k]);
+        }
+        if (side.fork) cudaEventDestroy(side.fork);
         if (ctl_h) cudaFreeHost(ctl_h);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -207,6 +213,13 @@ struct ts_handle {
                 if ((s = alloc(&pb.VSR[a], L.plane)) != TS_OK) return s;
         pb.ctl = ctl_d;
         tube_ctas = tube64_ctas(L, ph, pb.fold);
+        if (nd > 1) {
+            for (int k = 0; k < 2; ++k) {
+                TS_CUDA(cudaStreamCreateWithFlags(&side.stream[k], cudaStreamNonBlocking));
+                TS_CUDA(cudaEventCreateWithFlags(&side.join[k], cudaEventDisableTiming));
+            }
+            TS_CUDA(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming));
+        }
         return TS_OK;
     }
 
@@ -215,7 +228,7 @@ struct ts_handle {
 
     void enqueue_step() {
         if (cfg.precision == TS_PRECISION_MIXED) mixed_step(mb, ph, stream);
-        else plain_step(pb, ph, stream);
+        else plain_step(pb, ph, stream, nullptr, nullptr, nullptr, side.fork ? &side : nullptr);
     }
 
     ts_status graph_for(int k, cudaGraphExec_t* out) {

@@ -946,7 +946,20 @@ static void launch_flux(const PlainBufs& b, const Phys& ph, cudaStream_t st) {
 }
 
 cudaError_t plain_step(const PlainBufs& b, const Phys& ph, cudaStream_t st, cudaEvent_t* ev, int* n_launch,
-                       const char** names) {
+                       const char** names, const PlainSide* side) {
+    // axes 1 and 2 on their own branches
+    const int branches = side ? ph.nd - 1 : 0;
+    auto fork = [&] {
+        if (branches) cudaEventRecord(side->fork, st);
+        for (int k = 0; k < branches; ++k) cudaStreamWaitEvent(side->stream[k], side->fork, 0);
+    };
+    auto join = [&] {
+        for (int k = 0; k < branches; ++k) {
+            cudaEventRecord(side->join[k], side->stream[k]);
+            cudaStreamWaitEvent(st, side->join[k], 0);
+        }
+    };
+    const cudaStream_t st1 = branches > 0 ? side->stream[0] : st, st2 = branches > 1 ? side->stream[1] : st;
     const Layout& L = b.L;
     const dim3 blk(kPlainBlock);
     const dim3 cells((L.nx + kPlainBlock - 1) / kPlainBlock, L.ny, L.nz);
@@ -962,10 +975,12 @@ cudaError_t plain_step(const PlainBufs& b, const Phys& ph, cudaStream_t st, cuda
         ++nl;
         if (ev) cudaEventRecord(ev[nl], st);
     };
+    fork();
     k_ghost<0><<<ghost_grid(0), blk, 0, st>>>(b, ph);
     mark("k_ghost_x");
-    if (ph.nd > 1) { k_ghost<1><<<ghost_grid(1), blk, 0, st>>>(b, ph); mark("k_ghost_y"); }
-    if (ph.nd > 2) { k_ghost<2><<<ghost_grid(2), blk, 0, st>>>(b, ph); mark("k_ghost_z"); }
+    if (ph.nd > 1) { k_ghost<1><<<ghost_grid(1), blk, 0, st1>>>(b, ph); mark("k_ghost_y"); }
+    if (ph.nd > 2) { k_ghost<2><<<ghost_grid(2), blk, 0, st2>>>(b, ph); mark("k_ghost_z"); }
+    join();
     if (ph.viscous) {
         k_vgrad<<<cells, blk, 0, st>>>(b, ph);
         mark("k_vgrad");
@@ -981,14 +996,16 @@ cudaError_t plain_step(const PlainBufs& b, const Phys& ph, cudaStream_t st, cuda
         else launch_recon<1>(b, ph, blocks, st);
         mark("k_recon");
     }
+    fork();
     if (ph.nd == 3) launch_flux<0, 3>(b, ph, st);
     else if (ph.nd == 2) launch_flux<0, 2>(b, ph, st);
     else launch_flux<0, 1>(b, ph, st);
     mark("k_flux_x");
-    if (ph.nd == 3) launch_flux<1, 3>(b, ph, st);
-    else if (ph.nd == 2) launch_flux<1, 2>(b, ph, st);
+    if (ph.nd == 3) launch_flux<1, 3>(b, ph, st1);
+    else if (ph.nd == 2) launch_flux<1, 2>(b, ph, st1);
     if (ph.nd > 1) mark("k_flux_y");
-    if (ph.nd > 2) { launch_flux<2, 3>(b, ph, st); mark("k_flux_z"); }
+    if (ph.nd > 2) { launch_flux<2, 3>(b, ph, st2); mark("k_flux_z"); }
+    join();
     const unsigned rb = reduce_blocks(L);
     if (ph.nd == 3) k_dt<3><<<rb, blk, 0, st>>>(b, ph);
     else if (ph.nd == 2) k_dt<2><<<rb, blk, 0, st>>>(b, ph);

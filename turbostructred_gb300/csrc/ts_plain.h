@@ -47,9 +47,15 @@ int plain_partial_blocks(const Layout& L);
 // Enqueues one step.  With `ev` non-null, records ev[0] before the first
 // launch and ev[i+1] after launch i (ev needs kPlainMaxLaunches+1 events);
 // *n_launch receives the launch count and names[i] the kernel names.
+// With `side`, the ghost layers and the fluxes of the axes are launched beside
+// one another (the step is then captured into a graph).
 constexpr int kPlainMaxLaunches = 14;
+struct PlainSide {
+    cudaStream_t stream[2] = {nullptr, nullptr};
+    cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
+};
 cudaError_t plain_step(const PlainBufs& b, const Phys& ph, cudaStream_t st, cudaEvent_t* ev = nullptr,
-                       int* n_launch = nullptr, const char** names = nullptr);
+                       int* n_launch = nullptr, const char** names = nullptr, const PlainSide* side = nullptr);
 
 // 1D problems: many steps per launch by one thread-block cluster that keeps
 // the state on chip (ts_tube64.cu).  The CTAs of the cluster, or 0 when the
