@@ -92,7 +92,7 @@ __device__ __forceinline__ bool dabs_lt(double a, double b) {
 // ---------------------------------------------------------------------------
 // Fast: divisions, square roots and halvings on the integer pipe
 // (ts_exact64.cuh), correctly rounded like the hardware's, for operands in the
-// ranges stated there; anything else sets `bad` and the result is discarded.
+// ranges stated there (results that are subnormal, mostly); anything else sets `bad` and the result is discarded.
 // Plain: the hardware operations, for the faces and cells where Fast gave up
 // (zero, subnormal, infinite or NaN divisors and the like).  Both perform the
 // same additions and multiplications in the same order.
@@ -515,8 +515,13 @@ __device__ __forceinline__ void recon_value(double val, const double nm[ND], con
                     const u64 ad = (u64)__double_as_longlong(dabs(d2));
                     const u64 aa = __double2hiint(d2) < 0 ? aq : ap;
                     if (aa < ad) {
-                        o.bad |= !est32_ok(ad);
-                        const float r = est32_ok(aa) ? __fdividef(est32(aa), est32(ad)) : 0.0f;
+                        // estimates with the exponent of d2 taken out of both (a
+                        // subnormal a or d2 gives up)
+                        const bool an = (aa >> 52) != 0;
+                        o.bad |= (unsigned)(ad >> 52) - 1u >= 2046u || (!an && aa != 0);
+                        const u64 sc = ((ad >> 52) - 1023u) << 52, as = aa - sc;
+                        const float r = an && (long long)aa > (long long)sc && est32_ok(as)
+                                            ? __fdividef(est32(as), est32(ad - sc)) : 0.0f;
                         bool take = r < br * (1.0f - 3.8e-6f);
                         // (a zero or the same ratio cannot be undercut: local extrema,
                         // and states that differ by a few ulps)

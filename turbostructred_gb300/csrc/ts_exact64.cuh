@@ -125,10 +125,6 @@ TS_X64 u32 seed_rsqrt(u32 fbits) {
 #endif
 }
 
-// Exponent fields 513 .. 1533 (2^-510 .. 2^511): any quotient of two such
-// numbers is normal.
-TS_X64 bool mid_range(u32 e) { return e - 513u < 1021u; }
-
 // A divisor prepared once for any number of quotients: its 53-bit
 // significand B and Y = 2^114 / B to a few units.
 struct Divisor {
@@ -137,11 +133,11 @@ struct Divisor {
     u32 sign;
 };
 
-// b: exponent field in [513, 1533], else `bad`.
+// b: normal, else `bad`.
 TS_X64 Divisor divisor(double b, bool& bad) {
     const u32 hi = hi_of(b);
     const u32 e = (hi >> 20) & 0x7FFu;
-    bad |= !mid_range(e);
+    bad |= e - 1u >= 2046u;
     Divisor d;
     d.e = (int)e;
     d.sign = hi & 0x80000000u;
@@ -158,7 +154,8 @@ TS_X64 Divisor divisor(double b, bool& bad) {
     return d;
 }
 
-// RN(a / b).  a: zero, or exponent field in [513, 1533]; else `bad`.
+// RN(a / b).  a: zero or normal, with a quotient that is normal or rounds to
+// zero; else `bad`.
 TS_X64 double quotient(double a, const Divisor& d, bool& bad) {
     const u32 ahi = hi_of(a), alo = lo_of(a);
     const u32 sign = (ahi ^ d.sign) & 0x80000000u;
@@ -175,9 +172,11 @@ TS_X64 double quotient(double a, const Divisor& d, bool& bad) {
     const u64 R2 = ((A << 52) - n * d.B) << 1;
     n += (d.B - R2) >> 63;  // 2R > B: the next one is nearer
     n -= (d.B + R2) >> 63;  // 2R < -B: the previous one
-    const bool zero = is_zero(ahi, alo);
-    bad |= !(mid_range(e) || zero);
-    const u32 qhi = (u32)(n >> 32) + (((u32)((int)e - d.e + 1022 - (int)lt)) << 20);
+    const bool none = is_zero(ahi, alo);
+    const int E = (int)e - d.e + 1023 - (int)lt;  // (one more where n = 2^53: E = 0 counts as subnormal)
+    const bool zero = none || E < -52;  // less than half the smallest subnormal
+    bad |= !((e - 1u < 2046u || none) && ((u32)(E - 1) < 2046u || zero));
+    const u32 qhi = (u32)(n >> 32) + ((u32)(E - 1) << 20);
     return of_words((zero ? 0u : qhi) | sign, zero ? 0u : (u32)n);
 }
 
@@ -211,16 +210,15 @@ TS_X64 double root(double a, bool& bad) {
     return of_words((u32)(n >> 32) + ((u32)(k + 1022) << 20), (u32)n);
 }
 
-// RN(a b).  a and b: zero, or exponent fields in [513, 1533]; else `rare`
-// (nothing is wrong then: the caller lets the hardware multiply).  The exact
+// RN(a b).  a and b: zero or normal, with a product that is normal or rounds to
+// zero; else `rare` (nothing is wrong then: the caller lets the hardware multiply).  The exact
 // 106-bit product in four 32x32->64 multiply-adds, one bit of normalisation,
 // and the rounding carry added through the exponent: about 30 plain integer
 // operations, 12 to 14 clocks per warp and SM beside the FP64 pipe's 19.
 TS_X64 double mul(double a, double b, bool& rare) {
     const u32 ahi = hi_of(a), al = lo_of(a), bhi = hi_of(b), blo = lo_of(b);
-    const u32 ea = ahi & 0x7FF00000u, eb = bhi & 0x7FF00000u;
+    const u32 ea = ahi & 0x7FF00000u, eb = bhi & 0x7FF00000u;  // exponents in place
     const bool za = is_zero(ahi, al), zb = is_zero(bhi, blo);
-    rare = !((ea - (513u << 20) < (1021u << 20) || za) && (eb - (513u << 20) < (1021u << 20) || zb));
     const u32 ah = (ahi & 0xFFFFFu) | 0x100000u;
     const u64 B = join((bhi & 0xFFFFFu) | 0x100000u, blo) << 10;  // 63 bits
     const u32 bh = (u32)(B >> 32), bl = (u32)B;
@@ -237,7 +235,11 @@ TS_X64 double mul(double a, double b, bool& rare) {
     const u32 r = (pl << s) | ((u32)p0 != 0u ? 1u : 0u);
     // carry out of r + 0x7FFFFFFF + (nl & 1): above one half, or a tie and nl odd
     const u32 half_up = 0x7FFFFFFFu + (nl & 1u);
-    const u32 e = ea + eb + (top << 20) - (1024u << 20);  // with the leading bit of nh
+    const u32 es = ea + eb + (top << 20);  // the biased exponent + 1023: no carry out
+    const u32 e = es - (1024u << 20);      // with the leading bit of nh
+    const bool zero = za || zb || es < (971u << 20);  // less than half the smallest subnormal
+    rare = !((ea - (1u << 20) < (2046u << 20) || za) && (eb - (1u << 20) < (2046u << 20) || zb) &&
+             (e < (2046u << 20) || zero));
 #ifdef __CUDA_ARCH__
     u32 drop;
     asm("add.cc.u32 %0, %3, %4;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, %2, %5;"
@@ -249,7 +251,6 @@ TS_X64 double mul(double a, double b, bool& rare) {
     nh = (u32)(n >> 32) + e;
     nl = (u32)n;
 #endif
-    const bool zero = za || zb;
     return of_words((zero ? 0u : nh) | ((ahi ^ bhi) & 0x80000000u), zero ? 0u : nl);
 }
 
