@@ -167,3 +167,33 @@ def test_waves_that_reach_far_into_still_gas(ndims, solver, recon, tslib, oracle
     mom = np.abs(ref[..., 1:4])
     assert mom[mom > 0].min() < 1e-100  # the inputs do what they are for
     assert np.array_equal(got, ref) and info["time"] == rinfo["time"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["diagonal", "linear", "ulps", "offset", "random", "almost_diagonal"])
+@pytest.mark.parametrize("ndims", [2, 3])
+def test_limiter_ties(kind, ndims, tslib, oracle_mod):
+    """Slopes and limits that are equal, a few ulps apart or lost in the value's rounding: the limiter's smallest ratio is
+    the reference's whichever way it is found."""
+    from oracle import oracle as O
+    from turbostructred_gb300 import capi
+    n = (37, 37, 1) if ndims == 2 else (13, 13, 13)
+    r = np.random.default_rng(11)
+    x, y, z = [(np.arange(k) + 0.5) / k for k in n]
+    Z, Y, X = np.meshgrid(z, y, x, indexing="ij")
+    d = X + Y + (Z if ndims == 3 else 0.0)
+    f = {"diagonal": 0.3 * np.sin(7 * d), "linear": 0.25 * d, "ulps": r.integers(-2, 3, X.shape) * 2.0 ** -52,
+         "offset": 1e-9 * np.sin(9 * X) * np.cos(5 * Y), "random": 0.2 * r.uniform(-1, 1, X.shape),
+         "almost_diagonal": 0.3 * np.sin(7 * d) * (1 + 1e-6 * r.uniform(-1, 1, X.shape))}[kind]
+    rho, p = 1.0 + f, 1.0 + 0.5 * f
+    v = np.stack([0.1 + f, 0.1 + f, (0.1 + f) * (ndims == 3)], -1)
+    ic = np.concatenate([rho[..., None], rho[..., None] * v, (p / 0.4 + 0.5 * rho * (v * v).sum(-1))[..., None]], -1)
+    case = O.make_case(ndims=ndims, nx=n[0], ny=n[1], nz=n[2], periodic=(1, 1, 1), recon=3, solver=3, cfl=0.3)
+    full = oracle_mod.embed(case, ic)
+    ref, rinfo = oracle_mod.advance(case, full, 7)
+    with capi.Solver(capi.make_case(**case)) as s:
+        s.set_state(full, capi.LAYOUT_WITH_GHOSTS)
+        info = s.step(7)
+        got = s.get_state(capi.LAYOUT_WITH_GHOSTS)
+    assert np.isfinite(ref).all()
+    assert np.array_equal(got, ref) and info["time"] == rinfo["time"]

@@ -501,37 +501,70 @@ __device__ __forceinline__ void recon_value(double val, const double nm[ND], con
             } else {
                 // The limiter is the smallest of the rounded ratios a / d2
                 // (a = umax - val or umin - val) below 1.  Rounding is
-                // monotone, so only the smallest ratio is divided out: it is
-                // found on FP32 estimates (error < 2^-20), and estimates
-                // closer than 2^-18 are settled by their quotients.  A ratio
-                // with |a| >= |d2| rounds to 1 or more and is dropped.
+                // monotone, so only the smallest ratio is divided out.  d2 is the
+                // projection gs up to rounding: where no projection is
+                // lost in the value's rounding (val < 2^25 max|gs|) and the FP32
+                // estimates tell the smaller a from the larger and the largest
+                // |gs| from the next (2^-17 apart; estimates are good to 2^-20),
+                // the smallest ratio is that of these two, and only its d2 is formed (2
+                // FP64 additions of 8 in 2D and 12 in 3D: shear layer 1024^2 10.50 -> 9.84
+                // ms per pass).
                 const u64 ap = (u64)__double_as_longlong(am), aq = (u64)__double_as_longlong(dabs(an));
-                u64 ba = 0, bd = 0;
-                float br = 2.0f;
+                const u64 a1 = ap < aq ? ap : aq, a2 = ap < aq ? aq : ap;
+                u64 s1 = (u64)__double_as_longlong(dabs(gs[0])), s2 = 0;
 #pragma unroll
-                for (int f = 0; f < 2 * ND; ++f) {
-                    const double s = (f & 1) ? gs[f >> 1] : -gs[f >> 1];
-                    const double d2 = (val + s) - val;
-                    const u64 ad = (u64)__double_as_longlong(dabs(d2));
-                    const u64 aa = __double2hiint(d2) < 0 ? aq : ap;
-                    if (aa < ad) {
-                        // estimates with the exponent of d2 taken out of both (a
-                        // subnormal a or d2 gives up)
-                        const bool an = (aa >> 52) != 0;
-                        o.bad |= (unsigned)(ad >> 52) - 1u >= 2046u || (!an && aa != 0);
-                        const u64 sc = ((ad >> 52) - 1023u) << 52, as = aa - sc;
-                        const float r = an && (long long)aa > (long long)sc && est32_ok(as)
-                                            ? __fdividef(est32(as), est32(ad - sc)) : 0.0f;
-                        bool take = r < br * (1.0f - 3.8e-6f);
-                        // (a zero or the same ratio cannot be undercut: local extrema,
-                        // and states that differ by a few ulps)
-                        if (!take && r <= br * (1.0f + 3.8e-6f) && ba != 0 && !(aa == ba && ad == bd))
-                            take = ratio_less(__longlong_as_double(aa), __longlong_as_double(ad),
-                                              __longlong_as_double(ba), __longlong_as_double(bd));
-                        if (take) { ba = aa; bd = ad; br = r; }
-                    }
+                for (int a = 1; a < ND; ++a) {
+                    const u64 t = (u64)__double_as_longlong(dabs(gs[a]));
+                    if (t > s1) { s2 = s1; s1 = t; }
+                    else if (t > s2) s2 = t;
                 }
-                if (br < 2.0f) lmin = o.div(__longlong_as_double(ba), __longlong_as_double(bd));
+                const int es = (int)(s1 >> 52);
+                const bool clear = (unsigned)(es - 1) < 2046u && (int)(((unsigned)__double2hiint(val) >> 20) & 0x7FFu) - es <= 24;
+                const u64 sc = ((u64)es - 1023u) << 52;  // the exponent of s1, taken out of all
+                const float f1 = est32(s1 - sc);
+                const float f2 = (long long)s2 > (long long)sc && est32_ok(s2 - sc) ? est32(s2 - sc) : 0.0f;
+                const bool in = (a1 >> 52) != 0 && (long long)a1 > (long long)sc && est32_ok(a1 - sc) && est32_ok(a2 - sc);
+                const float e1 = est32(a1 - sc), e2 = est32(a2 - sc);
+                constexpr float kNear = 1.0f - 7.7e-6f;
+                if (clear && a1 == 0) {
+                    lmin = 0.0;  // a local extremum
+                } else if (clear && in && e1 > f1 * (2.0f - kNear)) {
+                    // every ratio is above 1
+                } else if (clear && in && e1 < f1 * kNear && f2 < f1 * kNear && e1 < e2 * kNear) {
+                    const double g1 = __longlong_as_double((long long)s1);
+                    const double d2 = ap < aq ? (val + g1) - val : val - (val - g1);
+                    lmin = o.div(__longlong_as_double((long long)a1), d2);
+                } else {
+                    // too close to tell: the same on every face's own d2, and
+                    // estimates closer than 2^-18 settled by their quotients.  A ratio
+                    // with |a| >= |d2| rounds to 1 or more and is dropped.
+                    u64 ba = 0, bd = 0;
+                    float br = 2.0f;
+#pragma unroll
+                    for (int f = 0; f < 2 * ND; ++f) {
+                        const double s = (f & 1) ? gs[f >> 1] : -gs[f >> 1];
+                        const double d2 = (val + s) - val;
+                        const u64 ad = (u64)__double_as_longlong(dabs(d2));
+                        const u64 aa = __double2hiint(d2) < 0 ? aq : ap;
+                        if (aa < ad) {
+                            // estimates with the exponent of d2 taken out of both (a
+                            // subnormal a or d2 gives up)
+                            const bool an = (aa >> 52) != 0;
+                            o.bad |= (unsigned)(ad >> 52) - 1u >= 2046u || (!an && aa != 0);
+                            const u64 sc = ((ad >> 52) - 1023u) << 52, as = aa - sc;
+                            const float r = an && (long long)aa > (long long)sc && est32_ok(as)
+                                                ? __fdividef(est32(as), est32(ad - sc)) : 0.0f;
+                            bool take = r < br * (1.0f - 3.8e-6f);
+                            // (a zero or the same ratio cannot be undercut: local extrema,
+                            // and states that differ by a few ulps)
+                            if (!take && r <= br * (1.0f + 3.8e-6f) && ba != 0 && !(aa == ba && ad == bd))
+                                take = ratio_less(__longlong_as_double(aa), __longlong_as_double(ad),
+                                                  __longlong_as_double(ba), __longlong_as_double(bd));
+                            if (take) { ba = aa; bd = ad; br = r; }
+                        }
+                    }
+                    if (br < 2.0f) lmin = o.div(__longlong_as_double(ba), __longlong_as_double(bd));
+                }
             }
         }
     }
