@@ -292,11 +292,7 @@ __global__ void __launch_bounds__(FNT, 3) k_flat2d(const __grid_constant__ ProbD
         }
         if (m > 0.0f) atomicMax(&ctl->srmax_bits, __float_as_uint(m));
         if (hh) atomicOr(&ctl->health, hh);
-        __threadfence();
-        if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
-            __threadfence();
-            finish_problem(ctl, mp.cfl);
-        }
+        if (count_in(&ctl->blocks_done) == gridDim.x - 1) finish_problem(ctl, mp.cfl);
     }
 }
 

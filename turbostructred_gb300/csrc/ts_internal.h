@@ -100,6 +100,18 @@ inline bool has_markers(const ts_config& c) {
     return false;
 }
 
+#ifdef __CUDACC__
+// Counts a block in: every write that happened before in its thread, and
+// through a barrier in its block, is visible to the block that is told the
+// last count.  (One release and acquire at the counter; a __threadfence on each
+// side of a plain atomic is a sequentially consistent fence each.)
+__device__ __forceinline__ unsigned int count_in(unsigned int* counter) {
+    unsigned int before;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+    return before;
+}
+#endif
+
 // Physics and method selection passed by value to kernels.
 struct Phys {
     int nd;

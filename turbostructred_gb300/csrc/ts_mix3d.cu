@@ -814,11 +814,7 @@ __device__ __forceinline__ void close3(const ProbDesc& d, int n_closes, float sr
         Ctl* ctl = d.ctl;
         if (m > 0.0f) atomicMax(&ctl->srmax_bits, __float_as_uint(m));
         if (hh) atomicOr(&ctl->health, hh);
-        __threadfence();
-        if (atomicAdd(&ctl->blocks_done, 1u) == (unsigned)(n_closes - 1)) {
-            __threadfence();
-            finish_problem(ctl, d.mp.cfl);
-        }
+        if (count_in(&ctl->blocks_done) == (unsigned)(n_closes - 1)) finish_problem(ctl, d.mp.cfl);
     }
 }
 

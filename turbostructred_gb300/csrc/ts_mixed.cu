@@ -659,11 +659,7 @@ __device__ __forceinline__ void close_item(const ProbDesc& d, float srmax, unsig
         if (m > 0.0f) atomicMax(&ctl->srmax_bits, __float_as_uint(m));
         if (hh) atomicOr(&ctl->health, hh);
         if (COUNT) {
-            __threadfence();
-            if (atomicAdd(&ctl->blocks_done, 1u) == (unsigned)(d.nq - 1)) {
-                __threadfence();
-                finish_problem(ctl, d.mp.cfl);
-            }
+            if (count_in(&ctl->blocks_done) == (unsigned)(d.nq - 1)) finish_problem(ctl, d.mp.cfl);
         }
     }
 }

@@ -730,12 +730,10 @@ __global__ void __launch_bounds__(kPlainBlock) k_dt(const __grid_constant__ Plai
         u64 m = wmin[0];
         for (int w = 1; w < kPlainBlock / 32; ++w) m = umin64(m, wmin[w]);
         b.partial[blockIdx.x] = __longlong_as_double((long long)m);
-        __threadfence();
-        last = (atomicAdd(&b.ctl->blocks_done, 1u) == (unsigned)(nblk - 1));
+        last = count_in(&b.ctl->blocks_done) == (unsigned)(nblk - 1);
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     u64 m = kInfBits;
     for (int t = threadIdx.x; t < nblk; t += kPlainBlock)
         m = umin64(m, (u64)__double_as_longlong(((volatile double*)b.partial)[t]));
@@ -883,17 +881,12 @@ __global__ void __launch_bounds__(kPlainBlock) k_update(const __grid_constant__ 
         for (int w = 0; w < kPlainBlock / 32; ++w) s += red[threadIdx.x][w];
         double* to = slots ? &b.norms[threadIdx.x * kNormSlots + blockIdx.x % kNormSlots] : &b.ctl->res[threadIdx.x];
         if (!dzero(s)) atomicAdd(to, s);
-        __threadfence();
     }
     __syncthreads();
     Ctl* ctl = b.ctl;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1;
-    }
+    if (threadIdx.x == 0) last = count_in(&ctl->blocks_done) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
-    __threadfence();
     // the slots of each norm, summed pairwise and cleared for the next step
     for (int v = wid; slots && v < NV; v += kPlainBlock / 32) {
         double s = __ldcg(&b.norms[v * kNormSlots + lane]);
