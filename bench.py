@@ -579,7 +579,7 @@ def run_tubes(args, rank, ws, lr, dist, emit=True):
                              "kernel": "k_mix_step (batched, one-row 1D tiles) and k_tube32",
                              "kernel_ms": None, "algorithmic_bytes": BYTES_PER_CELL_UPDATE * cu,
                              "basis": "80 B x the batch's cell-updates over the whole solve's wall time (stage "
-                                      "kernels, finish kernels, the cluster tail kernel and launch gaps): a lower "
+                                      "kernels, finish kernels, the resident cluster kernel and launch gaps): a lower "
                                       "bound of the kernels' own rate",
                              "peak_source": peak_kind},
                 "clocks": clocks, "gpu_launches": st["launches"],

@@ -247,11 +247,13 @@ ts_status ts_set_step_info(ts_handle* h, const ts_step_info* info);
 
 /* Launch shape of the mixed-precision fused kernel: the tile (threads per
    CTA along x and y; compiled shapes: 3D 32x8, 16x16, 32x16, each thread one
-   cell, marching z; 2D 260, 132, 68 one-row tiles marching y; 1D 512, 256,
-   128; one-row tiles own tx - 4 cells) and the number of chunks each tile
+   cell, marching z; 2D 260, 132, 96, 68, 64 one-row tiles marching y; 1D 512,
+   256, 128; one-row tiles own tx - 4 cells) and the number of chunks each tile
    column's march is cut into (0 = chosen from the grid and the SM count).
    Every face flux is a function of its two cells only; other tiles are
-   other compiled instances and agree to FP32 rounding.
+   other compiled instances and agree to FP32 rounding.  A handle whose tile
+   was never set picks it itself, small 2D problems (kernels that march
+   nothing) and 1D ones (resident on chip, many stages per launch) included.
    TS_ERR_UNSUPPORTED for the FP64 path or an uncompiled tile. */
 ts_status ts_set_tile(ts_handle* h, int32_t tx, int32_t ty, int32_t z_chunks);
 
@@ -366,15 +368,15 @@ ts_status ts_batch_get(ts_batch* b, int32_t id, double* values, ts_step_info* in
 ts_status ts_batch_remove(ts_batch* b, int32_t id);
 
 /* Launch shape for the problems of dimension nd: tx = threads of the
-   one-row tile along x (1D: 512, 256, 128; 2D: 260, 132, 68; the tile owns
-   tx - 4 cells), or 0 to pick per problem from its x extent; ty is ignored;
+   one-row tile along x (1D: 512, 256, 128; 2D: 260, 132, 96, 68, 64; the tile
+   owns tx - 4 cells), or 0 to pick per problem from its x extent; ty is ignored;
    and CTAs per SM of the persistent grid (0 = as many as fit). */
 ts_status ts_batch_set_tile(ts_batch* b, int32_t nd, int32_t tx, int32_t ty, int32_t ctas_per_sm);
 
-/* The batch's tail mode (on by default): once every unfinished problem is
-   1D, fits one thread-block cluster (at most 16 x 508 cells) and all of them
-   together fit the GPU at once, each launch advances every problem by up to
-   the requested number of stages in the cluster tail kernel, with the state
+/* The batch's tail mode (on by default): while every unfinished problem is
+   1D, of 4 to 8672 cells (one thread-block cluster), and all of them together
+   have at most 300000 cells, each launch advances every problem by up to the
+   requested number of stages in the resident cluster kernel, with the state
    kept on chip between stages; results are identical to the stage-by-stage
    path.  enable = 0 keeps the stage-by-stage path throughout. */
 ts_status ts_batch_set_tail(ts_batch* b, int32_t enable);
