@@ -117,6 +117,45 @@ __device__ __forceinline__ float flat_face(const MixPhys& mp, const FlatMem& s, 
     return flux32<SOLVER, A>(mp, UL, UR, F);
 }
 
+// finish_problem with every field read at once, beside the maximum: the block
+// that closes a step is alone, and each dependent trip to L2 is 0.3 us (200
+// stages of 128^2 1409 -> 1361 us).  (In k_mix_step it changes how the
+// compiler contracts the 1D Roe flux, and with it the results' last bits.)
+__device__ __forceinline__ void finish_at_once(Ctl* ctl, double cfl) {
+    const float m = __uint_as_float(*(volatile unsigned int*)&ctl->srmax_bits);
+    const double t0 = ctl->time, save_sol = ctl->save_sol, save_slice = ctl->save_slice, max_time = ctl->max_time;
+    const double sol = ctl->next_sol, slice = ctl->next_slice;
+    const int it = ctl->iteration + 1, par = ctl->parity ^ 1, run = ctl->run_mode, max_it = ctl->max_iteration;
+    double res[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) res[v] = ctl->res_acc[v];
+    // positive numbers have positive bit patterns (no comparison on the FP64 pipe)
+    const bool sols = __double_as_longlong(save_sol) > 0, slices = __double_as_longlong(save_slice) > 0;
+    double dt, raw;
+    step_size(cfl, m, dt, raw);
+    if (sols && (sol < t0 + dt)) dt = sol - t0;
+    if (slices && (slice < t0 + dt)) dt = slice - t0;
+    const double t1 = t0 + dt;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        ctl->res[v] = res[v];
+        ctl->res_acc[v] = 0.0;
+    }
+    ctl->dt_min_raw = raw;
+    ctl->dt = dt;
+    ctl->dt_apply = dt;
+    ctl->time = t1;
+    ctl->iteration = it;
+    ctl->parity = par;
+    ctl->srmax_bits = 0u;
+    ctl->blocks_done = 0u;
+    if (run) {
+        if (sols && (sol == t1)) ctl->next_sol = sol + save_sol;
+        if (slices && (slice == t1)) ctl->next_slice = slice + save_slice;
+        if (it == max_it || t1 >= max_time) ctl->stop_req = 1;
+    }
+}
+
 template <int SOLVER, int KIND>
 __global__ void __launch_bounds__(FNT, 3) k_flat2d(const __grid_constant__ ProbDesc d) {
     __shared__ FlatMem s;
@@ -292,7 +331,7 @@ __global__ void __launch_bounds__(FNT, 3) k_flat2d(const __grid_constant__ ProbD
         }
         if (m > 0.0f) atomicMax(&ctl->srmax_bits, __float_as_uint(m));
         if (hh) atomicOr(&ctl->health, hh);
-        if (count_in(&ctl->blocks_done) == gridDim.x - 1) finish_problem(ctl, mp.cfl);
+        if (count_in(&ctl->blocks_done) == gridDim.x - 1) finish_at_once(ctl, mp.cfl);
     }
 }
 
