@@ -463,8 +463,7 @@ struct ts_batch {
         for (int s = 0; s < capacity; ++s) {
             if (!slots[s].used || h_ctl[s].stop_req) continue;
             const ProbDesc& d = desc[s];
-            // the resident kernel forms no residual norms
-            if (d.L.nd != 1 || d.kn[0] < 4 || d.kn[0] > tube32_max_cells() || d.mp.norms) return TS_OK;
+            if (!tube32_serves(d)) return TS_OK;
             cells += d.kn[0];
             act.push_back(s);
         }
