@@ -163,9 +163,9 @@ struct Tune {
     int tx, ty, ctas;
 };
 
-// One-row tiles compiled for batched problems (threads along x).
+// One-row tiles that the autotuner offers (threads along x).
 const int kTiles1D[3] = {512, 256, 128};
-const int kTiles2D[5] = {260, 132, 96, 68, 64};
+const int kTiles2D[3] = {260, 132, 68};
 // Marching-axis rows per work item of a 2D problem: 64 when the listed
 // problems fill the CTA slots with such items, else the fewest with which
 // all items still run at once (a stage of a small set ends with its longest
@@ -463,7 +463,7 @@ struct ts_batch {
         for (int s = 0; s < capacity; ++s) {
             if (!slots[s].used || h_ctl[s].stop_req) continue;
             const ProbDesc& d = desc[s];
-            if (!tube32_serves(d)) return TS_OK;
+            if (!tube32_serves(d, false)) return TS_OK;
             cells += d.kn[0];
             act.push_back(s);
         }
@@ -1042,8 +1042,7 @@ ts_status ts_batch_autotune(ts_batch* b, int32_t stages, int32_t* tx_out, int32_
     // each with as many resident CTAs as fit, and capped at 2 and 1
     std::vector<Tune> cand;
     const int* tiles = nd == 1 ? kTiles1D : kTiles2D;
-    const int n_tiles = nd == 1 ? 3 : 5;
-    for (int k = -1; k < n_tiles; ++k) {
+    for (int k = -1; k < 3; ++k) {
         const int tx = k < 0 ? 0 : tiles[k];
         size_t bytes;
         int per = 0;

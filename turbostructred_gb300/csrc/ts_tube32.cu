@@ -379,11 +379,12 @@ cudaError_t config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg
 
 int tube32_max_cells() { return kTailMaxCluster * kMaxOwn; }
 
-bool tube32_serves(const ProbDesc& d) {
-    // (the compiler contracts the Venkatakrishnan limiter of the HLLC instance
-    // otherwise than in the stage kernel, seen at 40 cells: those keep the stage kernel)
-    const bool other = d.mp.solver == TS_RS_HLLC && d.mp.recon == TS_RECON_LINEAR_2POINTS_LIMITED &&
-                       d.mp.limiter == TS_LIM_VENKATAKRISHNAN;
+bool tube32_serves(const ProbDesc& d, bool one) {
+    // (the compiler contracts the Venkatakrishnan limiter otherwise than in the
+    // stage kernels, but for batched Roe problems; seen at 40 cells: the others
+    // keep the stage kernels)
+    const bool vk = d.mp.recon == TS_RECON_LINEAR_2POINTS_LIMITED && d.mp.limiter == TS_LIM_VENKATAKRISHNAN;
+    const bool other = vk && (one || d.mp.solver == TS_RS_HLLC);
     // no residual norms are formed
     return d.L.nd == 1 && d.kn[0] >= 4 && d.kn[0] <= tube32_max_cells() && !d.mp.norms && !other;
 }
