@@ -258,7 +258,7 @@ struct ts_batch {
     // page-locked staging: new problems are copied to up_h in turn and put in
     // place from there by a kernel on the upload stream (which has drained
     // before the buffer starts over); results are read into down_h
-    static constexpr size_t kStage = size_t(8) << 20;
+    static constexpr size_t kStage = size_t(8) << 20, kSmallStage = size_t(256) << 10;
     char *up_h = nullptr, *down_h = nullptr;
     size_t up_size = 0, up_used = 0;
     std::vector<int> quarantine;  // removed slots, reusable once the main stream has drained
@@ -688,9 +688,6 @@ ts_status ts_batch_create(int32_t device, size_t budget, ts_batch** out) {
     TB_CUDA(cudaStreamCreateWithFlags(&b->dstream, cudaStreamNonBlocking));
     TB_CUDA(cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming));
     TB_CUDA(b->arena.init(budget));
-    TB_CUDA(cudaHostAlloc((void**)&b->up_h, ts_batch::kStage, cudaHostAllocDefault));
-    b->up_size = ts_batch::kStage;
-    TB_CUDA(cudaHostAlloc((void**)&b->down_h, ts_batch::kStage, cudaHostAllocDefault));
     ts_status s = b->grow(64);
     if (s != TS_OK) return s;
     *out = b.release();
@@ -751,12 +748,15 @@ ts_status ts_batch_add(ts_batch* b, const ts_config* cfg, const double* values, 
     if (b->up_used + block > b->up_size) {
         TB_CUDA(cudaStreamSynchronize(us));
         b->up_used = 0;
-        if (block > b->up_size) {  // the geometry of a very long grid
+        // made when first needed: for states too, or for a server's geometry,
+        // control words and descriptors alone
+        const size_t want = std::max(block, staged ? ts_batch::kStage : ts_batch::kSmallStage);
+        if (want > b->up_size) {
             cudaFreeHost(b->up_h);
             b->up_h = nullptr;
             b->up_size = 0;
-            TB_CUDA(cudaHostAlloc((void**)&b->up_h, block, cudaHostAllocDefault));
-            b->up_size = block;
+            TB_CUDA(cudaHostAlloc((void**)&b->up_h, want, cudaHostAllocDefault));
+            b->up_size = want;
         }
     }
     Placing pl{};
@@ -915,6 +915,7 @@ ts_status ts_batch_get(ts_batch* b, int32_t id, double* values, ts_step_info* in
     // page-locked host memory is written in place, a small result through the
     // page-locked staging buffer
     const bool staged = values && !pinned && nvals * sizeof(double) <= ts_batch::kStage;
+    if (staged && !b->down_h) TB_CUDA(cudaHostAlloc((void**)&b->down_h, ts_batch::kStage, cudaHostAllocDefault));
     double* dst = pinned ? pinned : reinterpret_cast<double*>(b->down_h);
     if (values && !pinned && !staged) {
         if (b->dstage_doubles < nvals) {

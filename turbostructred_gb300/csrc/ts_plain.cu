@@ -21,18 +21,19 @@
 //                iteration and the Kernel::Run termination rules
 //
 // What bounds it: the FP64 pipe.  GB300 takes 19 clocks per SM for an FP64
-// warp instruction of any kind, comparisons, min/max and |x| included, while
-// the issue slots are 85 % idle.  So everything but the additions and
-// multiplications themselves runs on the integer pipe: divisions and square
-// roots (ts_exact64.cuh), comparisons, sign changes and halvings; terms that
-// are exact zeros are skipped where a whole warp agrees (transverse momentum
-// of 1D and 2D flows, constant neighbourhoods, equal fluxes); the slope
+// warp instruction of any kind, comparisons, min/max and |x| included.  So what
+// need not be there runs on the integer pipe: divisions, square roots and about
+// half of the products (ts_exact64.cuh), comparisons, sign changes and halvings;
+// terms that are exact zeros are skipped where a whole warp agrees (transverse
+// momentum of 1D and 2D flows, constant neighbourhoods, equal fluxes); the slope
 // projections lim * (slope * h/2) are formed once per cell instead of at each
-// of its faces; and the residual norms are summed per thread over many
-// cells before the block's reduction.  The results are bit for bit the same.
+// of its faces, and the limiter forms the one difference that decides it; the
+// residual norms are summed per thread over many cells before the block's
+// reduction.  The results are bit for bit the same.  The ghost layers and the
+// fluxes of the axes are branches of the captured step.
 // Measured on one GB300, time per step before and after: 3D blast 192^3 (Roe,
-// Barth-Jespersen) 28.4 -> 9.98 ms (k_recon 8.1 -> 0.69, each k_flux 5.9 ->
-// 2.7, k_update 3.0 -> 0.72); 2D shear layer 1024^2 (HLLC) 3.27 -> 0.70 ms.
+// Barth-Jespersen) 28.4 -> 8.6 ms; 2D shear layer 1024^2 (HLLC) 3.27 -> 0.61 ms;
+// 2D box 203x157 167 -> 63 us.  1D problems: ts_tube64.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
