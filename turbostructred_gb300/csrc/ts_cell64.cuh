@@ -619,9 +619,10 @@ __device__ __forceinline__ double face_flux(const Phys& ph, const double UL[NV],
 // either sign has a larger pattern than +inf), so they order like their bits.
 __device__ __forceinline__ u64 umin64(u64 a, u64 b) { return a < b ? a : b; }
 __device__ __forceinline__ u64 warp_min(u64 v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = umin64(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    // the least high word, then the least low word among its holders
+    const unsigned hi = (unsigned)(v >> 32), least = __reduce_min_sync(0xffffffffu, hi);
+    const unsigned lo = __reduce_min_sync(0xffffffffu, hi == least ? (unsigned)v : 0xffffffffu);
+    return (u64)least << 32 | lo;
 }
 
 // Bits of V / sr.
