@@ -24,7 +24,7 @@
 // its ends; the first of them also solves the face at its high end.
 //
 // Measured on one GB300, whole passes, stage kernels -> here: shock tube of
-// 1000 cells to its end time (Roe, first order, 1736 steps) 40.0 -> 16.7 ms;
+// 1000 cells to its end time (Roe, first order, 1736 steps) 40.0 -> 15.7 ms;
 // 397 cells, HLLC, Barth-Jespersen, 64 steps 1650 -> 757 us.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -111,9 +111,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube64(const __grid_constant
     const double Vend = b.ch[0][n + g0] * hy * hz;  // of the ghost cell beyond the high side
     const typename Safe::Div iv = o.divisor(V);
     const bool last_cell = own && i0 + tid == n - 1;
-    // ghost layers: cells 0, 1 and n-1, n-2
-    const int lo_layer = own && i0 + tid < GHOST ? i0 + tid : -1;
-    const int hi_layer = own && n - 1 - (i0 + tid) < GHOST ? n - 1 - (i0 + tid) : -1;
+    // ghost layers: of cells 0, 1 and n-1, n-2 (four cells at least).  Written when
+    // the launch ends: a store to global memory in a step has to complete before
+    // the barrier that follows it.
+    const bool at_hi = own && n - 1 - (i0 + tid) < GHOST;
+    const int layer = at_hi ? n - 1 - (i0 + tid) : (own && i0 + tid < GHOST ? i0 + tid : -1);
+    double ghost[NV] = {1.0, 0.0, 0.0, 0.0, 1.0};
     const int idl = bc_id(ph.bc.mark, 0, 0), idr = bc_id(ph.bc.mark, 1, 0);
     // where this cell's state also goes: the neighbours' halo cells
     double *to_left = nullptr, *to_right = nullptr;
@@ -147,31 +150,16 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube64(const __grid_constant
 #pragma unroll
                 for (int v = 0; v < NV; ++v) to_right[v * pu] = u[v];
             }
-            if (lo_layer >= 0) {
-                double g[NV];
-                double* dst = b.U + L.at(per ? n + lo_layer : -1 - lo_layer, 0, 0);
+            if (layer >= 0) {
+                // the ghost cell beyond the side (kept for the state's ghost layers)
 #pragma unroll
-                for (int v = 0; v < NV; ++v) g[v] = u[v];
+                for (int v = 0; v < NV; ++v) ghost[v] = u[v];
                 if (!per) {
-                    bc_values(ph, idl, 0, -1.0, u, g);
+                    bc_values(ph, at_hi ? idr : idl, 0, -1.0, u, ghost);
+                    const int to = at_hi ? m + 2 + layer : 1 - layer;
 #pragma unroll
-                    for (int v = 0; v < NV; ++v) sm[at.u + v * pu + 1 - lo_layer] = g[v];
+                    for (int v = 0; v < NV; ++v) sm[at.u + v * pu + to] = ghost[v];
                 }
-#pragma unroll
-                for (int v = 0; v < NV; ++v) dst[v * L.plane] = g[v];
-            }
-            if (hi_layer >= 0) {
-                double g[NV];
-                double* dst = b.U + L.at(per ? -1 - hi_layer : n + hi_layer, 0, 0);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) g[v] = u[v];
-                if (!per) {
-                    bc_values(ph, idr, 0, -1.0, u, g);
-#pragma unroll
-                    for (int v = 0; v < NV; ++v) sm[at.u + v * pu + m + 2 + hi_layer] = g[v];
-                }
-#pragma unroll
-                for (int v = 0; v < NV; ++v) dst[v * L.plane] = g[v];
             }
         }
         cluster.sync();
@@ -276,6 +264,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube64(const __grid_constant
     if (own) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) gu[v * L.plane] = u[v];
+    }
+    if (layer >= 0) {
+        double* dst = b.U + L.at(at_hi == !per ? n + layer : -1 - layer, 0, 0);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) dst[v * L.plane] = ghost[v];
     }
     health = __reduce_or_sync(0xffffffffu, health);
     if (lane == 0 && health) atomicOr(&b.ctl->health, health);
