@@ -91,3 +91,29 @@ def test_batch_of_mixed_sizes(sizes, tslib):
             res.append([b.get(i) for i in ids])
     for (a, ia), (c, ic) in zip(*res):
         assert np.array_equal(a, c) and ia["time"] == ic["time"] and ia["iteration"] == ic["iteration"]
+
+
+def test_unhealthy_tubes_among_many(tslib):
+    """A tube that turns non-physical in a large set is stopped where the stage kernels' waits stop it: the same
+    iteration, flags and state."""
+    from turbostructred_gb300 import capi
+    res = []
+    for tail in (True, False):
+        with capi.Batch(64 << 20) as b:
+            b.set_tail(tail)
+            ids = []
+            for k in range(180):
+                n = 64 + 5 * (k % 40)
+                ic = wave(n, 1, 1)
+                if k % 30 == 7:  # a strong rarefaction from the middle: no Roe solution
+                    ic[0, 0, :n // 2, 1], ic[0, 0, n // 2:, 1] = -20.0, 20.0
+                    ic[..., 4] = 0.02 + 0.5 * ic[..., 1] ** 2 / ic[..., 0]
+                ids.append(b.add(capi.make_case(ndims=1, nx=n, periodic=(0, 1, 1), recon=3 * (k % 2), solver=1, cfl=0.5,
+                                                max_iter=120, max_time=1e30, bc=kinds("natural")), ic))
+            b.run()
+            res.append([b.get(i) for i in ids])
+    assert sum(i["health"] != 0 for _, i in res[1]) >= 3  # the inputs do what they are for
+    for (a, ia), (c, ic) in zip(*res):
+        assert (ia["iteration"], ia["health"]) == (ic["iteration"], ic["health"])
+        assert np.array_equal(a, c, equal_nan=True)
+        assert ia["time"] == ic["time"] or (np.isnan(ia["time"]) and np.isnan(ic["time"]))

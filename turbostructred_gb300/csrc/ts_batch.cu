@@ -228,6 +228,7 @@ struct ts_batch {
     // launch, state on chip
     bool tail_enabled = true, tail_mode = false;
     std::vector<TailGroup> tails;
+    bool tail_stops = false;  // a non-physical state ends its problem at that stage
     int* d_tail = nullptr;
     int tail_cap = 0;
     Arena arena;
@@ -468,6 +469,12 @@ struct ts_batch {
             act.push_back(s);
         }
         if (act.empty() || cells > kTailCells) return TS_OK;
+        // A problem whose state turns non-physical is stopped by the host at the
+        // next wait; in the last few (one cluster of 508 cells per CTA each, all
+        // at once, one CTA per SM) at that stage already.
+        int widest = 1;
+        for (int s : act) widest = std::max(widest, (desc[s].kn[0] + 507) / 508);
+        tail_stops = widest <= kTailMaxCluster && (long long)act.size() * widest <= sms;
         auto ctas = [&](int s, int own) {
             // few distinct sizes: a launch each
             for (int c : {1, 2, 3, 4, 6, 8, 10, 12, 14})
@@ -534,19 +541,15 @@ struct ts_batch {
         ++stages;
     }
 
-    ts_status replan() {
-        stable = 0;
-        return rebuild();
-    }
-
     // Stages are launched one by one right after the work list changed (a
     // capture costs more than it saves when membership keeps changing, as in
     // a served stream); once the list has been stable for a few launches,
     // chunks of stages are captured into graphs and replayed.
     ts_status launch(int n) {
         if (dirty) {
-            ts_status s = replan();
+            ts_status s = rebuild();
             if (s != TS_OK) return s;
+            stable = 0;
         }
         if (groups.empty()) return TS_OK;
         if (tail_mode) {
@@ -561,7 +564,7 @@ struct ts_batch {
                     st = side[k % (kSide + 1) - 1];
                     if (k <= kSide) TB_CUDA(cudaStreamWaitEvent(st, fork, 0));
                 }
-                TB_CUDA(tube32_launch(g.solver, g.cluster, g.n, g.cells, d_desc, d_tail + g.first, n, st));
+                TB_CUDA(tube32_launch(g.solver, g.cluster, g.n, g.cells, d_desc, d_tail + g.first, n, tail_stops, st));
                 ++launches;
             }
             for (int k = 0; k < std::min(ng - 1, kSide); ++k) {
@@ -871,9 +874,7 @@ ts_status ts_batch_run(ts_batch* b, int32_t max_stages, int32_t* active) {
         if (a == 0) break;
         if (max_stages > 0 && done >= max_stages) break;
         if (2 * ia < il) b->dirty = true;  // most listed items belong to finished problems
-        if (b->dirty && (s = b->replan()) != TS_OK) return s;
-        // the resident kernel's problems end by themselves
-        int n = b->tail_mode ? std::max(chunk, 1024) : chunk;
+        int n = chunk;
         if (max_stages > 0) n = (int)std::min<long long>(n, max_stages - done);
         if ((s = b->launch(n)) != TS_OK) return s;
         if ((s = b->pull()) != TS_OK) return s;

@@ -140,7 +140,7 @@ bool tube32_serves(const ProbDesc& d, bool one);  // one: a single domain, else 
 bool tube32_ready(int solver, int cluster, int problems, int cells);
 cudaError_t tube32_launch_one(int cluster, const ProbDesc& d, int budget, cudaStream_t st);
 cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, const ProbDesc* d_probs, const int* d_list,
-                          int budget, cudaStream_t st);
+                          int budget, bool stop_unhealthy, cudaStream_t st);
 
 // 3D problems: the TMA-staged fused kernel (ts_mix3d.cu).  Compiled tiles
 // 32x8 and 16x16; smem bytes and resident CTAs per SM, or false.

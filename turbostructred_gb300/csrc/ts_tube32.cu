@@ -85,12 +85,13 @@ __device__ __forceinline__ float half_slope(int kind, float nm, float w0, float 
 // (with the descriptor in shared memory the compiler contracts the Roe
 // flux's multiply-adds differently, as it does in the batched k_mix_step: each
 // instance gives the bits of its counterpart).  Otherwise list holds the
-// problems' descriptor indices, and a non-physical state ends a
-// problem's loop (the host stops it).
+// problems' descriptor indices, and with stop_unhealthy a non-physical state
+// ends a problem's loop (the host stops it).
 template <int SOLVER, bool ONE>
 __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant__ ProbDesc one,
                                                            const ProbDesc* __restrict__ probs,
-                                                           const int* __restrict__ list, int budget) {
+                                                           const int* __restrict__ list, int budget,
+                                                           int stop_unhealthy) {
     extern __shared__ float sm[];
     __shared__ ProbDesc sd;
     __shared__ unsigned int smax[kTailMaxCluster * kMaxWarps];
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
         // srmax >= 0: its bits order like unsigned integers
         const unsigned int mbits = __reduce_max_sync(0xffffffffu, __float_as_uint(srmax));
         if (remote_max) *remote_max = mbits;
-        if (!ONE && health) {  // rare
+        if (!ONE && stop_unhealthy && health) {  // rare
             for (int k = 0; k < nblk; ++k) atomicOr(cluster.map_shared_rank(&shealth, k), health);
         }
         cg::cluster_group::arrival_token second = cluster.barrier_arrive();
@@ -416,12 +417,12 @@ cudaError_t tube32_launch_one(int cluster, const ProbDesc& d, int budget, cudaSt
         cfg.stream = st;
         return e != cudaSuccess ? e
                                 : cudaLaunchKernelEx(&cfg, k_tube32<S, true>, d, (const ProbDesc*)nullptr,
-                                                     (const int*)nullptr, budget);
+                                                     (const int*)nullptr, budget, 0);
     });
 }
 
 cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, const ProbDesc* d_probs, const int* d_list,
-                          int budget, cudaStream_t st) {
+                          int budget, bool stop_unhealthy, cudaStream_t st) {
     if (problems <= 0 || budget <= 0) return cudaSuccess;
     ProbDesc none;
     std::memset(&none, 0, sizeof none);
@@ -430,7 +431,8 @@ cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, cons
         cudaLaunchAttribute attr[1];
         cudaError_t e = config<S, false>(cluster, problems, cells, cfg, attr);
         cfg.stream = st;
-        return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k_tube32<S, false>, none, d_probs, d_list, budget);
+        return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k_tube32<S, false>, none, d_probs, d_list, budget,
+                                                          stop_unhealthy ? 1 : 0);
     });
 }
 
