@@ -67,7 +67,10 @@ __device__ __forceinline__ void bc_values(const Phys& ph, int side, int A, doubl
 // instructions were comparisons (measured with ncu).  dkey is monotone in the
 // value and gives -0 and +0 the same key, so dkey(a) < dkey(b) is exactly
 // a < b, and the sign tests below are exactly x > 0 and x < 0, for every
-// non-NaN a, b, x (a NaN only arises in a run whose health flags stop it).
+// non-NaN a, b, x.  A NaN orders by its bits here.  Where one can come from
+// physical cells (a face state of second order with a negative pressure: the
+// root of its sound speed), Fast gives the face up and Safe tells it apart;
+// k_recon's own comparisons meet one only in a cell that holds it already.
 __device__ __forceinline__ long long dkey(double x) {
     const long long b = __double_as_longlong(x);
     return b < 0 ? (b ^ 0x7FFFFFFFFFFFFFFFLL) + 1 : b;
@@ -77,6 +80,9 @@ __device__ __forceinline__ bool dpos(double x) { return __double_as_longlong(x) 
 __device__ __forceinline__ bool dneg(double x) {
     const long long b = __double_as_longlong(x);
     return b < 0 && b != (long long)0x8000000000000000ULL;
+}
+__device__ __forceinline__ bool dnan(double x) {
+    return ((u64)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFULL) > kInfBits;
 }
 __device__ __forceinline__ bool dzero(double x) { return x64::is_zero(x64::hi_of(x), x64::lo_of(x)); }
 // |x| and -x on the integer pipe
@@ -164,6 +170,12 @@ struct Safe : Fast {
         if (no) r = hw_half(a);
         return r;
     }
+    // fmin, fmax and the comparisons of Plain for NaN too: no face is solved again
+    __device__ __forceinline__ double min(double a, double b) { return (dlt(a, b) && !dnan(a)) || dnan(b) ? a : b; }
+    __device__ __forceinline__ double max(double a, double b) { return (dlt(a, b) || dnan(a)) && !dnan(b) ? b : a; }
+    __device__ __forceinline__ bool lt(double a, double b) { return dlt(a, b) && !dnan(a) && !dnan(b); }
+    __device__ __forceinline__ bool ge0(double a) { return !dneg(a) && !dnan(a); }
+    __device__ __forceinline__ bool le0(double a) { return !dpos(a) && !dnan(a); }
 };
 // FaceArith: 3D Roe faces use FastMul: those grids keep the pipes full.  A grid of 1D or 2D
 // ends in latency instead, which the integer products lengthen (2D box
