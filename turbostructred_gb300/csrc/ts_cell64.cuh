@@ -81,9 +81,9 @@ __device__ __forceinline__ bool dneg(double x) {
     const long long b = __double_as_longlong(x);
     return b < 0 && b != (long long)0x8000000000000000ULL;
 }
-__device__ __forceinline__ bool dnan(double x) {
-    return ((u64)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFULL) > kInfBits;
-}
+// a NaN that arithmetic made (its quiet bit is in the high word)
+__device__ __forceinline__ bool dnan(double x) { return (x64::hi_of(x) & 0x7FFFFFFFu) > 0x7FF00000u; }
+__device__ __forceinline__ bool dfinite(double x) { return (x64::hi_of(x) & 0x7FF00000u) != 0x7FF00000u; }
 __device__ __forceinline__ bool dzero(double x) { return x64::is_zero(x64::hi_of(x), x64::lo_of(x)); }
 // |x| and -x on the integer pipe
 __device__ __forceinline__ double dabs(double x) { return x64::of_words(x64::hi_of(x) & 0x7FFFFFFFu, x64::lo_of(x)); }

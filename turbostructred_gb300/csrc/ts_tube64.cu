@@ -192,8 +192,14 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube64(const __grid_constant
             if (s == n && !per) bc_values(ph, idr, 0, 1.0, UL, UR);
             const bool thin = dzero(UL[2]) && dzero(UR[2]) && dzero(UL[3]) && dzero(UR[3]);
             double lam;
-            if (__all_sync(__activemask(), thin)) lam = riemann<0, SOLVER, 1, Safe>(ph, UL, UR, F, o);
-            else lam = riemann<0, SOLVER, 3, Safe>(ph, UL, UR, F, o);
+            bool full = !__all_sync(__activemask(), thin);
+            if (!full) {
+                lam = riemann<0, SOLVER, 1, Safe>(ph, UL, UR, F, o);
+                // an infinity or NaN times a zero momentum is no zero (every factor of
+                // a transverse term is one of the mass flux's too)
+                full = !dfinite(F[0]);
+            }
+            if (full) lam = riemann<0, SOLVER, 3, Safe>(ph, UL, UR, F, o);
 #pragma unroll
             for (int v = 0; v < NV; ++v) sm[at.f + v * pf + tid] = F[v];
             sm[at.f + NV * pf + tid] = lam;
