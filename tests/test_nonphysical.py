@@ -10,6 +10,7 @@ STREAMS = {
     "colliding": ((1.0, 20.0, 1.0), (1.0, -20.0, 1.0)),
     "receding": ((1.0, -20.0, 0.4), (1.0, 20.0, 0.4)),
     "from_the_left": ((1.0, 20.0, 1.0), (1.0, 0.0, 1.0)),
+    "at_rest_without_pressure": ((1.0, 0.0, 0.0), (1.0, 0.0, 0.0)),  # no wave speed anywhere: an infinite time step
 }
 GRIDS = {1: [(4, 1, 1), (100, 1, 1), (4065, 1, 1)], 2: [(100, 6, 1)], 3: [(60, 5, 4)]}
 

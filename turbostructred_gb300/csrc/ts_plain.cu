@@ -808,7 +808,8 @@ __device__ __forceinline__ void update_cell(const PlainBufs& b, const Phys& ph, 
     for (int v = 0; v < NV; ++v) {
         u[v] = uo[v];
         nrm[v] = 0.0;
-        if (dzero(R[v])) continue;
+        // (dt is infinite where no cell has a wave speed)
+        if (dzero(R[v]) && dfinite(dt)) continue;
         u[v] = uo[v] + o.mul(dt, o.over(R[v], iv));
         nrm[v] = o.mul(V, dabs(R[v]));
     }

@@ -253,9 +253,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube64(const __grid_constant
         if ((save_sol > 0) && (next_sol < time + dt)) dt = next_sol - time;
         if ((save_slice > 0) && (next_slice < time + dt)) dt = next_slice - time;
         if (own) {
+            // (dt is infinite where no cell has a wave speed)
 #pragma unroll
             for (int v = 0; v < NV; ++v)
-                if (!dzero(R[v])) u[v] = u[v] + dt * rv[v];
+                if (!dzero(R[v]) || !dfinite(dt)) u[v] = u[v] + dt * rv[v];
             health |= health_of(ph, u);
         }
         time += dt;
