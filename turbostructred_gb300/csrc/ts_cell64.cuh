@@ -425,6 +425,19 @@ __device__ __noinline__ bool ratio_less(double a1, double d1, double a2, double 
 __device__ __forceinline__ float est32(u64 b) { return __uint_as_float((unsigned)(b >> 29) - 0xC0000000u); }
 __device__ __forceinline__ bool est32_ok(u64 b) { return (unsigned)(b >> 52) - 897u < 254u; }
 
+// Whether dividing zero by the distances gives zeros (Fast gives up a cell with
+// a distance of zero; Plain divides).
+template <class O, int N>
+__device__ __forceinline__ bool nonzero(const typename O::Div* d) {
+    if constexpr (std::is_same_v<O, Plain>) return false;
+    bool ok = true;
+    if constexpr (std::is_same_v<O, Safe>) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) ok = ok && !d[k].bad;
+    }
+    return ok;
+}
+
 // Slopes (Linear2PointsStencil.h:147-178 or ENO2PointsStencil.h:202-239) and,
 // for Linear2psLim, the limiter (Linear2psLim.h:305-374, Limiters.h:28-119) of
 // one variable of a cell from its value and its neighbours'.  d: divisors of
@@ -448,8 +461,9 @@ __device__ __forceinline__ void recon_value(double val, const double nm[ND], con
             if (kmax < kv) { umax = vn; kmax = kv; }
             if (kmin > kv) { umin = vn; kmin = kv; }
         }
-        // a constant neighbourhood (finite): slopes and projections are zero
-        if (kmax == kmin && (__double2hiint(val) & 0x7FF00000) != 0x7FF00000) {
+        // a constant neighbourhood (finite): slopes and projections are zero, but
+        // for a distance of zero (cells narrower than their coordinates' last bit)
+        if (kmax == kmin && dfinite(val) && nonzero<O, KIND == P_ENO2 ? 2 * ND : ND>(d)) {
 #pragma unroll
             for (int a = 0; a < ND; ++a) g[a] = proj[a] = 0.0;
             return;
