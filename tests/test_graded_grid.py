@@ -8,7 +8,7 @@ NAT = (5, 0.0, (0.0, 0.0, 0.0), 0.0)
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,q", [(600, 0.9), (4064, 0.985), (4065, 0.985)])
-@pytest.mark.parametrize("recon,lim", [(1, 0), (3, 0), (3, 1)])
+@pytest.mark.parametrize("recon,lim", [(1, 0), (2, 0), (3, 0), (3, 1)])
 @pytest.mark.parametrize("per", [0, 1])
 def test_distances_of_zero(n, q, recon, lim, per, tslib, oracle_mod):
     from oracle import oracle as O

@@ -69,8 +69,8 @@ __device__ __forceinline__ void bc_values(const Phys& ph, int side, int A, doubl
 // a < b, and the sign tests below are exactly x > 0 and x < 0, for every
 // non-NaN a, b, x.  A NaN orders by its bits here.  Where one can come from
 // physical cells (a face state of second order with a negative pressure: the
-// root of its sound speed), Fast gives the face up and Safe tells it apart;
-// k_recon's own comparisons meet one only in a cell that holds it already.
+// root of its sound speed, or a neighbour that has left the physical states),
+// Fast gives the face or the cell up and Safe tells it apart.
 __device__ __forceinline__ long long dkey(double x) {
     const long long b = __double_as_longlong(x);
     return b < 0 ? (b ^ 0x7FFFFFFFFFFFFFFFLL) + 1 : b;
@@ -425,11 +425,67 @@ __device__ __noinline__ bool ratio_less(double a1, double d1, double a2, double 
 __device__ __forceinline__ float est32(u64 b) { return __uint_as_float((unsigned)(b >> 29) - 0xC0000000u); }
 __device__ __forceinline__ bool est32_ok(u64 b) { return (unsigned)(b >> 52) - 897u < 254u; }
 
+// recon_value as the reference states it: for the cells that Fast gives up.  A
+// slope that is not finite enters the samples along the other axes too, times
+// the zero component of their offset.
+template <int ND, int KIND>
+__device__ __forceinline__ void recon_stated(double val, const double nm[ND], const double np[ND], const double* d,
+                                             const double* hs, double eps2, double g[ND], double& lmin,
+                                             double proj[ND]) {
+    double one[ND], gs[ND];
+    lmin = 1.0;
+#pragma unroll
+    for (int a = 0; a < ND; ++a) {
+        if (KIND == P_ENO2) {
+            const double gl = (val - nm[a]) / d[2 * a], gr = (np[a] - val) / d[2 * a + 1];
+            one[a] = fabs(gl) < fabs(gr) ? gl : gr;
+        } else {
+            one[a] = (np[a] - nm[a]) / d[a];
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < ND; ++a) {
+        g[a] = one[a];
+#pragma unroll
+        for (int b = 0; b < ND; ++b)
+            if (b != a) g[a] += one[b] * 0.0;
+        gs[a] = g[a] * hs[a];
+    }
+    if (KIND == P_LIM_BJ || KIND == P_LIM_VK) {
+        double umax = val, umin = val;
+#pragma unroll
+        for (int f = 0; f < 2 * ND; ++f) {
+            const double vn = (f & 1) ? np[f >> 1] : nm[f >> 1];
+            if (umax < vn) umax = vn;
+            if (umin > vn) umin = vn;
+        }
+        if (!(umax - umin < 3.0 * 2.2250738585072014e-308)) {
+            Plain o;
+            const double un = 0.5 * (umax - umin);
+#pragma unroll
+            for (int f = 0; f < 2 * ND; ++f) {
+                const double d2 = (val + ((f & 1) ? gs[f >> 1] : -gs[f >> 1])) - val;
+                if (!(d2 > 0 || d2 < 0)) continue;
+                const double um = d2 > 0 ? umax : umin;
+                double lv;
+                if (KIND == P_LIM_VK) {
+                    lv = venkat(um / un, val / un, d2 / un, eps2, o);
+                } else {
+                    const double r = (um - val) / d2;
+                    lv = r < 1.0 ? r : 1.0;
+                }
+                if (lmin > lv) lmin = lv;
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < ND; ++a) proj[a] = (KIND == P_LIM_BJ || KIND == P_LIM_VK) ? lmin * gs[a] : gs[a];
+}
+
 // Whether dividing zero by the distances gives zeros (Fast gives up a cell with
-// a distance of zero; Plain divides).
+// a distance of zero).
 template <class O, int N>
 __device__ __forceinline__ bool nonzero(const typename O::Div* d) {
-    if constexpr (std::is_same_v<O, Plain>) return false;
     bool ok = true;
     if constexpr (std::is_same_v<O, Safe>) {
 #pragma unroll
@@ -438,9 +494,10 @@ __device__ __forceinline__ bool nonzero(const typename O::Div* d) {
     return ok;
 }
 
-// Slopes (Linear2PointsStencil.h:147-178 or ENO2PointsStencil.h:202-239) and,
-// for Linear2psLim, the limiter (Linear2psLim.h:305-374, Limiters.h:28-119) of
-// one variable of a cell from its value and its neighbours'.  d: divisors of
+// As Fast and Safe form them: slopes (Linear2PointsStencil.h:147-178 or
+// ENO2PointsStencil.h:202-239) and, for Linear2psLim, the limiter
+// (Linear2psLim.h:305-374, Limiters.h:28-119) of one variable of a cell from
+// its value and its neighbours'.  d: divisors of
 // the slopes (ENO2: left and right); hs: half cell sizes.  g: slopes, lmin:
 // limiter, proj: the projections lim * (slope * h/2) to the high faces (their
 // negatives go to the low faces).
@@ -474,7 +531,7 @@ __device__ __forceinline__ void recon_value(double val, const double nm[ND], con
         if (KIND == P_ENO2) {
             const double gl = o.over(val - nm[a], d[2 * a]);
             const double gr = o.over(np[a] - val, d[2 * a + 1]);
-            g[a] = dabs_lt(gl, gr) ? gl : gr;
+            g[a] = dabs_lt(gl, gr) && !dnan(gr) ? gl : gr;
         } else {
             g[a] = o.over(np[a] - nm[a], d[a]);
         }
@@ -499,16 +556,6 @@ __device__ __forceinline__ void recon_value(double val, const double nm[ND], con
                     if (dzero(d2)) continue;
                     const double lv = venkat(dpos(d2) ? xm : xn, xu, o.over(d2, un), eps2, o);
                     if (o.lt(lv, lmin)) lmin = lv;
-                }
-            } else if constexpr (std::is_same_v<O, Plain>) {
-#pragma unroll
-                for (int f = 0; f < 2 * ND; ++f) {
-                    const double s = (f & 1) ? gs[f >> 1] : -gs[f >> 1];
-                    const double d2 = (val + s) - val;
-                    double lv = 1.0;
-                    if (d2 > 0) { const double r = am / d2; lv = r < 1.0 ? r : 1.0; }
-                    if (d2 < 0) { const double r = an / d2; lv = r < 1.0 ? r : 1.0; }
-                    if (lv < lmin) lmin = lv;
                 }
             } else if constexpr (std::is_same_v<O, Safe>) {
                 // as below, with every ratio below 1 divided out

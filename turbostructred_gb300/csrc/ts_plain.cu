@@ -497,7 +497,8 @@ __device__ __forceinline__ void recon_var(const PlainBufs& b, int v, long long c
         nm[a] = U[-st];
         np[a] = U[st];
     }
-    recon_value<ND, KIND, O>(U[0], nm, np, d, hs, eps2, g, lim, proj, o);
+    if constexpr (std::is_same_v<O, Plain>) recon_stated<ND, KIND>(U[0], nm, np, d, hs, eps2, g, lim, proj);
+    else recon_value<ND, KIND, O>(U[0], nm, np, d, hs, eps2, g, lim, proj, o);
 #pragma unroll
     for (int a = 0; a < ND; ++a) b.G[vidx(L, a * NV + v) + c] = b.fold ? proj[a] : g[a];
     if (!b.fold && (KIND == P_LIM_BJ || KIND == P_LIM_VK)) b.Lim[vidx(L, v) + c] = lim;
