@@ -331,6 +331,9 @@ struct ts_batch {
             desc[s].ctl = d_ctl + s;
         }
         TB_CUDA(cudaMemcpyAsync(d_desc, desc.data(), sizeof(ProbDesc) * cap, cudaMemcpyHostToDevice, stream));
+        // the new problem's descriptor is written on the upload stream and a finished
+        // one's read on the download stream, neither of which waits for this one
+        TB_CUDA(cudaStreamSynchronize(stream));
         dirty = true;
         return TS_OK;
     }
