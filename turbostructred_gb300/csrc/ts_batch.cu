@@ -1058,6 +1058,10 @@ ts_status ts_batch_autotune(ts_batch* b, int32_t stages, int32_t* tx_out, int32_
             if (c < per) cand.push_back(Tune{tx, 1, c});
     }
     const Tune saved = b->tune[nd];
+    // the tiles are those of the stage kernels: sets of 1D problems that the
+    // resident kernel serves would time it for every candidate
+    const bool tail = b->tail_enabled;
+    b->tail_enabled = false;
     const long long st0 = b->stages, la0 = b->launches;
     Tune best = saved;
     float best_ms = 1e30f;
@@ -1083,6 +1087,8 @@ ts_status ts_batch_autotune(ts_batch* b, int32_t stages, int32_t* tx_out, int32_
     cudaFree(snap_ctl);
     b->stages = st0;
     b->launches = la0;
+    b->tail_enabled = tail;
+    b->dirty = true;
     if (s != TS_OK) return s;
     if ((s = ts_batch_set_tile(b, nd, best.tx, best.ty, best.ctas)) != TS_OK) return s;
     if (tx_out) *tx_out = best.tx;
