@@ -225,7 +225,11 @@ ts_status ts_step(ts_handle* h, int32_t n_steps, ts_step_info* info);
    handle's stream around the whole run and around every kernel launch of up
    to 64 evenly spaced steps (launched one by one, not from a graph).
    Per-kernel times are averages per launch over those steps; names identify
-   the kernels of one step in launch order. */
+   the kernels of one step in launch order.  The axes of an FP64 step, which
+   ts_step captures as branches beside one another, run one after the other
+   here.  A 1D domain that is resident on chip makes the launches of ts_step,
+   up to 4096 steps each: one kernel, whose time per launch is the run's over
+   its launches. */
 #define TS_MAX_KERNELS 16
 typedef struct ts_timing {
     double total_ms;
