@@ -258,8 +258,11 @@ struct ts_batch {
     size_t dstage_doubles = 0;
     // page-locked staging: new problems are copied to up_h in turn and put in
     // place from there by a kernel on the upload stream (which has drained
-    // before the buffer starts over); results are read into down_h
+    // before the buffer starts over); results are read into down_h.  An axis of
+    // more than 10918 cells has more than kStagedPart of geometry, which is copied
+    // by itself: the buffer is kept, and page-locked.
     static constexpr size_t kStage = size_t(8) << 20, kSmallStage = size_t(256) << 10;
+    static constexpr size_t kStagedPart = size_t(256) << 10;
     char *up_h = nullptr, *down_h = nullptr;
     size_t up_size = 0, up_used = 0;
     std::vector<int> quarantine;  // removed slots, reusable once the main stream has drained
@@ -742,14 +745,17 @@ ts_status ts_batch_add(ts_batch* b, const ts_config* cfg, const double* values, 
     auto undo = [&]() { for (void* p : sl.mem) b->arena.give(p); sl = Slot(); };
     ProbDesc& d = b->desc[slot];
     std::memset(&d, 0, sizeof d);
-    // everything but a large state goes through one block of the page-locked
-    // staging buffer and one launch; a state that is page-locked already is read
-    // in place, a large one through device memory, and both are waited for
+    // everything but a large state and the geometry of a long axis goes through
+    // one block of the page-locked staging buffer and one launch; a state that is
+    // page-locked already is read in place, a large one through device memory, and
+    // both are waited for
     cudaStream_t us = b->ustream;
     const size_t nvals = (size_t)L.cells() * NV;
     const double* pinned = static_cast<const double*>(pinned_device_ptr(values, b->device));
     const bool staged = !pinned && nvals * sizeof(double) <= ts_batch::kStage / 2;
-    const size_t geo = sizeof(AxisGeo) * ((L.nx + 2 * L.gx) + (L.ny + 2 * L.gy) + (L.nz + 2 * L.gz));
+    auto part = [](size_t bytes) { return bytes <= ts_batch::kStagedPart ? bytes : 0; };
+    const size_t geo = part(sizeof(AxisGeo) * (L.nx + 2 * L.gx)) + part(sizeof(AxisGeo) * (L.ny + 2 * L.gy)) +
+                       part(sizeof(AxisGeo) * (L.nz + 2 * L.gz));
     const size_t block = geo + sizeof(Ctl) + sizeof(ProbDesc) + (staged ? nvals * sizeof(double) : 0) + 16 * 16;
     if (b->up_used + block > b->up_size) {
         TB_CUDA(cudaStreamSynchronize(us));
@@ -774,6 +780,8 @@ ts_status ts_batch_add(ts_batch* b, const ts_config* cfg, const double* values, 
         return at;
     };
     auto upload = [&](void* dst, const void* src, size_t bytes) {
+        // pageable source: staged before the call returns
+        if (!part(bytes)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, us) == cudaSuccess;
         if (pl.parts >= 5) return false;
         auto& p = pl.part[pl.parts++];
         p.at = (unsigned)((put(src, bytes) - b->up_h) / sizeof(int));
