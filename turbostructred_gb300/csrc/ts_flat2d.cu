@@ -56,7 +56,7 @@ int flat_kind(const MixPhys& mp) {
 // ENO2PointsStencil.h:20-58, Linear2psLim.h:63-132, Limiters.h:28-115).
 template <int KIND>
 __device__ __forceinline__ void slopes2(float w0, const float (&nm)[2], const float (&np)[2], const AxisGeo (&g)[2],
-                                        float eps2, float (&dd)[2]) {
+                                        float eps2, float top, float (&dd)[2]) {
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
         if (KIND == FK_ENO2) {
@@ -73,7 +73,7 @@ __device__ __forceinline__ void slopes2(float w0, const float (&nm)[2], const fl
     if (KIND == FK_LIM_BJ) {
         // the smallest admissible ratio over the four face projections; with
         // both slopes 0 the ratio is dropped by fminf
-        lim = fminf(1.0f, quot(fminf(umax - w0, w0 - umin), fmaxf(fabsf(dd[0]), fabsf(dd[1]))));
+        lim = fminf(top, quot(fminf(umax - w0, w0 - umin), fmaxf(fabsf(dd[0]), fabsf(dd[1]))));
     } else if (umax - umin > 0.0f) {
         const float iun = 2.0f / (umax - umin);
 #pragma unroll
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(FNT, 3) k_flat2d(const __grid_constant__ ProbD
                     const float nm[2] = {s.w[v][ry + 1][rx], s.w[v][ry][rx + 1]};
                     const float np[2] = {s.w[v][ry + 1][rx + 2], s.w[v][ry + 2][rx + 1]};
                     float dd[2];
-                    slopes2<KIND>(s.w[v][ry + 1][rx + 1], nm, np, g, eps2, dd);
+                    slopes2<KIND>(s.w[v][ry + 1][rx + 1], nm, np, g, eps2, mp.lim_top, dd);
                     s.d[0][v][ry][rx] = dd[0];
                     s.d[1][v][ry][rx] = dd[1];
                 }

@@ -39,9 +39,9 @@ __device__ __forceinline__ double f32_to_f64(float f) {
     return __hiloint2double((int)hi, (int)(b << 29));
 }
 
-// a / b without the scaling that the compiler's approximate division does for
-// |b| > 2^126: the same bits below that, and some six instructions less in each
-// limiter (3D blast 256^3: 1.091 -> 1.073 ms per stage, whole passes).  Where the
+// a / b for |b| <= 2^126, without the scaling that the compiler's approximate
+// division does above (where this one gives 0): the same bits, and some six
+// instructions less in each limiter, whose divisors MixPhys::lim_top bounds (3D blast 256^3: 1.091 -> 1.073 ms per stage, whole passes).  Where the
 // quotient enters a sum (HLLC) the compiler would fuse it: not used there.
 __device__ __forceinline__ float quot(float a, float b) { return __fdividef(a, b); }
 

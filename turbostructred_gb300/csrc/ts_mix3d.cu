@@ -223,12 +223,13 @@ __host__ __device__ __forceinline__ int kind_of(const MixPhys& mp) {
 // reconstruction of Linear2PointsStencil.h:66-97, ENO2PointsStencil.h:20-58
 // and Linear2psLim.h:63-132 with the Barth-Jespersen and Venkatakrishnan
 // limiters (Limiters.h:28-115), in FP32: dd[ax] the unlimited half-slope
-// (explicitly rounded) and lim the limiter factor (1 without a limiter).  The
+// (explicitly rounded) and lim the limiter factor (1 without a limiter; their
+// product is the limited one: MixPhys::lim_top).  The
 // caller forms the face states as fma(+-dd, lim, w0) on every code path, so a
 // ring cell's states are the same bits in every CTA that computes them.
 template <int KIND>
 __device__ __forceinline__ void half_slopes(float w0, const float nm[3], const float np[3], const AxisGeo g[3],
-                                            float eps2, float dd[3], float& lim) {
+                                            float eps2, float top, float dd[3], float& lim) {
     lim = 1.0f;
     if (KIND == K_ENO2) {
 #pragma unroll
@@ -250,7 +251,7 @@ __device__ __forceinline__ void half_slopes(float w0, const float nm[3], const f
             umin = fminf(umin, fminf(nm[ax], np[ax]));
             dmax = fmaxf(dmax, fabsf(dd[ax]));
         }
-        lim = fminf(1.0f, quot(fminf(umax - w0, w0 - umin), dmax));
+        lim = fminf(top, quot(fminf(umax - w0, w0 - umin), dmax));
     }
     if (KIND == K_LIM_VK) {
         float umax = w0, umin = w0;
@@ -545,7 +546,7 @@ __device__ __forceinline__ void reconstruct(const ProbDesc& d, const Item3& it, 
             np[1] = smw[T::w(s0, v, box + T::BX)];
             nm[2] = smw[T::w(sm1, v, box)];
             np[2] = smw[T::w(sp1, v, box)];
-            if (KIND != K_PWC) half_slopes<KIND>(w0, nm, np, g, eps2, dd, lim);
+            if (KIND != K_PWC) half_slopes<KIND>(w0, nm, np, g, eps2, d.mp.lim_top, dd, lim);
             // face states as explicit FMAs (never split or re-fused by the
             // compiler): a ring cell's state is computed by its own CTA and
             // by the neighbouring CTA along different code paths, and must

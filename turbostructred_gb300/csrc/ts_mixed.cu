@@ -345,7 +345,7 @@ __device__ __forceinline__ void recon_k(const ProbDesc& d, float* sm, int p, con
                     umin = fminf(umin, fminf(nm[ax], np[ax]));
                     dmax = fmaxf(dmax, fabsf(dd[ax]));
                 }
-                const float lim = fminf(1.0f, quot(fminf(umax - w0, w0 - umin), dmax));
+                const float lim = fminf(d.mp.lim_top, quot(fminf(umax - w0, w0 - umin), dmax));
 #pragma unroll
                 for (int ax = 0; ax < T::NAX; ++ax) dd[ax] *= lim;
             }
@@ -960,6 +960,8 @@ ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, con
     d.ctl = ctl;
     const AxisGeo* axis_geo[3];
     const int goff[3] = {L.gx, L.gy, L.gz};
+    std::vector<AxisGeo> axes[3];
+    float ks = 0.0f;  // the largest
     ts_status s;
     // per-axis geometry with ghost entries on active axes
     for (int a = 0; a < 3; ++a) {
@@ -967,7 +969,8 @@ ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, con
         const std::vector<double>& Hh = a == 0 ? g.hx : (a == 1 ? g.hy : g.hz);
         const int n = L.n(a);
         const int gw = a == 0 ? L.gx : (a == 1 ? L.gy : L.gz);
-        std::vector<AxisGeo> geo(n + 2 * gw);
+        std::vector<AxisGeo>& geo = axes[a];
+        geo.resize(n + 2 * gw);
         auto xc = [&](int i) {  // centre of cell i (reference ghosts at -1 and n, beyond extrapolated)
             if (i >= -1 && i <= n) return X[i + 1];
             if (i < -1) return X[0] - (double)(-1 - i) * Hh[0];
@@ -991,8 +994,17 @@ ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, con
                 e.ir = (float)(1.0 / (xp - x0));
                 e.ih = (float)(1.0 / (i >= n || i < 0 ? hc(i) : h));
                 geo[i + gw] = e;
+                ks = std::max(ks, e.ks);
             }
         }
+    }
+    float top = 1.0f;
+    if (c.reconstruction == TS_RECON_LINEAR_2POINTS_LIMITED && c.limiter != TS_LIM_VENKATAKRISHNAN)
+        while (ks > 0.25f * top && top < 0x1p24f) top *= 2.0f;
+    for (int a = 0; a < 3; ++a) {
+        std::vector<AxisGeo>& geo = axes[a];
+        if (top != 1.0f)
+            for (AxisGeo& e : geo) e.ks /= top;
         void* p;
         if ((s = alloc(sizeof(AxisGeo) * geo.size(), &p)) != TS_OK) return s;
         if (!upload(p, geo.data(), sizeof(AxisGeo) * geo.size())) {
@@ -1028,6 +1040,7 @@ ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, con
     m.einf = (float)m.einf_d;
     m.eps = (float)ph.eps;
     m.cfl = ph.cfl;
+    m.lim_top = top;
     // the six sides' BCs inline; a position-dependent side's extra kinds in
     // device memory
     MixBcKinds kinds;

@@ -19,6 +19,7 @@ struct AxisGeo {
     float h;      // cell size
     float hh;     // h / 2
     float ks;     // h / (2 (x[i+1] - x[i-1])): central slope -> half projection
+                  // (over MixPhys::lim_top with the Barth-Jespersen limiter)
     float il;     // 1 / (x[i] - x[i-1])
     float ir;     // 1 / (x[i+1] - x[i])
     float ih;     // 1 / h
@@ -42,6 +43,11 @@ struct MixPhys {
     int force, accel;      // source terms on (kernel.h:941-989)
     float sigma[3], g[3];  // Sigma, UniformAcceleration
     int norms;             // form the residual norms sum V |R| (kernel.h:326)
+    float lim_top;         // Barth-Jespersen: no limiting, a power of two.  1 where every
+                           // ks is at most 1/4 (uniform axes, and graded ones away from
+                           // the joints of their blocks); else the least for which the
+                           // scaled ks are, so that no half-slope is above 2^126, the
+                           // largest divisor of quot()
 };
 
 // The extra BC kinds of position-dependent sides (table entries 6..).

@@ -52,7 +52,8 @@ struct Tube32Mem {
 enum { T_LINEAR = 1, T_ENO2 = 2, T_LIM_BJ = 3, T_LIM_VK = 4 };
 
 // Limited half-slope of one variable (as recon_k of the stage kernel).
-__device__ __forceinline__ float half_slope(int kind, float nm, float w0, float np, const AxisGeo& g, float eps2) {
+__device__ __forceinline__ float half_slope(int kind, float nm, float w0, float np, const AxisGeo& g, float eps2,
+                                            float top) {
     float dd;
     if (kind == T_ENO2) {
         const float gl = (w0 - nm) * g.il, gr = (np - w0) * g.ir;
@@ -64,7 +65,7 @@ __device__ __forceinline__ float half_slope(int kind, float nm, float w0, float 
     const float umax = fmaxf(w0, fmaxf(nm, np)), umin = fminf(w0, fminf(nm, np));
     float lim = 1.0f;
     if (kind == T_LIM_BJ) {
-        lim = fminf(1.0f, quot(fminf(umax - w0, w0 - umin), fabsf(dd)));
+        lim = fminf(top, quot(fminf(umax - w0, w0 - umin), fabsf(dd)));
     } else if (umax - umin > 0.0f) {
         const float iun = 2.0f / (umax - umin);
 #pragma unroll
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
                 float* o = sm + at.d + rl + 1;
 #pragma unroll
                 for (int v = 0; v < NV; ++v)
-                    o[v * pd] = half_slope(kind, s[v * pw - 1], s[v * pw], s[v * pw + 1], g, eps2);
+                    o[v * pd] = half_slope(kind, s[v * pw - 1], s[v * pw], s[v * pw + 1], g, eps2, mp.lim_top);
             }
             __syncthreads();
         }
