@@ -1,0 +1,101 @@
+"""The mixed kernels that stand in for another one give its bits (what decides which problems they serve): the
+resident 1D kernel and the stage kernel, single and batched; the 2D kernel that marches nothing and the marching one
+with rows of 64, 96 and 132 threads; the two 3D tiles, but for first-order HLLC."""
+import itertools
+
+import numpy as np
+import pytest
+
+from test_flat2d import SIDES, kinds, wave
+
+pytestmark = pytest.mark.gpu
+SCHEMES = [(0, 0), (1, 0), (2, 0), (3, 0), (3, 1)]
+BCS = sorted(SIDES) + ["periodic"]
+STEPS = 25
+
+
+def case(nd, n, recon, lim, solver, bc, stiff, **kw):
+    from turbostructred_gb300 import capi
+    nx, ny, nz = n
+    per = bc == "periodic"
+    src = dict(uniform_acceleration=(0.1, -0.2, 0.05)[:3], external_force=(0.05, 0.02, 0.0)) if bc in ("wall", "periodic") else {}
+    graded = {0: [(0.0, 1.02, nx)]} if bc == "natural" else {}
+    return capi.make_case(ndims=nd, nx=nx, ny=ny, nz=nz, periodic=(int(per), int(per or nd < 2), int(per or nd < 3)),
+                          recon=recon, limiter=lim, solver=solver, eps=0.1 if solver == 1 and bc == "symmetry" else 0.0,
+                          cfl=0.3, gamma=4.4 if stiff else 1.4, eos=int(stiff), p_inf=0.7 if stiff else 0.0, blocks=graded,
+                          bc=kinds("natural" if per else bc), **src, **kw)
+
+
+def state(n, stiff):
+    u = wave(*n, w3=True)
+    # a jump beside the wave, and no transverse momentum in a part of it
+    u[..., n[0] // 3:, :] *= 0.7
+    u[..., : n[0] // 5, 2:4] = 0.0
+    if stiff:
+        u[..., 4] += 4.4 * 0.7 / 3.4
+    return u
+
+
+def run(c, u, tile=None):
+    from turbostructred_gb300 import capi
+    with capi.Solver(c, precision=1) as s:
+        if tile:
+            s.set_tile(*tile)
+        s.set_state(u)
+        info = s.step(STEPS)
+        return s.get_state(), info
+
+
+def same(a, b):
+    (u, i), (v, k) = a, b
+    assert i["health"] == k["health"] == 0
+    assert np.array_equal(u, v) and i["time"] == k["time"] and i["dt"] == k["dt"]
+
+
+@pytest.mark.parametrize("recon,lim", SCHEMES)
+@pytest.mark.parametrize("solver", [1, 3])
+@pytest.mark.parametrize("bc", BCS)
+@pytest.mark.parametrize("stiff", [False, True])
+def test_single_1d(recon, lim, solver, bc, stiff, tslib):
+    for n in (40, 131, 1000):
+        c, u = case(1, (n, 1, 1), recon, lim, solver, bc, stiff), state((n, 1, 1), stiff)
+        same(run(c, u), run(c, u, (256, 1, 0)))
+
+
+@pytest.mark.parametrize("recon,lim", SCHEMES)
+@pytest.mark.parametrize("solver", [1, 3])
+@pytest.mark.parametrize("bc", BCS)
+@pytest.mark.parametrize("stiff", [False, True])
+def test_single_2d(recon, lim, solver, bc, stiff, tslib):
+    for n in ((75, 41, 1), (3, 130, 1)):
+        c, u = case(2, n, recon, lim, solver, bc, stiff), state(n, stiff)
+        flat = run(c, u)
+        for tx in (64, 96, 132):
+            same(flat, run(c, u, (tx, 1, 0)))
+
+
+@pytest.mark.parametrize("recon,lim", SCHEMES)
+@pytest.mark.parametrize("solver", [1, 3])
+@pytest.mark.parametrize("bc", BCS)
+def test_tiles_3d(recon, lim, solver, bc, tslib):
+    if recon == 0 and solver == 3:
+        pytest.skip("first-order HLLC: contracted differently in the two tiles; always 32x8")
+    c, u = case(3, (37, 21, 13), recon, lim, solver, bc, False), state((37, 21, 13), False)
+    same(run(c, u, (32, 8, 0)), run(c, u, (16, 16, 0)))
+
+
+@pytest.mark.parametrize("solver", [1, 3])
+@pytest.mark.parametrize("stiff", [False, True])
+def test_batched_1d(solver, stiff, tslib):
+    from turbostructred_gb300 import capi
+    combos = [(r, l, bc, n) for (r, l), bc, n in itertools.product(SCHEMES, BCS, (40, 131, 700))]
+    res = []
+    for tail in (True, False):
+        with capi.Batch(128 << 20) as b:
+            b.set_tail(tail)
+            ids = [b.add(case(1, (n, 1, 1), r, l, solver, bc, stiff, max_iter=STEPS, max_time=1e30), state((n, 1, 1), stiff))
+                   for r, l, bc, n in combos]
+            b.run()
+            res.append([b.get(i) for i in ids])
+    for a, c in zip(*res):
+        same(a, c)

@@ -470,7 +470,7 @@ struct ts_batch {
         for (int s = 0; s < capacity; ++s) {
             if (!slots[s].used || h_ctl[s].stop_req) continue;
             const ProbDesc& d = desc[s];
-            if (!tube32_serves(d, false)) return TS_OK;
+            if (!tube32_serves(d)) return TS_OK;
             cells += d.kn[0];
             act.push_back(s);
         }

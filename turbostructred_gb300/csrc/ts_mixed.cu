@@ -1126,7 +1126,7 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
     }
     if ((s = mixed_set_tile(mb, tx, ty, 0, err, st)) != TS_OK) return s;
     if (L.nd == 2 && L.cells() <= kFlatCells) mb.flat = flat2d_tiles(d, &d.ncx);
-    if (tube32_serves(d, true)) {
+    if (tube32_serves(d)) {
         // about 30 cells, a warp, per CTA while the cluster has CTAs left
         const int ctas = std::min(kTailMaxCluster, std::max(1, L.nx / 30));
         if (tube32_ready(d.mp.solver, ctas, 1, L.nx)) mb.tube = ctas;

@@ -142,7 +142,7 @@ ts_status mixed_set_tile(MixedBufs& mb, int tx, int ty, int zchunks, std::string
 // d_list: descriptor indices; cells: those of the largest problem.
 constexpr int kTailMaxCluster = 16;
 int tube32_max_cells();
-bool tube32_serves(const ProbDesc& d, bool one);  // one: a single domain, else batched
+bool tube32_serves(const ProbDesc& d);
 bool tube32_ready(int solver, int cluster, int problems, int cells);
 cudaError_t tube32_launch_one(int cluster, const ProbDesc& d, int budget, cudaStream_t st);
 cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, const ProbDesc* d_probs, const int* d_list,

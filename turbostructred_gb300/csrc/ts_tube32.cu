@@ -51,8 +51,11 @@ struct Tube32Mem {
 
 enum { T_LINEAR = 1, T_ENO2 = 2, T_LIM_BJ = 3, T_LIM_VK = 4 };
 
-// Limited half-slope of one variable (as recon_k of the stage kernel).
-__device__ __forceinline__ float half_slope(int kind, float nm, float w0, float np, const AxisGeo& g, float eps2,
+// Limited half-slope of one variable (as recon_k of the stage kernel); h3 = h^3.
+// The Venkatakrishnan ratio, ((dm^2 + eps^2) + 2 q dm) / (dm^2 + 2 q^2 + dm q +
+// eps^2) with eps^2 = (K h)^3 and K = 5 (Limiters.h:93-115, Constants.h:11), has the
+// FMAs that the compiler makes of it there, eps^2 among them.
+__device__ __forceinline__ float half_slope(int kind, float nm, float w0, float np, const AxisGeo& g, float h3,
                                             float top) {
     float dd;
     if (kind == T_ENO2) {
@@ -74,7 +77,10 @@ __device__ __forceinline__ float half_slope(int kind, float nm, float w0, float 
             if (d2 == 0.0f) continue;
             const float dm = ((d2 > 0.0f ? umax : umin) - w0) * iun;
             const float q = d2 * iun;
-            lim = fminf(lim, ((dm * dm + eps2) + 2.0f * q * dm) / (dm * dm + 2.0f * q * q + dm * q + eps2));
+            const float q2 = 2.0f * q, dm2 = __fmul_rn(dm, dm);
+            const float num = __fmaf_rn(q2, dm, __fmaf_rn(125.0f, h3, dm2));
+            const float den = __fmaf_rn(125.0f, h3, __fmaf_rn(dm, q, __fmaf_rn(q2, q, dm2)));
+            lim = fminf(lim, num / den);
         }
     }
     return __fmul_rn(dd, lim);
@@ -152,11 +158,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
         ri = ri < 0 ? ri + n : ri - n;
     }
     AxisGeo g{};
-    float eps2 = 0.0f;
-    if (rec) {
-        g = geo[ri];
-        eps2 = 125.0f * (g.h * g.h * g.h);  // (K h)^3 with K = 5 (Limiters.h:93-96, Constants.h:11)
-    }
+    if (rec) g = geo[ri];
+    const float h3 = g.h * g.h * g.h;
     // the own cell's factors (k_mix_step: cell_geo, residual_of)
     const AxisGeo gx = geo[own ? i0 + tid : 0];
     const float cfx = gx.ih * ih1;
@@ -231,7 +234,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
                 float* o = sm + at.d + rl + 1;
 #pragma unroll
                 for (int v = 0; v < NV; ++v)
-                    o[v * pd] = half_slope(kind, s[v * pw - 1], s[v * pw], s[v * pw + 1], g, eps2, mp.lim_top);
+                    o[v * pd] = half_slope(kind, s[v * pw - 1], s[v * pw], s[v * pw + 1], g, h3, mp.lim_top);
             }
             __syncthreads();
         }
@@ -381,14 +384,9 @@ cudaError_t config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg
 
 int tube32_max_cells() { return kTailMaxCluster * kMaxOwn; }
 
-bool tube32_serves(const ProbDesc& d, bool one) {
-    // (the compiler contracts the Venkatakrishnan limiter otherwise than in the
-    // stage kernels, but for batched Roe problems; seen at 40 cells: the others
-    // keep the stage kernels)
-    const bool vk = d.mp.recon == TS_RECON_LINEAR_2POINTS_LIMITED && d.mp.limiter == TS_LIM_VENKATAKRISHNAN;
-    const bool other = vk && (one || d.mp.solver == TS_RS_HLLC);
+bool tube32_serves(const ProbDesc& d) {
     // no residual norms are formed
-    return d.L.nd == 1 && d.kn[0] >= 4 && d.kn[0] <= tube32_max_cells() && !d.mp.norms && !other;
+    return d.L.nd == 1 && d.kn[0] >= 4 && d.kn[0] <= tube32_max_cells() && !d.mp.norms;
 }
 
 bool tube32_ready(int solver, int cluster, int problems, int cells) {
