@@ -379,7 +379,7 @@ ts_status ts_batch_remove(ts_batch* b, int32_t id);
 ts_status ts_batch_set_tile(ts_batch* b, int32_t nd, int32_t tx, int32_t ty, int32_t ctas_per_sm);
 
 /* The batch's tail mode (on by default): while every unfinished problem is
-   1D, of 4 to 8672 cells (one thread-block cluster), and all of them together
+   1D, of at most 8672 cells (one thread-block cluster), and all of them together
    have at most 300000 cells, each launch advances every problem by up to the
    requested number of stages in the resident cluster kernel, with the state
    kept on chip between stages; results are identical to the stage-by-stage

@@ -386,11 +386,11 @@ int tube32_max_cells() { return kTailMaxCluster * kMaxOwn; }
 
 bool tube32_serves(const ProbDesc& d) {
     // no residual norms are formed
-    return d.L.nd == 1 && d.kn[0] >= 4 && d.kn[0] <= tube32_max_cells() && !d.mp.norms;
+    return d.L.nd == 1 && d.kn[0] <= tube32_max_cells() && !d.mp.norms;
 }
 
 bool tube32_ready(int solver, int cluster, int problems, int cells) {
-    if (cluster < 1 || cluster > kTailMaxCluster || cells < 4 || (cells + cluster - 1) / cluster > kMaxOwn) return false;
+    if (cluster < 1 || cluster > kTailMaxCluster || cells < 2 || (cells + cluster - 1) / cluster > kMaxOwn) return false;
     auto fits = [&]<int S, bool ONE>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
