@@ -41,12 +41,8 @@ constexpr int kMaxWarps = kMaxThreads / 32;
 // Shared memory of a CTA that owns up to `own` cells (floats).
 struct Tube32Mem {
     int w, d, f, total;  // working copy, half-slopes, face fluxes
-    TS_HD explicit Tube32Mem(int own) {
-        w = 0;
-        d = w + NV * (own + 4);
-        f = d + NV * (own + 2);
-        total = f + (NV + 1) * (own + 1);
-    }
+    TS_HD constexpr explicit Tube32Mem(int own)
+        : w(0), d(w + NV * (own + 4)), f(d + NV * (own + 2)), total(f + (NV + 1) * (own + 1)) {}
 };
 
 enum { T_LINEAR = 1, T_ENO2 = 2, T_LIM_BJ = 3, T_LIM_VK = 4 };
@@ -86,8 +82,6 @@ __device__ __forceinline__ float half_slope(int kind, float nm, float w0, float 
     return __fmul_rn(dd, lim);
 }
 
-// list: the problems' descriptor indices (null: descriptor 0 alone).  A
-// non-physical state ends a batched problem's loop (the host stops it).
 // ONE: a single domain, its descriptor a kernel parameter as in k_mix_step
 // (with the descriptor in shared memory the compiler contracts the Roe
 // flux's multiply-adds differently, as it does in the batched k_mix_step: each
@@ -361,8 +355,11 @@ auto with_solver(int solver, F&& f) {
     return solver == TS_RS_HLLC ? f.template operator()<TS_RS_HLLC>() : f.template operator()<TS_RS_ROE_PIKE>();
 }
 
-template <int S, bool ONE>
-cudaError_t config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
+// Static and dynamic shared memory of the largest CTA: within what needs no opt-in.
+static_assert(sizeof(float) * Tube32Mem(kMaxOwn).total + sizeof(ProbDesc) + 4 * kTailMaxCluster * kMaxWarps + 64 <=
+              48 << 10);
+
+void config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
     cfg = cudaLaunchConfig_t{};
     cfg.gridDim = dim3((unsigned)(cluster * problems));
     cfg.blockDim = dim3((unsigned)block_threads(cluster, cells));
@@ -373,11 +370,6 @@ cudaError_t config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    // static and dynamic shared memory together may pass 48 KB
-    cudaError_t e = cudaFuncSetAttribute(k_tube32<S, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(float) * Tube32Mem(kMaxOwn).total));
-    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k_tube32<S, ONE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return e;
 }
 
 }  // namespace
@@ -395,7 +387,10 @@ bool tube32_ready(int solver, int cluster, int problems, int cells) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         int active = 0;
-        if (config<S, ONE>(cluster, problems, cells, cfg, attr) != cudaSuccess ||
+        config(cluster, problems, cells, cfg, attr);
+        // (clusters of more than 8 CTAs: allowed once per instance, before any launch)
+        if ((cluster > 8 &&
+             cudaFuncSetAttribute(k_tube32<S, ONE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
             cudaOccupancyMaxActiveClusters(&active, k_tube32<S, ONE>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             return false;
@@ -412,11 +407,9 @@ cudaError_t tube32_launch_one(int cluster, const ProbDesc& d, int budget, cudaSt
     return with_solver(d.mp.solver, [&]<int S>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
-        cudaError_t e = config<S, true>(cluster, 1, d.kn[0], cfg, attr);
+        config(cluster, 1, d.kn[0], cfg, attr);
         cfg.stream = st;
-        return e != cudaSuccess ? e
-                                : cudaLaunchKernelEx(&cfg, k_tube32<S, true>, d, (const ProbDesc*)nullptr,
-                                                     (const int*)nullptr, budget, 0);
+        return cudaLaunchKernelEx(&cfg, k_tube32<S, true>, d, (const ProbDesc*)nullptr, (const int*)nullptr, budget, 0);
     });
 }
 
@@ -428,10 +421,9 @@ cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, cons
     return with_solver(solver, [&]<int S>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
-        cudaError_t e = config<S, false>(cluster, problems, cells, cfg, attr);
+        config(cluster, problems, cells, cfg, attr);
         cfg.stream = st;
-        return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k_tube32<S, false>, none, d_probs, d_list, budget,
-                                                          stop_unhealthy ? 1 : 0);
+        return cudaLaunchKernelEx(&cfg, k_tube32<S, false>, none, d_probs, d_list, budget, stop_unhealthy ? 1 : 0);
     });
 }
 

@@ -30,7 +30,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "ts_cell64.cuh"
 #include "ts_plain.h"
