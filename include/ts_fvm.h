@@ -379,9 +379,10 @@ ts_status ts_batch_remove(ts_batch* b, int32_t id);
 ts_status ts_batch_set_tile(ts_batch* b, int32_t nd, int32_t tx, int32_t ty, int32_t ctas_per_sm);
 
 /* The batch's tail mode (on by default): while every unfinished problem is
-   1D, of at most 8672 cells (one thread-block cluster), and all of them together
-   have at most 300000 cells, each launch advances every problem by up to the
-   requested number of stages in the resident cluster kernel, with the state
+   1D, of at most 8672 cells (one thread-block cluster), and the set is one that
+   the resident cluster kernel is the faster for (from 70000 cells of problems of
+   thousands of cells to 300000 of problems of a hundred), each launch advances
+   every problem by up to the requested number of stages there, with the state
    kept on chip between stages; results are identical to the stage-by-stage
    path.  enable = 0 keeps the stage-by-stage path throughout. */
 ts_status ts_batch_set_tail(ts_batch* b, int32_t enable);

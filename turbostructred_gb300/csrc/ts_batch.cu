@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <array>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -149,13 +150,35 @@ struct Group {
 struct TailGroup {
     int solver, cluster, cells, n, first;
 };
-// Sets of 1D problems of at most this many cells in all run in the resident
-// kernel.  Measured, resident against stage launches (tubes of 64 to 4096
-// cells): 9481 cells in all, 300 stages 1.2 / 3.4 ms; 193377, 300 stages 5.7 /
-// 6.7; 285269, 200 stages 5.0 / 5.7; 353694, 200 stages 6.3 / 6.3; 3988212, 60
-// stages 25.8 / 15.0 (its two CTAs of 256 threads per SM are fewer warps than
-// the stage kernel's, and every stage waits for its cluster twice).
+// Which sets of 1D problems run in the resident kernel: those of at most
+// kTailCells cells in all whose modelled time there is the shorter one, in us per
+// stage.  Resident: 3.8 + 0.0046 x (threads per CTA) for each round of the clusters
+// that the GPU holds at once (several launches share the rounds, at some loss).
+// Stage launches: their warps in rounds of 32 per SM, 8 us at least, 0.75 for each
+// further launch of a stage, and 0.6 ms + 0.5 ms per launch until stages are captured
+// into graphs, which counts for sets with few stages left.  Fitted on 42 mixed and 90
+// uniform sets of tubes of 64 to 8192 cells.  Measured, resident / stages: 2400 of
+// 124 cells 17.4 / 21.4, 600 of 500 19.2 / 18.3, 150 of 1000 12.9 / 10.4, 48 of 4096
+// 20.4 / 16.6, 9 of 8192 12.7 / 8.0, 50 of 6000 40.3 / 17.3; whole runs of 300 stages:
+// 192 of 64 to 4096 (193377 cells) 5.7 / 6.7 ms, 50 of 6000 12.3 / 6.1.
 constexpr long long kTailCells = 300000;
+struct TailModel {
+    double rounds = 0.0, round_us = 0.0;
+    int launches = 0;
+    void add(int problems, int at_once, int threads) {
+        rounds += (double)problems / at_once;
+        round_us = std::max(round_us, 3.8 + 0.0046 * threads);
+        ++launches;
+    }
+    double resident_us() const {
+        return round_us * (launches == 1 ? std::ceil(rounds) : std::max(1.0, rounds + 0.06 * launches));
+    }
+    static double stages_us(long long warps, int launches, int sms, long long left) {
+        const double r = (double)warps / (32.0 * sms);
+        return std::max(8.0, 5.0 + 2.2 * std::ceil(r) + 4.3 * r) + 0.75 * (launches - 1) +
+               (600.0 + 500.0 * launches) / (double)left;
+    }
+};
 
 // Launch policy of one dimension: a fixed tile or (tx = 0) a tile chosen per
 // problem from its x extent; ctas = resident CTAs per SM (0: as many as fit).
@@ -457,21 +480,25 @@ struct ts_batch {
     }
 
     // Tail mode when every unfinished problem is 1D and fits one cluster, and
-    // the set is one that the resident kernel is faster for: few enough cells
-    // (kTailCells).  While the clusters fit the GPU at one CTA per SM they are
-    // made of CTAs as small as that allows (latency), otherwise of CTAs of up to 254
-    // cells (fewer halo cells); problems of equal solver and cluster size share a launch.
+    // the set is one that the resident kernel is faster for (TailModel).  While
+    // the clusters fit the GPU at one CTA per SM they are made of CTAs as small as
+    // that allows (latency), otherwise of CTAs of up to 254 cells (fewer halo
+    // cells), or 508 where all of them then run at once; problems of equal solver
+    // and cluster size share a launch.
     ts_status plan_tail() {
         tail_mode = false;
         tails.clear();
         if (!tail_enabled) return TS_OK;
         std::vector<int> act;
-        long long cells = 0;
+        long long cells = 0, warps = 0, left = 1;
         for (int s = 0; s < capacity; ++s) {
             if (!slots[s].used || h_ctl[s].stop_req) continue;
             const ProbDesc& d = desc[s];
             if (!tube32_serves(d)) return TS_OK;
             cells += d.kn[0];
+            warps += (long long)d.nq * ((slots[s].tx + 31) / 32);
+            const long long n = (long long)h_ctl[s].max_iteration - h_ctl[s].iteration;
+            left = std::max(left, n > 0 ? n : INT_MAX);  // (past its last iteration: ends by time)
             act.push_back(s);
         }
         if (act.empty() || cells > kTailCells) return TS_OK;
@@ -487,6 +514,32 @@ struct ts_batch {
                 if (c * own >= desc[s].kn[0]) return c;
             return kTailMaxCluster;
         };
+        // the launches with CTAs of up to `own` cells (no cluster fits the GPU: none)
+        std::vector<int> flat;
+        std::vector<TailGroup> plan;
+        auto plan_for = [&](int own) {
+            std::map<std::array<int, 2>, std::vector<int>> bykey;
+            for (int s : act) bykey[{desc[s].mp.solver, ctas(s, own)}].push_back(s);
+            TailModel model;
+            flat.clear();
+            plan.clear();
+            for (auto& kv : bykey) {
+                TailGroup g{kv.first[0], kv.first[1], 0, (int)kv.second.size(), (int)flat.size()};
+                for (int s : kv.second) {
+                    g.cells = std::max(g.cells, desc[s].kn[0]);
+                    flat.push_back(s);
+                }
+                int threads = 0;
+                const int at_once = tube32_at_once(g.solver, false, g.cluster, g.n, g.cells, &threads);
+                if (!at_once) {
+                    model.launches = 0;
+                    return model;
+                }
+                model.add(g.n, at_once, threads);
+                plan.push_back(g);
+            }
+            return model;
+        };
         int own = 30;
         for (int t : {30, 62, 126, 254}) {
             own = t;
@@ -494,19 +547,17 @@ struct ts_batch {
             for (int s : act) all += ctas(s, t);
             if (all <= sms) break;
         }
-        std::map<std::array<int, 2>, std::vector<int>> bykey;
-        for (int s : act) bykey[{desc[s].mp.solver, ctas(s, own)}].push_back(s);
-        std::vector<int> flat;
-        std::vector<TailGroup> plan;
-        for (auto& kv : bykey) {
-            TailGroup g{kv.first[0], kv.first[1], 0, (int)kv.second.size(), (int)flat.size()};
-            for (int s : kv.second) {
-                g.cells = std::max(g.cells, desc[s].kn[0]);
-                flat.push_back(s);
-            }
-            if (!tube32_ready(g.solver, g.cluster, g.n, g.cells)) return TS_OK;
-            plan.push_back(g);
+        TailModel model = plan_for(own);
+        if (model.launches && model.rounds > 1.0 && own == 254) {
+            // one CTA per SM of twice the cells, where that saves a round (75 tubes of
+            // 1000 cells: 8.3 -> 5.7 us per stage)
+            const double us = model.resident_us();
+            model = plan_for(508);
+            if (!model.launches || model.resident_us() >= us) model = plan_for(own);
         }
+        if (!model.launches) return TS_OK;
+        const int stage_launches = (int)groups.size() + (fused_close ? 0 : 1);
+        if (!tail_stops && model.resident_us() > TailModel::stages_us(warps, stage_launches, sms, left)) return TS_OK;
         if ((int)flat.size() > tail_cap) {
             cudaFree(d_tail);
             d_tail = nullptr;

@@ -1129,7 +1129,7 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
     if (tube32_serves(d)) {
         // about 30 cells, a warp, per CTA while the cluster has CTAs left
         const int ctas = std::min(kTailMaxCluster, std::max(1, L.nx / 30));
-        if (tube32_ready(d.mp.solver, ctas, 1, L.nx)) mb.tube = ctas;
+        if (tube32_at_once(d.mp.solver, true, ctas, 1, L.nx) > 0) mb.tube = ctas;
     }
     return TS_OK;
 }

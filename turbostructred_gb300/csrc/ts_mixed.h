@@ -143,7 +143,9 @@ ts_status mixed_set_tile(MixedBufs& mb, int tx, int ty, int zchunks, std::string
 constexpr int kTailMaxCluster = 16;
 int tube32_max_cells();
 bool tube32_serves(const ProbDesc& d);
-bool tube32_ready(int solver, int cluster, int problems, int cells);
+// The clusters that the GPU holds at once (0: none; to be asked for before a
+// launch), and the threads of their CTAs.  one: a single domain, else batched.
+int tube32_at_once(int solver, bool one, int cluster, int problems, int cells, int* threads = nullptr);
 cudaError_t tube32_launch_one(int cluster, const ProbDesc& d, int budget, cudaStream_t st);
 cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, const ProbDesc* d_probs, const int* d_list,
                           int budget, bool stop_unhealthy, cudaStream_t st);

@@ -381,9 +381,10 @@ bool tube32_serves(const ProbDesc& d) {
     return d.L.nd == 1 && d.kn[0] <= tube32_max_cells() && !d.mp.norms;
 }
 
-bool tube32_ready(int solver, int cluster, int problems, int cells) {
-    if (cluster < 1 || cluster > kTailMaxCluster || cells < 2 || (cells + cluster - 1) / cluster > kMaxOwn) return false;
-    auto fits = [&]<int S, bool ONE>() {
+int tube32_at_once(int solver, bool one, int cluster, int problems, int cells, int* threads) {
+    if (cluster < 1 || cluster > kTailMaxCluster || cells < 2 || (cells + cluster - 1) / cluster > kMaxOwn) return 0;
+    if (threads) *threads = block_threads(cluster, cells);
+    auto at_once = [&]<int S, bool ONE>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         int active = 0;
@@ -393,12 +394,12 @@ bool tube32_ready(int solver, int cluster, int problems, int cells) {
              cudaFuncSetAttribute(k_tube32<S, ONE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
             cudaOccupancyMaxActiveClusters(&active, k_tube32<S, ONE>, &cfg) != cudaSuccess) {
             cudaGetLastError();
-            return false;
+            return 0;
         }
-        return active > 0;
+        return active;
     };
     return with_solver(solver, [&]<int S>() {
-        return fits.template operator()<S, true>() && fits.template operator()<S, false>();
+        return one ? at_once.template operator()<S, true>() : at_once.template operator()<S, false>();
     });
 }
 
