@@ -846,7 +846,9 @@ bool mixed_launch_batch(int nd, int tx, int ty, int solver, int grid, const Prob
 
 // 2D problems of at most this many cells (362 x 362) march nothing: stage
 // times, k_flat2d against k_mix_step: 128^2 6.9 / 11.4 us, 256^2 11.1 / 14.0,
-// 384^2 17.5 / 17.4, 512^2 27.4 / 24.3.
+// 384^2 17.5 / 17.4, 512^2 27.4 / 24.3.  With residual norms half as many: its
+// tiles are smaller than a marching item, and each adds its norms by atomics (with
+// norms 128^2 8.9 / 12.5 us, 256^2 23.2 / 23.0, 300^2 26.7 / 21.6, 362^2 38.2 / 25.4).
 constexpr long long kFlatCells = 1LL << 17;
 
 void mixed_tile_cells(int nd, int tx, int ty, int* cx, int* cy) {
@@ -1109,8 +1111,9 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
     // 2D: rows of 64 threads, two full warps for 60 cells, where 132 threads
     // put a fifth warp behind 128: 1024^2 58.7 us per stage against 59.5, 768^2
     // 33.7 / 38.0, 512^2 21.7 / 24.0, 400x900 26.5 / 30.8 (96 threads: 60.0, 34.4,
-    // 22.9, 26.6)
-    int tx = L.nd == 3 ? 32 : (L.nd == 2 ? 64 : 256);
+    // 22.9, 26.6).  With residual norms 132, which add them half as often (512^2 30.9
+    // against 32.4, 1024x512 38.4 / 39.9).
+    int tx = L.nd == 3 ? 32 : (L.nd == 2 ? (d.mp.norms ? 132 : 64) : 256);
     int ty = L.nd == 3 ? 8 : 1;
     if (L.nd == 3) {
         // 16x16 tiles where they cover the grid with enough fewer columns
@@ -1125,7 +1128,7 @@ ts_status mixed_init(const ts_config& c, const Layout& L, const Phys& ph, const 
         if (same && 1.05 * plan3d(cols(16, 16), L.nz, slots, &z) < plan3d(cols(32, 8), L.nz, slots, &z)) tx = ty = 16;
     }
     if ((s = mixed_set_tile(mb, tx, ty, 0, err, st)) != TS_OK) return s;
-    if (L.nd == 2 && L.cells() <= kFlatCells) mb.flat = flat2d_tiles(d, &d.ncx);
+    if (L.nd == 2 && L.cells() <= (d.mp.norms ? kFlatCells / 2 : kFlatCells)) mb.flat = flat2d_tiles(d, &d.ncx);
     if (tube32_serves(d)) {
         // about 30 cells, a warp, per CTA while the cluster has CTAs left
         const int ctas = std::min(kTailMaxCluster, std::max(1, L.nx / 30));
