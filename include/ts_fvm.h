@@ -373,7 +373,8 @@ ts_status ts_batch_remove(ts_batch* b, int32_t id);
 
 /* Launch shape for the problems of dimension nd: tx = threads of the
    one-row tile along x (1D: 512, 256, 128; 2D: 260, 132, 96, 68, 64; the tile
-   owns tx - 4 cells), or 0 to pick per problem from its x extent; ty is ignored;
+   owns tx - 4 cells), or 0 to pick (1D: per problem from its x extent; 2D: one
+   for the problems that are running, from all of theirs); ty is ignored;
    and CTAs per SM of the persistent grid (0 = as many as fit).  It is the shape
    of the stage kernels: sets of 1D problems in tail mode (below) do without. */
 ts_status ts_batch_set_tile(ts_batch* b, int32_t nd, int32_t tx, int32_t ty, int32_t ctas_per_sm);

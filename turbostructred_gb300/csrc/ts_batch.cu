@@ -199,29 +199,29 @@ constexpr int kMostRows = 64;
 // stage kernel; longer lists use the separate finish kernel.
 constexpr long long kFusedCloseItems = 1024;
 
-// The one-row tile of a problem with nx cells per row.  1D: the tile that
-// covers the row with the fewest warp-slots per cell, charging each column
-// ~4 warps of fixed cost (setup, barriers, close).
-int pick_tile(int nd, int nx) {
-    // 2D: the row that covers nx cells with the fewest warps (the threads beyond a
-    // multiple of 32 cost a warp: 132 threads five for 128 cells, 64 threads two
-    // for 60, 96 three for 92)
-    if (nd == 2) {
-        int best = 132, least = 1 << 30;
-        for (int t : {132, 96, 68, 64}) {
-            int cx, cy;
-            mixed_tile_cells(nd, t, 1, &cx, &cy);
-            const int warps = (nx + cx - 1) / cx * ((t + 31) / 32);
-            if (warps < least) { least = warps; best = t; }
-        }
-        return best;
-    }
+// Tiles for 2D sets: a set takes the one that covers its rows with the fewest
+// warps (the threads beyond a multiple of 32 cost a warp: 132 threads five for 128
+// cells, 64 threads two for 60, 96 three for 92).  One for the whole set, so that a
+// stage is one launch per solver: with each problem's own tile, launches side by
+// side, 42 problems of 200 to 600 cells a side took 586 us per stage against 314
+// in rows of 64, 24 of 64 to 512 163 / 87.
+constexpr int kTiles2DAuto[] = {132, 96, 68, 64};
+long long warps_of(int tx, int nx) {
+    int cx, cy;
+    mixed_tile_cells(2, tx, 1, &cx, &cy);
+    return (long long)((nx + cx - 1) / cx) * ((tx + 31) / 32);
+}
+
+// The one-row tile of a 1D problem of nx cells: the one that covers the row with
+// the fewest warp-slots per cell, charging each column ~4 warps of fixed cost
+// (setup, barriers, close).
+int pick_tile(int nx) {
     const int* c = kTiles1D;
     int best = c[0];
     double best_cost = 1e300;
     for (int k = 0; k < 3; ++k) {
         int cx, cy;
-        mixed_tile_cells(nd, c[k], 1, &cx, &cy);
+        mixed_tile_cells(1, c[k], 1, &cx, &cy);
         const double cols = std::ceil((double)nx / cx);
         const double cost = cols * ((c[k] + 31) / 32 + 4) / (double)nx;
         if (cost < best_cost - 1e-12) { best_cost = cost; best = c[k]; }
@@ -267,6 +267,7 @@ struct ts_batch {
     bool dirty = true;
     int stable = 0;  // launches since the work list last changed
     int rows = kMostRows;  // per work item of a 2D problem
+    int tile2d = 132;      // of the 2D problems (no tile set)
     std::map<std::array<int, 3>, int> resident;  // CTAs per SM of a tile and solver
     std::map<int, cudaGraphExec_t> graphs;
     Tune tune[4] = {{0, 0, 0}, {0, 1, 0}, {0, 1, 0}, {0, 0, 0}};
@@ -380,25 +381,36 @@ struct ts_batch {
         return rows == kMostRows ? std::max(1, ny / rows) : (ny + rows - 1) / rows;
     }
 
-    // The rows per item for the unfinished 2D problems; their items are dealt
-    // again when it changes.
-    ts_status plan_rows() {
+    // The tile of the unfinished 2D problems and the rows per item; their items
+    // are dealt again when one of them changes.
+    ts_status plan_2d() {
         std::vector<int> act;
         for (int s = 0; s < capacity; ++s)
             if (slots_used(s) && desc[s].L.nd == 2) act.push_back(s);
         if (act.empty()) return TS_OK;
+        int tile = tile2d;
+        long long least = LLONG_MAX;
+        for (int t : kTiles2DAuto) {
+            long long warps = 0;
+            for (int s : act) warps += warps_of(t, desc[s].kn[0]) * desc[s].kn[2];
+            if (warps < least) {
+                least = warps;
+                tile = t;
+            }
+        }
+        const int tx = tune[2].tx > 0 ? tune[2].tx : tile;
         int want = kMostRows;
         for (int r : kRowsPerItem) {
             long long warps = 0;
-            for (int s : act)
-                warps += (long long)desc[s].ncol * chunks_of(desc[s].kn[2], r) * ((slots[s].tx + 31) / 32);
+            for (int s : act) warps += warps_of(tx, desc[s].kn[0]) * chunks_of(desc[s].kn[2], r);
             if (warps <= 24LL * sms) {  // what the marching tiles are compiled for
                 want = r;
                 break;
             }
         }
-        if (want == rows) return TS_OK;
+        if (want == rows && tile == tile2d) return TS_OK;
         rows = want;
+        tile2d = tile;
         for (int s : act) {
             place(s);
             TB_CUDA(cudaMemcpyAsync(d_desc + s, &desc[s], sizeof(ProbDesc), cudaMemcpyHostToDevice, stream));
@@ -411,7 +423,7 @@ struct ts_batch {
     void place(int s) {
         ProbDesc& d = desc[s];
         const int nd = d.L.nd;
-        slots[s].tx = tune[nd].tx > 0 ? tune[nd].tx : pick_tile(nd, d.kn[0]);
+        slots[s].tx = tune[nd].tx > 0 ? tune[nd].tx : (nd == 2 ? tile2d : pick_tile(d.kn[0]));
         slots[s].ty = 1;
         const int chunks = nd >= 2 ? chunks_of(d.kn[2], rows) : 1;
         mixed_items(d, slots[s].tx, 1, chunks, (long long)sms);
@@ -420,7 +432,7 @@ struct ts_batch {
     // Work items of unfinished problems, grouped by (nd, solver), each group
     // sorted by problem size, largest first.
     ts_status rebuild() {
-        ts_status rs = plan_rows();
+        ts_status rs = plan_2d();
         if (rs != TS_OK) return rs;
         std::map<std::array<int, 4>, std::vector<int>> bykey;
         for (int s = 0; s < capacity; ++s) {
