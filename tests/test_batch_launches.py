@@ -39,3 +39,13 @@ def test_2d_sets_take_one_tile(sides, tslib):
     assert launches <= 3 * STAGES
     for tile in (64, 132):
         same(got, run(probs, tile)[1])
+
+
+@pytest.mark.parametrize("sizes", [tuple(64 + 21 * k for k in range(22)), (30, 61, 125, 250, 600, 900, 1500, 2100, 3000, 4000),
+                                   (4000,) * 9, (8600, 5)])
+def test_1d_sets_in_few_launches(sizes, tslib):
+    """Sets that run at once on the GPU: at most as many launches as there are streams for all stages."""
+    probs = [(case(1, n, 1, 1 + 2 * (k % 2), 3 * (k % 3 > 0)), wave(n, 1, 1)) for k, n in enumerate(sizes)]
+    launches, got = run(probs)
+    assert launches <= 5
+    same(got, run(probs, tail=False)[1])

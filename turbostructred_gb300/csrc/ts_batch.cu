@@ -152,26 +152,34 @@ struct TailGroup {
 };
 // Which sets of 1D problems run in the resident kernel: those of at most
 // kTailCells cells in all whose modelled time there is the shorter one, in us per
-// stage.  Resident: 3.8 + 0.0046 x (threads per CTA) for each round of the clusters
-// that the GPU holds at once (several launches share the rounds, at some loss).
-// Stage launches: their warps in rounds of 32 per SM, 8 us at least, 0.75 for each
-// further launch of a stage, and 0.6 ms + 0.5 ms per launch until stages are captured
-// into graphs, which counts for sets with few stages left.  Fitted on 42 mixed and 90
-// uniform sets of tubes of 64 to 8192 cells.  Measured, resident / stages: 2400 of
-// 124 cells 17.4 / 21.4, 600 of 500 19.2 / 18.3, 150 of 1000 12.9 / 10.4, 48 of 4096
-// 20.4 / 16.6, 9 of 8192 12.7 / 8.0, 50 of 6000 40.3 / 17.3; whole runs of 300 stages:
-// 192 of 64 to 4096 (193377 cells) 5.7 / 6.7 ms, 50 of 6000 12.3 / 6.1.
+// stage.  Resident: 2.4 + (threads per CTA) x (0.0068 + 0.0027 x further CTAs per SM)
+// for each round of the clusters that the GPU holds at once, and for each launch
+// that waits for another on its stream.  Stage launches: their warps in rounds of
+// 32 per SM, 8 us at least, 0.75 for each further launch of a stage, and 0.6 ms + 0.5
+// ms per launch until stages are captured into graphs, which counts for sets with
+// few stages left.  Fitted on 170 sets of tubes of 64 to 8600 cells.  Measured,
+// resident / stages: 2400 of 124 cells 17.4 / 21.4, 600 of 500 19.2 / 18.3, 150 of
+// 1000 12.9 / 10.4, 48 of 4096 20.4 / 16.6, 9 of 8192 12.7 / 8.0, 50 of 6000 40.3 /
+// 17.3; whole runs of 300 stages: 192 of 64 to 4096 (193377 cells) 5.7 / 6.7 ms, 50 of
+// 6000 12.3 / 6.1.
 constexpr long long kTailCells = 300000;
 struct TailModel {
-    double rounds = 0.0, round_us = 0.0;
-    int launches = 0;
-    void add(int problems, int at_once, int threads) {
+    double rounds = 0.0;
+    long long ctas = 0;
+    int launches = 0, threads = 0;
+    void add(int problems, int cluster, int at_once, int cta_threads) {
         rounds += (double)problems / at_once;
-        round_us = std::max(round_us, 3.8 + 0.0046 * threads);
+        ctas += (long long)problems * cluster;
+        threads = std::max(threads, cta_threads);
         ++launches;
     }
-    double resident_us() const {
-        return round_us * (launches == 1 ? std::ceil(rounds) : std::max(1.0, rounds + 0.06 * launches));
+    double resident_us(int streams, int sms) const {
+        const double per_sm = (double)ctas / std::max(1.0, rounds) / sms;
+        const double round = 2.4 + threads * (0.0068 + 0.0027 * (std::min(4.0, std::max(1.0, per_sm)) - 1.0));
+        // (clusters of wide CTAs of several launches do not fill the last of the SMs)
+        const double one = threads > 288 ? 0.9 : 1.0;
+        const double r = launches == 1 ? std::ceil(rounds) : (rounds <= one ? 1.0 : std::max(1.9, rounds + 0.3));
+        return round * std::max(r, (double)((launches + streams - 1) / streams));
     }
     static double stages_us(long long warps, int launches, int sms, long long left) {
         const double r = (double)warps / (32.0 * sms);
@@ -269,6 +277,9 @@ struct ts_batch {
     int rows = kMostRows;  // per work item of a 2D problem
     int tile2d = 132;      // of the 2D problems (no tile set)
     std::map<std::array<int, 3>, int> resident;  // CTAs per SM of a tile and solver
+    // clusters of the resident kernel that the GPU holds at once, and their CTAs'
+    // threads, by solver, CTAs and cells per CTA
+    std::map<std::array<int, 3>, std::array<int, 2>> at_once;
     std::map<int, cudaGraphExec_t> graphs;
     Tune tune[4] = {{0, 0, 0}, {0, 1, 0}, {0, 1, 0}, {0, 0, 0}};
     // uploads of admitted problems and read-backs of finished ones run on
@@ -492,11 +503,7 @@ struct ts_batch {
     }
 
     // Tail mode when every unfinished problem is 1D and fits one cluster, and
-    // the set is one that the resident kernel is faster for (TailModel).  While
-    // the clusters fit the GPU at one CTA per SM they are made of CTAs as small as
-    // that allows (latency), otherwise of CTAs of up to 254 cells (fewer halo
-    // cells), or 508 where all of them then run at once; problems of equal solver
-    // and cluster size share a launch.
+    // the set is one that the resident kernel is faster for (TailModel).
     ts_status plan_tail() {
         tail_mode = false;
         tails.clear();
@@ -520,18 +527,19 @@ struct ts_batch {
         int widest = 1;
         for (int s : act) widest = std::max(widest, (desc[s].kn[0] + 507) / 508);
         tail_stops = widest <= kTailMaxCluster && (long long)act.size() * widest <= sms;
-        auto ctas = [&](int s, int own) {
-            // few distinct sizes: a launch each
-            for (int c : {1, 2, 3, 4, 6, 8, 10, 12, 14})
+        // A plan: CTAs of up to `own` cells, clusters of the listed sizes, a launch for
+        // each that is used and for each solver.
+        typedef std::vector<int> Sizes;
+        auto ctas = [&](int s, int own, const Sizes& sizes) {
+            for (int c : sizes)
                 if (c * own >= desc[s].kn[0]) return c;
-            return kTailMaxCluster;
+            return sizes.back();
         };
-        // the launches with CTAs of up to `own` cells (no cluster fits the GPU: none)
         std::vector<int> flat;
         std::vector<TailGroup> plan;
-        auto plan_for = [&](int own) {
+        auto plan_for = [&](int own, const Sizes& sizes) {
             std::map<std::array<int, 2>, std::vector<int>> bykey;
-            for (int s : act) bykey[{desc[s].mp.solver, ctas(s, own)}].push_back(s);
+            for (int s : act) bykey[{desc[s].mp.solver, ctas(s, own, sizes)}].push_back(s);
             TailModel model;
             flat.clear();
             plan.clear();
@@ -541,35 +549,40 @@ struct ts_batch {
                     g.cells = std::max(g.cells, desc[s].kn[0]);
                     flat.push_back(s);
                 }
-                int threads = 0;
-                const int at_once = tube32_at_once(g.solver, false, g.cluster, g.n, g.cells, &threads);
-                if (!at_once) {
-                    model.launches = 0;
-                    return model;
-                }
-                model.add(g.n, at_once, threads);
+                auto& at = at_once[{g.solver, g.cluster, (g.cells + g.cluster - 1) / g.cluster}];  // asked for once
+                if (!at[1]) at[0] = tube32_at_once(g.solver, false, g.cluster, g.n, g.cells, &at[1]);
+                if (!at[0]) return TailModel();
+                model.add(g.n, g.cluster, at[0], at[1]);
                 plan.push_back(g);
             }
             return model;
         };
-        int own = 30;
-        for (int t : {30, 62, 126, 254}) {
-            own = t;
-            long long all = 0;
-            for (int s : act) all += ctas(s, t);
-            if (all <= sms) break;
+        // Few distinct sizes waste few CTAs, more of them are more launches.  CTAs as
+        // small as one per SM allows, else of 254 cells, or of 508 where that is faster.
+        static const Sizes kSizes[] = {{1, 2, 3, 4, 6, 8, 10, 12, 14, 16}, {1, 2, 4, 8, 16}, {1, 4, 16}, {2, 16}, {16}};
+        const Sizes* sizes = nullptr;
+        int own = 0;
+        double us = 1e300;
+        for (const Sizes& z : kSizes) {
+            if (&z != kSizes && (long long)act.size() > sms) break;  // rounds count then, not launches
+            for (int t : {30, 62, 126, 254, 508}) {
+                long long all = 0;
+                for (int s : act) all += ctas(s, t, z);
+                if (all > sms && t < 254) continue;
+                const TailModel m = plan_for(t, z);
+                const double now = m.launches ? m.resident_us(kSide + 1, sms) : 1e300;
+                if (now < (&z == kSizes ? 0.98 : 0.9) * us) {
+                    us = now;
+                    own = t;
+                    sizes = &z;
+                }
+                if (all <= sms) break;
+            }
         }
-        TailModel model = plan_for(own);
-        if (model.launches && model.rounds > 1.0 && own == 254) {
-            // one CTA per SM of twice the cells, where that saves a round (75 tubes of
-            // 1000 cells: 8.3 -> 5.7 us per stage)
-            const double us = model.resident_us();
-            model = plan_for(508);
-            if (!model.launches || model.resident_us() >= us) model = plan_for(own);
-        }
-        if (!model.launches) return TS_OK;
+        if (!sizes) return TS_OK;
+        plan_for(own, *sizes);
         const int stage_launches = (int)groups.size() + (fused_close ? 0 : 1);
-        if (!tail_stops && model.resident_us() > TailModel::stages_us(warps, stage_launches, sms, left)) return TS_OK;
+        if (!tail_stops && us > TailModel::stages_us(warps, stage_launches, sms, left)) return TS_OK;
         if ((int)flat.size() > tail_cap) {
             cudaFree(d_tail);
             d_tail = nullptr;
