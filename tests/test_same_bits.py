@@ -99,3 +99,22 @@ def test_batched_1d(solver, stiff, tslib):
             res.append([b.get(i) for i in ids])
     for a, c in zip(*res):
         same(a, c)
+
+
+@pytest.mark.parametrize("n", [4064, 4065, 8160, 8672])
+@pytest.mark.parametrize("recon,lim", [(0, 0), (3, 0), (3, 1)])
+@pytest.mark.parametrize("solver", [1, 3])
+def test_wide_ctas(n, recon, lim, solver, tslib):
+    """On both sides of the CTAs that send one CFL maximum each, single and batched."""
+    from turbostructred_gb300 import capi
+    u = state((n, 1, 1), False)
+    c = case(1, (n, 1, 1), recon, lim, solver, "moving", False, max_iter=STEPS, max_time=1e30)
+    same(run(c, u), run(c, u, (256, 1, 0)))
+    res = []
+    for tail in (True, False):
+        with capi.Batch(64 << 20) as b:
+            b.set_tail(tail)
+            i = b.add(c, u)
+            b.run()
+            res.append(b.get(i))
+    same(*res)

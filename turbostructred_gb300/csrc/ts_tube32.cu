@@ -82,13 +82,29 @@ __device__ __forceinline__ float half_slope(int kind, float nm, float w0, float 
     return __fmul_rn(dd, lim);
 }
 
+// a >= b on the integer pipe: every warp forms it at every stage, and an FP64
+// comparison of 16 of them is 300 clocks.
+__device__ __forceinline__ bool at_least(double a, double b) {
+    auto key = [](double x) {
+        const long long k = __double_as_longlong(x);
+        return k < 0 ? (long long)0x8000000000000000ULL - k : k;
+    };
+    const long long inf = 0x7FF0000000000000LL, x = key(a), y = key(b);
+    return x >= y && x <= inf && y >= -inf && x >= -inf && y <= inf;
+}
+
 // ONE: a single domain, its descriptor a kernel parameter as in k_mix_step
 // (with the descriptor in shared memory the compiler contracts the Roe
 // flux's multiply-adds differently, as it does in the batched k_mix_step: each
 // instance gives the bits of its counterpart).  Otherwise list holds the
 // problems' descriptor indices, and with stop_unhealthy a non-physical state
 // ends a problem's loop (the host stops it).
-template <int SOLVER, bool ONE>
+// WIDE, for CTAs of more than kWideThreads: each CTA sends its CFL maximum instead of
+// each of its warps, a barrier more, but 16 values instead of up to 16 x 17 for
+// every warp to send and read (one tube, batched, 7487 cells 6.07 -> 5.68 us per
+// stage, with at_least; 480 cells would take 3.07 instead of 2.96).
+constexpr int kWideThreads = 256;
+template <int SOLVER, bool ONE, bool WIDE>
 __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant__ ProbDesc one,
                                                            const ProbDesc* __restrict__ probs,
                                                            const int* __restrict__ list, int budget,
@@ -96,7 +112,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
     extern __shared__ float sm[];
     __shared__ ProbDesc sd;
     __shared__ unsigned int smax[kTailMaxCluster * kMaxWarps];
-    __shared__ unsigned int shealth;
+    __shared__ unsigned int shealth, wmax[kMaxWarps];
     cg::cluster_group cluster = cg::this_cluster();
     const int nblk = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, W = blockDim.x >> 5;
@@ -136,6 +152,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
     float dtf = __double2float_rn(ctl->dt_apply);
     int iteration = ctl->iteration, par = ctl->parity;
     const int max_iteration = ctl->max_iteration, run_mode = ctl->run_mode;
+    const bool sols = save_sol > 0, slices = save_slice > 0;
     double u[NV];
     float r[NV];
 #pragma unroll
@@ -171,7 +188,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
     // boundary images beyond a non-periodic side: of cells 0, 1 and n-1, n-2
     const int lo_img = own && !per && i0 + tid < 2 ? i0 + tid : -1;
     const int hi_img = own && !per && n - 1 - (i0 + tid) < 2 ? n - 1 - (i0 + tid) : -1;
-    unsigned int* const remote_max = lane < nblk ? cluster.map_shared_rank(smax, lane) + rank * W + wid : nullptr;
+    const int sent = WIDE ? 1 : W;  // values of a CTA
+    unsigned int* const remote_max =
+        lane < nblk && (!WIDE || wid == 0) ? cluster.map_shared_rank(smax, lane) + rank * sent + (WIDE ? 0 : wid) : nullptr;
     unsigned int health = 0;
     bool stop = false;
     cluster.sync();  // every CTA has started: its shared memory may be written
@@ -267,7 +286,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
             srmax = fmaxf(srmax, (fsx * (lxl + lxr)) * iv);
         }
         // srmax >= 0: its bits order like unsigned integers
-        const unsigned int mbits = __reduce_max_sync(0xffffffffu, __float_as_uint(srmax));
+        unsigned int mbits = __reduce_max_sync(0xffffffffu, __float_as_uint(srmax));
+        if (WIDE) {
+            if (lane == 0) wmax[wid] = mbits;
+            __syncthreads();
+            if (wid == 0) mbits = __reduce_max_sync(0xffffffffu, lane < W ? wmax[lane] : 0u);
+        }
         if (remote_max) *remote_max = mbits;
         if (!ONE && stop_unhealthy && health) {  // rare
             for (int k = 0; k < nblk; ++k) atomicOr(cluster.map_shared_rank(&shealth, k), health);
@@ -299,19 +323,19 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_tube32(const __grid_constant
         cluster.barrier_wait(std::move(second));
         // dt and the step's bookkeeping (finish_with)
         unsigned int all = 0;
-        for (int k = lane; k < nblk * W; k += 32) all = max(all, smax[k]);
+        for (int k = lane; k < nblk * sent; k += 32) all = max(all, smax[k]);
         all = __reduce_max_sync(0xffffffffu, all);
         step_size(mp.cfl, __uint_as_float(all), dt, raw);
-        if ((save_sol > 0) && (next_sol < time + dt)) dt = next_sol - time;
-        if ((save_slice > 0) && (next_slice < time + dt)) dt = next_slice - time;
+        if (sols && (next_sol < time + dt)) dt = next_sol - time;
+        if (slices && (next_slice < time + dt)) dt = next_slice - time;
         dtf = __double2float_rn(dt);
         time += dt;
         iteration += 1;
         par ^= 1;
         if (run_mode) {
-            if ((save_sol > 0) && (next_sol == time)) next_sol += save_sol;
-            if ((save_slice > 0) && (next_slice == time)) next_slice += save_slice;
-            stop = iteration == max_iteration || time >= max_time;
+            if (sols && (next_sol == time)) next_sol += save_sol;
+            if (slices && (next_slice == time)) next_slice += save_slice;
+            stop = iteration == max_iteration || at_least(time, max_time);
         }
         const bool finished = stop;
         if (!ONE && shealth) stop = true;
@@ -350,9 +374,13 @@ int own_cells(int cluster, int cells) {
 }
 int block_threads(int cluster, int cells) { return (own_cells(cluster, cells) + 2 + 31) / 32 * 32; }
 
+// Calls f.template operator()<SOLVER, WIDE>() for a launch.
 template <class F>
-auto with_solver(int solver, F&& f) {
-    return solver == TS_RS_HLLC ? f.template operator()<TS_RS_HLLC>() : f.template operator()<TS_RS_ROE_PIKE>();
+auto with_instance(int solver, int threads, F&& f) {
+    auto go = [&]<int S>() {
+        return threads > kWideThreads ? f.template operator()<S, true>() : f.template operator()<S, false>();
+    };
+    return solver == TS_RS_HLLC ? go.template operator()<TS_RS_HLLC>() : go.template operator()<TS_RS_ROE_PIKE>();
 }
 
 // Static and dynamic shared memory of the largest CTA: within what needs no opt-in.
@@ -383,34 +411,35 @@ bool tube32_serves(const ProbDesc& d) {
 
 int tube32_at_once(int solver, bool one, int cluster, int problems, int cells, int* threads) {
     if (cluster < 1 || cluster > kTailMaxCluster || cells < 2 || (cells + cluster - 1) / cluster > kMaxOwn) return 0;
-    if (threads) *threads = block_threads(cluster, cells);
-    auto at_once = [&]<int S, bool ONE>() {
+    const int nt = block_threads(cluster, cells);
+    if (threads) *threads = nt;
+    auto at_once = [&]<int S, bool ONE, bool WIDE>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         int active = 0;
         config(cluster, problems, cells, cfg, attr);
         // (clusters of more than 8 CTAs: allowed once per instance, before any launch)
-        if ((cluster > 8 &&
-             cudaFuncSetAttribute(k_tube32<S, ONE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
-            cudaOccupancyMaxActiveClusters(&active, k_tube32<S, ONE>, &cfg) != cudaSuccess) {
+        if ((cluster > 8 && cudaFuncSetAttribute(k_tube32<S, ONE, WIDE>, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                                 1) != cudaSuccess) ||
+            cudaOccupancyMaxActiveClusters(&active, k_tube32<S, ONE, WIDE>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
         return active;
     };
-    return with_solver(solver, [&]<int S>() {
-        return one ? at_once.template operator()<S, true>() : at_once.template operator()<S, false>();
+    return with_instance(solver, nt, [&]<int S, bool WIDE>() {
+        return one ? at_once.template operator()<S, true, WIDE>() : at_once.template operator()<S, false, WIDE>();
     });
 }
 
 cudaError_t tube32_launch_one(int cluster, const ProbDesc& d, int budget, cudaStream_t st) {
     if (budget <= 0) return cudaSuccess;
-    return with_solver(d.mp.solver, [&]<int S>() {
+    return with_instance(d.mp.solver, block_threads(cluster, d.kn[0]), [&]<int S, bool WIDE>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         config(cluster, 1, d.kn[0], cfg, attr);
         cfg.stream = st;
-        return cudaLaunchKernelEx(&cfg, k_tube32<S, true>, d, (const ProbDesc*)nullptr, (const int*)nullptr, budget, 0);
+        return cudaLaunchKernelEx(&cfg, k_tube32<S, true, WIDE>, d, (const ProbDesc*)nullptr, (const int*)nullptr, budget, 0);
     });
 }
 
@@ -419,12 +448,12 @@ cudaError_t tube32_launch(int solver, int cluster, int problems, int cells, cons
     if (problems <= 0 || budget <= 0) return cudaSuccess;
     ProbDesc none;
     std::memset(&none, 0, sizeof none);
-    return with_solver(solver, [&]<int S>() {
+    return with_instance(solver, block_threads(cluster, cells), [&]<int S, bool WIDE>() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         config(cluster, problems, cells, cfg, attr);
         cfg.stream = st;
-        return cudaLaunchKernelEx(&cfg, k_tube32<S, false>, none, d_probs, d_list, budget, stop_unhealthy ? 1 : 0);
+        return cudaLaunchKernelEx(&cfg, k_tube32<S, false, WIDE>, none, d_probs, d_list, budget, stop_unhealthy ? 1 : 0);
     });
 }
 
