@@ -1002,7 +1002,7 @@ ts_status mixed_problem(const ts_config& c, const Layout& L, const Phys& ph, con
     }
     float top = 1.0f;
     if (c.reconstruction == TS_RECON_LINEAR_2POINTS_LIMITED && c.limiter != TS_LIM_VENKATAKRISHNAN)
-        while (ks > 0.25f * top && top < 0x1p24f) top *= 2.0f;
+        while (ks > kMaxKs * top && top < 0x1p24f) top *= 2.0f;
     for (int a = 0; a < 3; ++a) {
         std::vector<AxisGeo>& geo = axes[a];
         if (top != 1.0f)

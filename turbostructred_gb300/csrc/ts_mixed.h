@@ -43,11 +43,12 @@ struct MixPhys {
     int force, accel;      // source terms on (kernel.h:941-989)
     float sigma[3], g[3];  // Sigma, UniformAcceleration
     int norms;             // form the residual norms sum V |R| (kernel.h:326)
-    float lim_top;         // Barth-Jespersen: no limiting, a power of two.  1 where every
-                           // ks is at most 1/4 (uniform axes, and graded ones away from
-                           // the joints of their blocks); else the least for which the
-                           // scaled ks are, so that no half-slope is above 2^126, the
-                           // largest divisor of quot()
+    float lim_top;         // Barth-Jespersen: no limiting, a power of two.  1 where no ks is
+                           // above kMaxKs: half-slopes stay below 2^126, the largest
+                           // divisor of quot(), while neighbouring values differ by less
+                           // than 2.9e38 (beyond, E + p overflows).  Else, at joints of
+                           // blocks, the least for which the scaled ks are not; half-slopes
+                           // below 2.4e-38 are zero then
 };
 
 // The extra BC kinds of position-dependent sides (table entries 6..).
@@ -56,6 +57,10 @@ struct MixBcKinds {
     float state[TS_MAX_BC_KINDS][5];
     float vel[TS_MAX_BC_KINDS][3];
 };
+
+// The largest ks of an axis graded by up to 2 from cell to cell: of its end cells
+// (1 / (3 + 1/q); 1/4 on a uniform axis).
+constexpr float kMaxKs = 0.2858f;
 
 // Everything the fused kernel needs about one problem (lives in device memory).
 // The kernel works on kernel axes 0 (x), 1 (the tile's second axis, 3D
