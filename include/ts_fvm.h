@@ -388,10 +388,10 @@ ts_status ts_batch_set_tile(ts_batch* b, int32_t nd, int32_t tx, int32_t ty, int
    path.  enable = 0 keeps the stage-by-stage path throughout. */
 ts_status ts_batch_set_tail(ts_batch* b, int32_t enable);
 
-/* Autotuner: times `stages` stages of the current batch for the per-problem
-   policy and every compiled tile, each at several CTA counts, restoring the
-   problems' states after each trial, and keeps the fastest; *tx (0: per
-   problem), *ty, *ctas_per_sm receive the choice for the batch's dominant
+/* Autotuner: times `stages` stages of the current batch, in stage launches,
+   for the batch's own choice and for tiles of 512, 256 and 128 (1D) or 260, 132 and
+   68 threads (2D), each at several CTA counts, restoring the problems' states
+   after each trial, and keeps the fastest; *tx (0: the batch's choice), *ty, *ctas_per_sm receive the choice for the batch's dominant
    dimension. */
 ts_status ts_batch_autotune(ts_batch* b, int32_t stages, int32_t* tx, int32_t* ty, int32_t* ctas_per_sm);
 

@@ -132,9 +132,9 @@ struct FastMul : Fast {
     }
 };
 // Safe: Fast whose operations fall back one by one instead of giving up: for
-// kernels in which a warp's latency is all that counts and the tails of a
-// wave (momenta below 2^-510, of cells that a perturbation has just reached)
-// would send some warp through the second arithmetic at every step.
+// kernels in which a warp's latency is all that counts, and a subnormal result
+// (in the tails of a wave, of cells that a perturbation has just reached) would send
+// some warp through the second arithmetic at every step.
 static __device__ __noinline__ double hw_div(double a, double b) { return a / b; }
 static __device__ __noinline__ double hw_sqrt(double a) { return sqrt(a); }
 static __device__ __noinline__ double hw_half(double a) { return a * 0.5; }

@@ -18,10 +18,10 @@
 // integers, or a square root, that is a 54-bit odd integer would need an
 // operand of more than 53 bits.
 //
-// Operands outside the ranges stated at each routine (zero divisors,
-// subnormals, infinities, NaN, very large or small exponents) are not
-// handled: the routine reports them through `bad` and the caller takes the
-// hardware operation instead.  A zero dividend is handled (signed zero).
+// Every normal operand is taken.  Zero divisors, subnormal operands and results,
+// infinities and NaN are not: the routine reports them through `bad` and the
+// caller takes the hardware operation instead.  A zero dividend, and a result
+// that rounds to zero, are signed zeros.
 //
 // Compiles for the host too (the seed is then 1.0f / x, any seed within
 // 2^-21 serves).

@@ -3,8 +3,8 @@
 //
 // What bounds it: latency.  A small grid leaves most of the chip idle, and the
 // marching kernel (k_mix_step) takes five dependent rows of loads and three
-// passes of three barriers for the one row that each CTA then owns (12.3 us
-// per stage at 128 x 128).  Here all 288 cells of the tile and its 2-cell halo
+// passes of three barriers for the one row that each CTA then owns (10.4 us
+// per stage at 128 x 128, in rows of 64 threads, against 6.1).  Here all 288 cells of the tile and its 2-cell halo
 // are loaded at once, one per thread; the slopes of the 200 cells that the
 // faces need, the 132 x faces (threads 0..131) and 160 y faces (threads
 // 160..319), and the 128 residuals each take one pass, with a barrier between.  A

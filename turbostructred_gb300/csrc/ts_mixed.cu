@@ -845,8 +845,8 @@ bool mixed_launch_batch(int nd, int tx, int ty, int solver, int grid, const Prob
 }
 
 // 2D problems of at most this many cells (362 x 362) march nothing: stage
-// times, k_flat2d against k_mix_step: 128^2 6.9 / 11.4 us, 256^2 11.1 / 14.0,
-// 384^2 17.5 / 17.4, 512^2 27.4 / 24.3.  With residual norms half as many: its
+// times, k_flat2d against k_mix_step: 64^2 6.1 / 10.2 us, 128^2 6.1 / 10.4, 256^2
+// 10.8 / 13.0, 362^2 16.4 / 16.2.  With residual norms half as many: its
 // tiles are smaller than a marching item, and each adds its norms by atomics (with
 // norms 128^2 8.9 / 12.5 us, 256^2 23.2 / 23.0, 300^2 26.7 / 21.6, 362^2 38.2 / 25.4).
 constexpr long long kFlatCells = 1LL << 17;
