@@ -384,7 +384,7 @@ auto with_instance(int solver, int threads, F&& f) {
 }
 
 // Static and dynamic shared memory of the largest CTA: within what needs no opt-in.
-static_assert(sizeof(float) * Tube32Mem(kMaxOwn).total + sizeof(ProbDesc) + 4 * kTailMaxCluster * kMaxWarps + 64 <=
+static_assert(sizeof(float) * Tube32Mem(kMaxOwn).total + sizeof(ProbDesc) + 4 * (kTailMaxCluster + 1) * kMaxWarps + 64 <=
               48 << 10);
 
 void config(int cluster, int problems, int cells, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
